@@ -2,8 +2,8 @@
 
 ``listed()`` names the cases, ``draw(rng)`` gives one more of the same ranges, ``prepare(case, seed)`` makes what a
 program holds before the call, ``run(state)`` is one pass through the public entry points, ``work(case)`` the bytes and
-operations a pass cannot do without, and ``tolerance(case)`` how far the outputs of another correct implementation at
-the same precision may lie apart.
+operations a pass cannot do without, ``tolerance(case)`` how far the outputs of another correct implementation at the
+same precision may lie apart, and ``exact(case, seed)`` the outputs in 64 bits.
 
 Kinds of case (all tensors bf16 [B, H, L, D]; a (batch, head) unit is one attention problem):
 
@@ -404,3 +404,133 @@ def tolerance(case):
         # rows that attend it then differ by that key's share
         tol["max"] = 0.3
     return tol
+
+
+# ----------------------------------------------------------------------------------------------- the same in 64 bits
+def _probabilities(q, k, scale, keep=None):
+    """Softmax rows of one (batch, head) unit in fp64, with the row maxima and sums of the scores; ``keep``: a mask."""
+    s = (q.double() @ k.double().T) * scale
+    if keep is not None:
+        s.masked_fill_(~keep, float("-inf"))
+    m = s.max(-1, keepdim=True).values
+    s.sub_(m).exp_()
+    n = s.sum(-1, keepdim=True)
+    return s.div_(n), m, n
+
+
+def _by_group(p, rows):
+    """Sums over groups of ``rows`` query rows."""
+    pad = -p.shape[0] % rows
+    return torch.nn.functional.pad(p, (0, 0, 0, pad)).view(-1, rows, p.shape[1]).sum(1)
+
+
+def _listed_attention(q, k, v, scale, lists, rows):
+    """Attention of each group of ``rows`` query rows over the keys of its list, fp64."""
+    out = []
+    for g in range(lists.shape[0]):
+        i = lists[g].long()
+        out.append(_probabilities(q[g * rows:(g + 1) * rows], k[i], scale)[0] @ v[i].double())
+    return torch.cat(out)
+
+
+def _units(fn, B, H):
+    """fn(b, h) gives a tuple of tensors of one unit; stacked to [B, H, ...]."""
+    got = [[fn(b, h) for h in range(H)] for b in range(B)]
+    return [torch.stack([torch.stack([got[b][h][i] for h in range(H)]) for b in range(B)]) for i in range(len(got[0][0]))]
+
+
+def _exact_layer(c, s):
+    B, H = c["B"], c["H"]
+    a, e = s["start"], s["end"]
+    q, k, v = (s["qkv"][:, :, i].permute(0, 2, 1, 3).double() for i in range(3))
+    cos, sin = s["cos"][a:e].double(), s["sin"][a:e].double()
+
+    def turn(x):
+        x = x / x.norm(dim=-1, keepdim=True)
+        x0, x1 = x[..., 0::2], x[..., 1::2]
+        return torch.stack([cos * x0 - sin * x1, sin * x0 + cos * x1], -1).flatten(-2)
+    q, k = turn(q) * s["scale_mul"].double().view(1, H, 1, 1), turn(k)
+    out = {"q": q, "k": k, "v": v}
+    # the attention reads what the prologue stores, which is bf16
+    Q = q.bfloat16()
+    Kc = torch.cat([s["k_cache"][:, :, :a], k.bfloat16()], 2)
+    V = torch.cat([s["v_cache"][:, :, :a], v.bfloat16()], 2)
+    route, rows = c["route"], GROUP
+    if route == "dense":
+        out["o"], = _units(lambda b, h: (_probabilities(Q[b, h], Kc[b, h], 1.0)[0] @ V[b, h].double(),), B, H)
+    elif route == "csla":
+        m = _csla_mask(c["scale"]).cuda().repeat_interleave(128, 0).repeat_interleave(128, 1)[:e - a, :e]
+        out["o"], = _units(lambda b, h: (_probabilities(Q[b, h], Kc[b, h], 1.0, m)[0] @ V[b, h].double(),), B, H)
+    elif route == "full":
+        top = P.indices_count(0.05, e, MULTIPLE)
+
+        def unit(b, h):
+            p = _probabilities(Q[b, h], Kc[b, h], 1.0)[0]
+            o = p @ V[b, h].double()
+            lists = _by_group(p, rows).topk(top, -1).indices
+            return o, o - _listed_attention(Q[b, h], Kc[b, h], V[b, h], 1.0, lists, rows)
+        out["o"], out["cache"] = _units(unit, B, H)
+        out.update(lists=None, counts=None)
+    else:
+        lists, _, count, cache = s["before"]
+        band = s["layer"].sparse_attn.local_inds[c["scale"]][0].cuda()
+        Gk, Gs = band.shape[0], lists.shape[2]
+        near = ((torch.arange(Gk).float() + 0.5) / Gk * Gs - 0.5).round().long().clamp(0, Gs - 1)
+        side, prev = SCALES[c["scale"]], SCALES[c["scale"] - 1]
+
+        def unit(b, h):
+            mine = torch.cat([lists[b, h, near.cuda(), :count], band], -1)
+            grid = cache[b, h].double().view(prev, prev, -1).permute(2, 0, 1)[None]
+            grid = torch.nn.functional.interpolate(grid, size=(side, side), mode="bilinear", align_corners=False)
+            return grid[0].flatten(1).T + _listed_attention(Q[b, h], Kc[b, h], V[b, h], 1.0, mine, rows),
+        out["o"], = _units(unit, B, H)
+        out.update(lists=None, counts=None)
+    return out
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs, in fp64 by plain torch; ``None`` for selections and for ``evict``, whose
+    outputs are copies of inputs chosen by bf16-rounded scores."""
+    c = case
+    kind, B, H = c["kind"], c["B"], c["H"]
+    if kind == "evict":
+        return None
+    s = prepare(c, seed)
+    if kind == "layer":
+        return _exact_layer(c, s)
+    if kind == "score":
+        sc = s["scale"]
+        out = []
+        for i, q in s["q"].items():
+            n = CUM[i + 1]
+            row, = _units(lambda b, h: (_probabilities(q[b, h], s["k"][b, h, :n], sc)[0].sum(0, keepdim=True),), B, H)
+            out.append((row, None) if round(0.1 * n) else (row,))
+        return out
+    q, k, v, sc = s["q"], s["k"], s["v"], s["scale"]
+    if kind == "mask":
+        def unit(b, h):
+            p = _probabilities(q[b, h], k[b, h], sc)[0]
+            return p @ v[b, h].double(), _by_group(p, 128)
+        o, cs = _units(unit, B, H)
+        return {"o": o, "cs": cs, "mask": None}
+    if kind == "block":
+        def unit(b, h):
+            m = s["mask"][b, h].repeat_interleave(c["block"], 0).repeat_interleave(c["block"], 1)[:c["Lq"], :c["Lkv"]]
+            return _probabilities(q[b, h], k[b, h], sc, m)[0] @ v[b, h].double(),
+        return _units(unit, B, H)[0]
+    if kind == "given":
+        def unit(b, h):
+            p, m, n = _probabilities(q[b, h], k[b, h], sc)
+            total = m.exp() * n
+            return p @ v[b, h].double(), _by_group(p * (total * s["p"][b, h].double()), GROUP), 1 / total
+        return _units(unit, B, H)
+    if kind == "group":
+        def unit(b, h):
+            p, m, n = _probabilities(q[b, h], k[b, h], sc)
+            o, cs = p @ v[b, h].double(), _by_group(p, c["rows"])
+            lists = cs.topk(c["keep"], -1).indices
+            return (o, m[:, 0] * math.log2(math.e), n[:, 0], cs,
+                    s["o"][b, h].double() + _listed_attention(q[b, h], k[b, h], v[b, h], sc, lists, c["rows"]))
+        o, M, L, cs, out = _units(unit, B, H)
+        return {"o": o, "M": M, "L": L, "cs": cs, "lists": None, "counts": None, "out": out}
+    raise ValueError(kind)
