@@ -9,13 +9,17 @@
 // separate multiplies and add/subtract), one rounding to bf16 at the end: the reference keeps q and k in
 // fp32 and casts them to v's dtype at every call site.
 // rope(x)[2i] = cos[p,i] x[2i] - sin[p,i] x[2i+1],  rope(x)[2i+1] = sin[p,i] x[2i] + cos[p,i] x[2i+1],
-// p = rope_start + l.  One warp per (b, l, h) row, two rows per iteration; a lane holds c/32 consecutive elements
-// (whole pairs).
+// p = rope_start + l.
+//
+// Bound by HBM (12 c bytes per token and head, every byte once) as long as the arithmetic stays below it: c / 8 lanes
+// share a (b, l, h) row and hold 8 consecutive elements each (16-byte accesses), a warp takes one token and a few heads
+// so that the rotation table is read once for all of them, and every index is 32-bit.  A warp per row with 4 or 2
+// elements per lane, 64-bit index divisions and a library division per element was bound by instruction issue:
+// 66 us for 2 x 4096 tokens x 16 heads x 128 and 256 us for 8 x 4096, now 37 and 136 us (5.9 TB/s).
 #include <math.h>
 
-#include <type_traits>
-
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace lvar {
 
@@ -38,89 +42,150 @@ struct PrologueParams {
   int B, L, H;
 };
 
-template <int EPL>  // elements per lane: 2 (c = 64) or 4 (c = 128)
-__global__ void __launch_bounds__(256) qkv_prologue_kernel(const PrologueParams p) {
-  constexpr int C = EPL * 32;
-  constexpr int ROWS = 2;  // (b, l, h) rows per warp and iteration: their nine loads are issued before any arithmetic
-  using Vec = typename std::conditional<EPL == 4, uint2, uint32_t>::type;
+// a / b rounded to nearest, for r = 1 / b rounded to nearest: the residual of the first quotient is exact in a fused
+// multiply-add and corrects it (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990).  Three instructions per element once the row's reciprocal is known.
+__device__ __forceinline__ float div_by(float a, float b, float r) {
+  const float q = __fmul_rn(a, r);
+  return fmaf(fmaf(-q, b, a), r, q);
+}
+
+template <bool WIDE>
+__device__ __forceinline__ uint4 load8(const __nv_bfloat16* p) {
+  if (WIDE) return *reinterpret_cast<const uint4*>(p);
+  const uint2 lo = reinterpret_cast<const uint2*>(p)[0], hi = reinterpret_cast<const uint2*>(p)[1];
+  return make_uint4(lo.x, lo.y, hi.x, hi.y);
+}
+template <bool WIDE>
+__device__ __forceinline__ void store8(__nv_bfloat16* p, const uint4& v) {
+  if (WIDE) {
+    *reinterpret_cast<uint4*>(p) = v;
+  } else {
+    reinterpret_cast<uint2*>(p)[0] = make_uint2(v.x, v.y);
+    reinterpret_cast<uint2*>(p)[1] = make_uint2(v.z, v.w);
+  }
+}
+template <bool WIDE>
+__device__ __forceinline__ void load4f(const float* p, float (&out)[4]) {
+  if (WIDE) {
+    const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+    out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[i] = __ldg(p + i);
+  }
+}
+
+// One warp: one token, ROWS * 32 / (C / 8) of its heads, all loads issued before any arithmetic.  WIDE: every base
+// and stride allows 16-byte accesses (else 8-byte ones, and single floats from the tables).
+template <int C, bool WIDE>
+__global__ void __launch_bounds__(256) qkv_prologue_kernel(const PrologueParams p, int units, int chunks) {
+  constexpr int LPR = C / 8;        // lanes per row
+  constexpr int RPW = 32 / LPR;     // rows per warp at a time
+  constexpr int ROWS = 2;           // rows per lane
   const int lane = threadIdx.x & 31;
-  const int64_t rows = (int64_t)p.B * p.L * p.H;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t row0 = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row0 < rows; row0 += warps * ROWS) {
-    Vec raw[ROWS][3];
-    int hh[ROWS], ll[ROWS], bb_[ROWS];
-    float cs[ROWS][EPL / 2], sn[ROWS][EPL / 2];
+  const int unit = (int)blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
+  if (unit >= units) return;
+  const int t = unit / chunks;      // token over the batch
+  const int b = t / p.L, l = t - b * p.L;
+  const int h0 = (unit - t * chunks) * (ROWS * RPW) + lane / LPR;
+  const int e0 = (lane % LPR) * 8;  // this lane's first element
+  const __nv_bfloat16* src = p.qkv + b * p.s_b + l * p.s_l + e0;
+  uint4 raw[ROWS][3];
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-      const int64_t row = row0 + r * warps;
-      if (row >= rows) continue;
-      hh[r] = (int)(row % p.H);
-      ll[r] = (int)((row / p.H) % p.L);
-      bb_[r] = (int)(row / ((int64_t)p.H * p.L));
-      const __nv_bfloat16* src = p.qkv + bb_[r] * p.s_b + ll[r] * p.s_l + hh[r] * p.s_h + lane * EPL;
+  for (int r = 0; r < ROWS; ++r) {
+    const int h = h0 + r * RPW;
+    if (h < p.H) {
 #pragma unroll
-      for (int which = 0; which < 3; ++which) raw[r][which] = *reinterpret_cast<const Vec*>(src + which * p.s_w);
-      if (p.cos_t != nullptr) {
-        const int64_t base = (int64_t)(p.rope_start + ll[r]) * (C / 2) + (lane * EPL >> 1);
-#pragma unroll
-        for (int e = 0; e < EPL / 2; ++e) {
-          cs[r][e] = p.cos_t[base + e];
-          sn[r][e] = p.sin_t[base + e];
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-      const int64_t row = row0 + r * warps;
-      if (row >= rows) continue;  // warp-uniform
-      const int h = hh[r], l = ll[r], b = bb_[r];
-#pragma unroll
-      for (int which = 0; which < 3; ++which) {
-        __nv_bfloat16 el[EPL];
-        *reinterpret_cast<Vec*>(el) = raw[r][which];
-        __nv_bfloat16* dst;
-        if (which == 0) {
-          dst = p.q_out + b * p.q_sb + h * p.q_sh + (int64_t)l * p.q_sl;
-        } else if (which == 1) {
-          dst = p.k_cache + b * p.k_sb + h * p.k_sh + (int64_t)(p.cache_pos + l) * p.k_sl;
-        } else {
-          dst = p.v_cache + b * p.v_sb + h * p.v_sh + (int64_t)(p.cache_pos + l) * p.v_sl;
-        }
-        dst += lane * EPL;
-        if (which < 2) {
-          float x[EPL];
-#pragma unroll
-          for (int e = 0; e < EPL; ++e) x[e] = __bfloat162float(el[e]);
-          if (p.scale_mul != nullptr) {
-            float ssq = 0.f;
-#pragma unroll
-            for (int e = 0; e < EPL; ++e) ssq = fmaf(x[e], x[e], ssq);
-#pragma unroll
-            for (int d = 16; d >= 1; d >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, d);
-            const float denom = fmaxf(sqrtf(ssq), 1e-12f);
-            const float mul = which == 0 ? p.scale_mul[h] : 1.0f;
-#pragma unroll
-            for (int e = 0; e < EPL; ++e) {
-              x[e] = __fdiv_rn(x[e], denom);
-              if (which == 0) x[e] = __fmul_rn(x[e], mul);
-            }
-          }
-          if (p.cos_t != nullptr) {
-#pragma unroll
-            for (int e = 0; e < EPL; e += 2) {
-              const float c1 = cs[r][e >> 1], s1 = sn[r][e >> 1];
-              const float a = x[e], b2 = x[e + 1];
-              x[e] = __fsub_rn(__fmul_rn(c1, a), __fmul_rn(s1, b2));
-              x[e + 1] = __fadd_rn(__fmul_rn(s1, a), __fmul_rn(c1, b2));
-            }
-          }
-#pragma unroll
-          for (int e = 0; e < EPL; ++e) el[e] = __float2bfloat16_rn(x[e]);
-        }
-        *reinterpret_cast<Vec*>(dst) = *reinterpret_cast<const Vec*>(el);
-      }
+      for (int which = 0; which < 3; ++which) raw[r][which] = load8<WIDE>(src + h * p.s_h + which * p.s_w);
+    } else {
+      raw[r][0] = raw[r][1] = raw[r][2] = make_uint4(0, 0, 0, 0);
     }
   }
+  float cs[4], sn[4];
+  if (p.cos_t != nullptr) {
+    const int64_t base = (int64_t)(p.rope_start + l) * (C / 2) + (e0 >> 1);
+    load4f<WIDE>(p.cos_t + base, cs);
+    load4f<WIDE>(p.sin_t + base, sn);
+  }
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    const int h = h0 + r * RPW;
+    const bool live = h < p.H;  // lanes past the last head still take part in the shuffles
+    uint4 out[2];
+#pragma unroll
+    for (int which = 0; which < 2; ++which) {
+      const uint32_t u[4] = {raw[r][which].x, raw[r][which].y, raw[r][which].z, raw[r][which].w};
+      float x[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        x[2 * i] = __uint_as_float(u[i] << 16);
+        x[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
+      }
+      if (p.scale_mul != nullptr) {
+        // squares of EPS consecutive elements are summed in order, then a pairwise tree over the row's 32 such sums
+        constexpr int EPS = C / 32;
+        constexpr int NS = 8 / EPS;  // sums this lane starts with
+        float ssq[NS];
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+          ssq[i] = 0.f;
+#pragma unroll
+          for (int e = 0; e < EPS; ++e) ssq[i] = fmaf(x[i * EPS + e], x[i * EPS + e], ssq[i]);
+#pragma unroll
+          for (int d = LPR / 2; d >= 1; d >>= 1) ssq[i] += __shfl_xor_sync(0xffffffffu, ssq[i], d);
+        }
+#pragma unroll
+        for (int d = NS / 2; d >= 1; d >>= 1)
+#pragma unroll
+          for (int i = 0; i < d; ++i) ssq[i] += ssq[i + d];
+        const float denom = fmaxf(sqrtf(ssq[0]), 1e-12f);
+        const float mul = which == 0 && live ? p.scale_mul[h] : 1.0f;
+        if (ssq[0] < INFINITY) {
+          // denom lies in [1e-12, 2^64] and no quotient overflows
+          const float inv = __frcp_rn(denom);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) x[e] = div_by(x[e], denom, inv);
+        } else {  // an infinite or NaN sum of squares
+#pragma unroll
+          for (int e = 0; e < 8; ++e) x[e] = __fdiv_rn(x[e], denom);
+        }
+        if (which == 0) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) x[e] = __fmul_rn(x[e], mul);
+        }
+      }
+      if (p.cos_t != nullptr) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float a = x[2 * i], b2 = x[2 * i + 1];
+          x[2 * i] = __fsub_rn(__fmul_rn(cs[i], a), __fmul_rn(sn[i], b2));
+          x[2 * i + 1] = __fadd_rn(__fmul_rn(sn[i], a), __fmul_rn(cs[i], b2));
+        }
+      }
+      out[which] = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]),
+                              pack_bf16x2(x[6], x[7]));
+    }
+    if (live) {
+      const int64_t pos = p.cache_pos + l;
+      store8<WIDE>(p.q_out + b * p.q_sb + h * p.q_sh + l * p.q_sl + e0, out[0]);
+      store8<WIDE>(p.k_cache + b * p.k_sb + h * p.k_sh + pos * p.k_sl + e0, out[1]);
+      store8<WIDE>(p.v_cache + b * p.v_sb + h * p.v_sh + pos * p.v_sl + e0, raw[r][2]);
+    }
+  }
+}
+
+template <int C>
+int launch_c(const PrologueParams& p, bool wide, cudaStream_t stream) {
+  constexpr int HEADS = 2 * 32 / (C / 8);  // heads per warp
+  const int chunks = (p.H + HEADS - 1) / HEADS;
+  const int64_t units = (int64_t)p.B * p.L * chunks;
+  LVAR_REQUIRE(units < (1ll << 31) - 8, LVAR_ERR_LIMIT, "too many rows");
+  const unsigned blocks = (unsigned)((units + 7) / 8);
+  if (wide) qkv_prologue_kernel<C, true><<<blocks, 256, 0, stream>>>(p, (int)units, chunks);
+  else qkv_prologue_kernel<C, false><<<blocks, 256, 0, stream>>>(p, (int)units, chunks);
+  LVAR_CUDA_OK(cudaGetLastError());
+  return LVAR_OK;
 }
 
 }  // namespace
@@ -148,13 +213,11 @@ int launch_qkv_prologue(const void* qkv, int64_t s_b, int64_t s_l, int64_t s_w, 
   p.v_cache = static_cast<__nv_bfloat16*>(v_cache); p.v_sb = v_sb; p.v_sh = v_sh; p.v_sl = v_sl;
   p.cache_pos = cache_pos;
   p.B = B; p.L = L; p.H = H;
-  const int64_t rows = (int64_t)B * L * H;
-  int64_t blocks = (rows + 7) / 8;
-  if (blocks > 148 * 8) blocks = 148 * 8;
-  if (c == 128) qkv_prologue_kernel<4><<<(unsigned)blocks, 256, 0, stream>>>(p);
-  else qkv_prologue_kernel<2><<<(unsigned)blocks, 256, 0, stream>>>(p);
-  LVAR_CUDA_OK(cudaGetLastError());
-  return LVAR_OK;
+  // 16-byte accesses where every row starts on a 16-byte boundary; 8-byte ones otherwise
+  bool wide = (uintptr_t)rope_cos % 16 == 0 && (uintptr_t)rope_sin % 16 == 0;
+  for (int64_t s : strides) wide = wide && s % 8 == 0;
+  for (uintptr_t a : ptrs) wide = wide && a % 16 == 0;
+  return c == 128 ? launch_c<128>(p, wide, stream) : launch_c<64>(p, wide, stream);
 }
 
 }  // namespace lvar

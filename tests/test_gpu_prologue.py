@@ -65,3 +65,58 @@ def test_prologue_argument_errors(K):
         K.qkv_prologue(qkv, None, None, None, 0, cache, cache.clone(), 0)
     with pytest.raises(RuntimeError, match="bfloat16"):
         K.qkv_prologue(qkv.float(), None, None, None, 0, cache, cache.clone(), 0)
+
+
+@pytest.mark.parametrize("B,L,H,c", [(1, 1, 1, 128), (2, 7, 3, 128), (1, 5, 4, 64), (3, 2, 9, 64), (2, 33, 16, 128), (1, 3, 17, 64)])
+def test_prologue_8_byte_rows_give_the_same_bits(K, B, L, H, c):
+    """Rows on 16-byte boundaries and rows that are only 8-byte aligned, head counts off the warp's share, and rows
+    with extreme, infinite and NaN elements: the same bits from both kernels, and those of plain division."""
+    g = torch.Generator().manual_seed(B * 1000 + L * 10 + H)
+    qkv = torch.randn(B, L, 3, H, c, generator=g).bfloat16()
+    qkv[0, 0, 0, 0, 0] = float("inf")
+    qkv[0, 0, 1, 0, 1] = float("nan")
+    qkv[0, 0, 1, 0, 2] = 3e38
+    if L > 1:
+        qkv[0, 1, 0, 0, :4] = torch.tensor([3e38, -3e38, 1e-38, 5.0])   # the sum of squares overflows
+        qkv[0, 1, 1, 0] *= 1e-25                                         # the norm is clamped
+        qkv[0, 1, 1, H - 1] = 0.0
+    qkv = qkv.cuda()
+    sm = (torch.rand(H, generator=g) * 4).cuda()
+    ang = torch.rand(L + 2, c // 2, generator=g) * 6
+    cos, sin = ang.cos().cuda(), ang.sin().cuda()
+
+    def caches(shift):
+        return [torch.zeros(B * H * (L + 3) * c + 4, dtype=torch.bfloat16, device="cuda")[shift:shift + B * H * (L + 3) * c]
+                .view(B, H, L + 3, c) for _ in range(2)]
+    k0, v0 = caches(0)
+    q0 = K.qkv_prologue(qkv, sm, cos, sin, 2, k0, v0, 3)
+    shifted = torch.zeros(qkv.numel() + 4, dtype=torch.bfloat16, device="cuda")[4:].view(qkv.shape)   # 8-byte aligned
+    shifted.copy_(qkv)
+    k1, v1 = caches(4)
+    q1 = K.qkv_prologue(shifted, sm, cos, sin, 2, k1, v1, 3)
+    for a, b in ((q0, q1), (k0, k1), (v0, v1)):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+    assert torch.equal(v0[:, :, 3:].view(torch.int16), qkv[:, :, 2].permute(0, 2, 1, 3).contiguous().view(torch.int16))
+
+    # the row's sum of squares in the kernel's order: c/32 consecutive squares, then pairs at distance 16, 8, ..., 1
+    def unit(x, mul):
+        x = x.permute(0, 2, 1, 3).float()
+        parts = torch.zeros(x.shape[:-1] + (32,), device="cuda", dtype=torch.float64)
+        xd = x.double().view(*x.shape[:-1], 32, c // 32)
+        for e in range(c // 32):                       # fp32 fused multiply-add: one rounding of the exact sum
+            parts = (parts + xd[..., e] * xd[..., e]).float().double()
+        s = parts.float()
+        for d in (16, 8, 4, 2, 1):
+            s = s[..., :d] + s[..., d:]
+        n = s.sqrt()
+        n = torch.where(n > 1e-12, n, torch.tensor(1e-12, device="cuda"))
+        x = x / n
+        if mul is not None:
+            x = x * mul.view(1, H, 1, 1)
+        x0, x1 = x[..., 0::2], x[..., 1::2]
+        cs, sn = cos[2:], sin[2:]
+        return torch.stack([cs * x0 - sn * x1, sn * x0 + cs * x1], -1).flatten(-2).bfloat16()
+    for got, want in ((q0, unit(qkv[:, :, 0], sm)), (k0[:, :, 3:], unit(qkv[:, :, 1], None))):
+        fin = torch.isfinite(want)
+        assert torch.equal(torch.isnan(got), torch.isnan(want))
+        assert torch.equal(got[fin], want[fin])
