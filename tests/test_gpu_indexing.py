@@ -199,3 +199,23 @@ def test_topk_is_torch_topk_on_the_same_gpu(K):
     same_val = torch.gather(s, -1, got)
     inc = (got[:, 1:] > got[:, :-1]) | (same_val[:, 1:] != same_val[:, :-1])
     assert inc.all()                                                   # lower index first among equals
+
+
+@pytest.mark.parametrize("k_len,src_cols,cnt,band_count", [(10521, 6425, 1280, 128), (77, 77, 77, 0), (77, 80, 70, 5), (78, 10, 72, 6),
+                                                            (79, 79, 0, 3), (5, 5, 4, 0), (4, 4, 4, 0), (1, 3, 0, 0)])
+def test_sparse_step_lists_row_edges(K, k_len, src_cols, cnt, band_count):
+    """Row lengths of every remainder modulo 4 (rows then start off 16-byte boundaries), full and empty rows, lists
+    shorter than cnt, a source with padded rows: every element against a direct restatement."""
+    torch.manual_seed(k_len + cnt)
+    B, H, Gs, Gk = 2, 3, 4, 5
+    inds = torch.randint(-5, 2 * k_len + 5, (B, H, Gs, src_cols + 3), dtype=torch.int32)[..., :src_cols]
+    remap = torch.tensor([0, 3, 1, 2, 2], dtype=torch.int32)
+    band = torch.randint(0, k_len, (Gk, band_count), dtype=torch.int32) if band_count else None
+    rep = 1 if src_cols >= cnt else -(-cnt // src_cols)
+    want = torch.zeros(B, H, Gk, k_len, dtype=torch.int32)
+    want[..., :cnt] = inds[:, :, remap.long()][..., torch.arange(cnt) // rep].clamp(0, k_len - 1)
+    if band_count:
+        want[..., cnt:cnt + band_count] = band
+    src = inds.cuda()
+    got, counts = K.sparse_step_lists(src, remap.cuda(), band.cuda() if band_count else None, cnt, k_len, count_value=9)
+    assert torch.equal(got.cpu(), want) and (counts == 9).all()
