@@ -11,6 +11,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace lvar {
 
@@ -20,67 +21,144 @@ constexpr int kMaxWindow = 64;
 
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
-// One warp per pass handles 32 / (D/8) keys: D/8 lanes read one 16-byte piece of a key row each.
+// 1 / sqrt(D) as fp32.  A bf16 logit times this constant rounds to the same bf16 value as the quotient by
+// sqrt(D), for every bf16 value (checked over all of them by tests/test_scalekv_oracle.py), so the per-logit division
+// is a multiplication.
 template <int D>
-__global__ void __launch_bounds__(256)
+__device__ __forceinline__ constexpr float inv_sqrt_d() { return D == 64 ? 0.125f : 0.08838834764831845f; }
+
+constexpr int kScoreThreads = 64;                // a thread owns two keys
+constexpr int kScoreKeys = 2 * kScoreThreads;    // keys per block
+constexpr int kQGroup = 8;                       // window queries in flight: four packed pairs
+
+template <int D>
+constexpr size_t scores_smem_bytes(int w) {
+  return (size_t)kScoreKeys * (D * 2 + 16) + (size_t)((w + kQGroup - 1) / kQGroup) * D * kQGroup * 4;
+}
+
+// Bound by the fp32 pipe: the summation order of a logit is part of the result (its bf16 rounding decides which keys
+// stay), so the products stay on packed fp32 multiply-adds: D/8 partial sums of 8 consecutive elements, each added up
+// in ascending order, then a pairwise tree over the partial sums p and p + D/16, p + D/32, ...  A thread owns two
+// whole keys and a group of 8 queries, so that one 16-byte shared-memory read of queries feeds four packed
+// multiply-adds; the tree is walked in the order that closes its pairs at once (a binary counter), which keeps at most
+// log2(D/8) + 1 partial sums per logit alive.  Nothing crosses lanes.  32 heads x 6425
+// keys x 16 queries, D = 128: 43 us; 103 us with a key shared by as many lanes as it has 16-byte pieces, which
+// spends four shuffles and sixteen lanes' rounding arithmetic on every logit.
+template <int D>
+__global__ void __launch_bounds__(kScoreThreads, 5)
 scalekv_scores_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
                       const int32_t* __restrict__ window, float* __restrict__ scores, int H, int Lq, int Lkv,
                       int64_t q_sb, int64_t q_sh, int64_t q_sl, int64_t k_sb, int64_t k_sh, int64_t k_sl, int w,
-                      int offset, float sqrt_d) {
-  constexpr int LPK = D / 8;        // lanes per key
-  constexpr int KPP = 32 / LPK;     // keys per warp pass
-  __shared__ __align__(16) __nv_bfloat16 wq[kMaxWindow * D];
+                      int offset) {
+  constexpr int NP = D / 8;             // 16-byte pieces of a row = leaves of the summation tree
+  constexpr int LEVELS = D == 128 ? 4 : 3;
+  constexpr int ROW = D * 2 + 16;       // bytes of a staged key row: 16-byte reads of neighbouring rows hit all banks
+  extern __shared__ __align__(16) uint8_t sh_keys[];
+  float* qf = reinterpret_cast<float*>(sh_keys + kScoreKeys * ROW);  // [query group][D][8] fp32, zeros past w
   __shared__ int wcol[kMaxWindow];
   const int bh = blockIdx.y, b = bh / H, h = bh % H;
   const __nv_bfloat16* qb = q + b * q_sb + h * q_sh;
   const __nv_bfloat16* kb = k + b * k_sb + h * k_sh;
+  const int j0 = blockIdx.x * kScoreKeys;
+  for (int t = threadIdx.x; t < kScoreKeys * NP; t += kScoreThreads) {
+    const int r = t / NP, c = t % NP;
+    const int j = min(j0 + r, Lkv - 1);
+    cp_async_16(smem_u32(sh_keys + r * ROW + c * 16), kb + (int64_t)j * k_sl + c * 8);
+  }
+  cp_async_commit();
   // the window queries: query row clamp(window[i] - offset, 0, Lq - 1)
-  for (int t = threadIdx.x; t < w * (D / 8); t += blockDim.x) {
-    const int i = t / (D / 8), c = t % (D / 8);
-    const int row = min(max(window[i] - offset, 0), Lq - 1);
-    reinterpret_cast<uint4*>(wq)[i * (D / 8) + c] = *reinterpret_cast<const uint4*>(qb + (int64_t)row * q_sl + c * 8);
+  const int groups = (w + kQGroup - 1) / kQGroup;
+  for (int t = threadIdx.x; t < groups * kQGroup * NP; t += kScoreThreads) {
+    const int i = t % (groups * kQGroup), c = t / (groups * kQGroup);
+    uint4 raw = make_uint4(0, 0, 0, 0);
+    if (i < w) {
+      const int row = min(max(window[i] - offset, 0), Lq - 1);
+      raw = *reinterpret_cast<const uint4*>(qb + (int64_t)row * q_sl + c * 8);
+    }
+    const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
+    float* dst = qf + ((i / kQGroup) * D + c * 8) * kQGroup + i % kQGroup;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      dst[(2 * e) * kQGroup] = __uint_as_float(u[e] << 16);
+      dst[(2 * e + 1) * kQGroup] = __uint_as_float(u[e] & 0xffff0000u);
+    }
   }
   if (threadIdx.x < w) wcol[threadIdx.x] = window[threadIdx.x];
+  cp_async_wait<0>();
   __syncthreads();
 
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int sub = lane / LPK, piece = lane % LPK;
-  const int keys_per_block = nwarps * KPP;
-  for (int j0 = blockIdx.x * keys_per_block; j0 < Lkv; j0 += gridDim.x * keys_per_block) {
-    const int j = j0 + warp * KPP + sub;
-    float kf[8];
-    if (j < Lkv) {
-      const uint4 raw = *reinterpret_cast<const uint4*>(kb + (int64_t)j * k_sl + piece * 8);
-      const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
+  float total[2] = {0.f, 0.f};
+  for (int g = 0; g < groups; ++g) {
+    uint64_t stack[LEVELS + 1][2][4];  // [tree level][key][query pair]; compile-time indices only
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        kf[2 * e] = __uint_as_float(u[e] << 16);
-        kf[2 * e + 1] = __uint_as_float(u[e] & 0xffff0000u);
+    for (int n = 0; n < NP; ++n) {
+      // leaf n of the walk is the piece whose number is n with its bits reversed
+      int piece = 0;
+#pragma unroll
+      for (int bit = 0; bit < LEVELS; ++bit) piece |= ((n >> bit) & 1) << (LEVELS - 1 - bit);
+      asm volatile("" ::: "memory");  // a piece's shared-memory reads stay with it: hoisted, they would spill
+      uint64_t acc[2][4];
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y) acc[x][y] = 0ull;
+      uint32_t ku[2][4];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(sh_keys + (threadIdx.x + x * kScoreThreads) * ROW + piece * 16);
+        ku[x][0] = raw.x; ku[x][1] = raw.y; ku[x][2] = raw.z; ku[x][3] = raw.w;
       }
-    } else {
+      const ulonglong2* qp = reinterpret_cast<const ulonglong2*>(qf + (g * D + piece * 8) * kQGroup);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) kf[e] = 0.f;
-    }
-    float total = 0.f;
-    for (int i = 0; i < w; ++i) {
-      const uint4 raw = reinterpret_cast<const uint4*>(wq)[i * (D / 8) + piece];
-      const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
-      float dot = 0.f;
+      for (int d = 0; d < 8; ++d) {
+        const ulonglong2 qa = qp[2 * d], qc = qp[2 * d + 1];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        dot = fmaf(__uint_as_float(u[e] << 16), kf[2 * e], dot);
-        dot = fmaf(__uint_as_float(u[e] & 0xffff0000u), kf[2 * e + 1], dot);
+        for (int x = 0; x < 2; ++x) {
+          const uint32_t u = ku[x][d >> 1];
+          const float kv = __uint_as_float((d & 1) ? (u & 0xffff0000u) : (u << 16));
+          const uint64_t kk = pack_f32x2(kv, kv);
+          acc[x][0] = ffma2(qa.x, kk, acc[x][0]);
+          acc[x][1] = ffma2(qa.y, kk, acc[x][1]);
+          acc[x][2] = ffma2(qc.x, kk, acc[x][2]);
+          acc[x][3] = ffma2(qc.y, kk, acc[x][3]);
+        }
       }
+      // binary counter: every trailing one bit of n closes a pair of the tree
 #pragma unroll
-      for (int d = LPK / 2; d >= 1; d >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, d);
-      // logit rounded to bf16 (matmul output), divided by sqrt(D) in fp32 and rounded again (bf16 / scalar)
-      total += bf16_round(bf16_round(dot) / sqrt_d);
+      for (int lev = 0; lev <= LEVELS; ++lev) {
+        if (((n + 1) & ((1 << lev) - 1)) != 0) break;
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+          for (int y = 0; y < 4; ++y) {
+            if (lev > 0) acc[x][y] = fadd2(stack[lev - 1][x][y], acc[x][y]);
+          }
+        if (((n >> lev) & 1) == 0) {
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int y = 0; y < 4; ++y) stack[lev][x][y] = acc[x][y];
+        }
+      }
     }
-    if (piece == 0 && j < Lkv) {
-      bool in_window = false;
-      for (int i = 0; i < w; ++i) in_window |= (wcol[i] == j);
-      scores[(int64_t)bh * Lkv + j] = in_window ? -INFINITY : bf16_round(total);
-    }
+    // the closed tree: logit rounded to bf16 (matmul output), divided by sqrt(D) and rounded again (bf16 / scalar)
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        float lo, hi;
+        unpack_f32x2(stack[LEVELS][x][y], lo, hi);
+        if (g * kQGroup + 2 * y < w) total[x] += bf16_round(bf16_round(lo) * inv_sqrt_d<D>());
+        if (g * kQGroup + 2 * y + 1 < w) total[x] += bf16_round(bf16_round(hi) * inv_sqrt_d<D>());
+      }
+  }
+#pragma unroll
+  for (int x = 0; x < 2; ++x) {
+    const int j = j0 + threadIdx.x + x * kScoreThreads;
+    if (j >= Lkv) continue;
+    bool in_window = false;
+    for (int i = 0; i < w; ++i) in_window |= (wcol[i] == j);
+    scores[(int64_t)bh * Lkv + j] = in_window ? -INFINITY : bf16_round(total[x]);
   }
 }
 
@@ -140,19 +218,19 @@ int launch_scalekv_scores(const void* q, const void* k, const int32_t* window, f
   for (int64_t s : strides)
     LVAR_REQUIRE(s % 8 == 0 && s >= 0, LVAR_ERR_ARG, "tensor strides must be non-negative multiples of 8 elements");
   LVAR_REQUIRE((int64_t)B * H <= 65535, LVAR_ERR_UNSUPPORTED, "B*H must be <= 65535");
-  const int keys_per_block = 8 * (32 / (D / 8));
-  int bx = (Lkv + keys_per_block - 1) / keys_per_block;
-  if (bx > 148 * 4) bx = 148 * 4;
-  dim3 grid((unsigned)bx, (unsigned)(B * H));
-  const float sqrt_d = sqrtf((float)D);
+  dim3 grid((unsigned)((Lkv + kScoreKeys - 1) / kScoreKeys), (unsigned)(B * H));
   const auto* qp = static_cast<const __nv_bfloat16*>(q);
   const auto* kp = static_cast<const __nv_bfloat16*>(k);
-  if (D == 128)
-    scalekv_scores_kernel<128><<<grid, 256, 0, stream>>>(qp, kp, window, scores, H, Lq, Lkv, q_sb, q_sh, q_sl, k_sb, k_sh,
-                                                         k_sl, w, offset, sqrt_d);
-  else
-    scalekv_scores_kernel<64><<<grid, 256, 0, stream>>>(qp, kp, window, scores, H, Lq, Lkv, q_sb, q_sh, q_sl, k_sb, k_sh,
-                                                        k_sl, w, offset, sqrt_d);
+  const size_t smem = D == 128 ? scores_smem_bytes<128>(w) : scores_smem_bytes<64>(w);
+  if (D == 128) {
+    LVAR_CUDA_OK(cudaFuncSetAttribute(scalekv_scores_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)scores_smem_bytes<128>(kMaxWindow)));
+    scalekv_scores_kernel<128><<<grid, kScoreThreads, smem, stream>>>(qp, kp, window, scores, H, Lq, Lkv, q_sb, q_sh, q_sl,
+                                                                      k_sb, k_sh, k_sl, w, offset);
+  } else {
+    scalekv_scores_kernel<64><<<grid, kScoreThreads, smem, stream>>>(qp, kp, window, scores, H, Lq, Lkv, q_sb, q_sh, q_sl,
+                                                                     k_sb, k_sh, k_sl, w, offset);
+  }
   LVAR_CUDA_OK(cudaGetLastError());
   return LVAR_OK;
 }

@@ -79,3 +79,34 @@ def test_scalekv_argument_errors(K):
         K.scalekv_scores(q, q, w, 0)
     with pytest.raises(RuntimeError, match="bfloat16"):
         K.scalekv_scores(q.float(), q, w[:4], 0)
+
+
+@pytest.mark.parametrize("D,Lkv,w", [(128, 1, 1), (128, 128, 16), (128, 129, 7), (128, 6425, 16), (64, 127, 8), (64, 700, 64),
+                                     (128, 300, 64), (64, 257, 9)])
+def test_scores_bits_follow_the_stated_order(K, D, Lkv, w):
+    """The order of a logit's sum is fixed: D/8 sums of 8 consecutive products, then pairs p and p + D/16, p + D/32, ...
+    Products of bf16 numbers are exact in fp32, so plain fp32 arithmetic restates it bit for bit."""
+    g = torch.Generator().manual_seed(Lkv + w)
+    B, H, Lq = 1, 3, max(w, min(Lkv, 100))
+    q = torch.randn(B, H, Lq, D, generator=g).bfloat16().cuda()
+    kbig = torch.randn(B, H, Lkv, 2 * D, generator=g).bfloat16().cuda()
+    k = kbig[..., D:]                                    # rows of a wider buffer
+    window = torch.randperm(max(Lkv, w), generator=g)[:w].sort().values.to(torch.int32).cuda()
+    offset = Lkv - Lq
+    got = K.scalekv_scores(q, k, window, offset)
+    wq = q[:, :, (window.long() - offset).clamp(0, Lq - 1)].float()
+    prod = (wq.unsqueeze(3) * k.float().unsqueeze(2)).view(B, H, w, Lkv, D // 8, 8)
+    part = torch.zeros_like(prod[..., 0])
+    for e in range(8):
+        part = part + prod[..., e]
+    while part.shape[-1] > 1:
+        half = part.shape[-1] // 2
+        part = part[..., :half] + part[..., half:]
+    logit = (part[..., 0].bfloat16().float() / torch.tensor(float(D)).sqrt().cuda()).bfloat16().float()
+    total = torch.zeros(B, H, Lkv, device="cuda")
+    for i in range(w):
+        total = total + logit[:, :, i]
+    total = total.bfloat16().float()
+    inside = window[window < Lkv].long()
+    total[..., inside] = float("-inf")
+    assert torch.equal(got, total)

@@ -66,3 +66,13 @@ def test_host_mirror_agrees_with_oracle():
         sk.ScaleKVCluster([], layer_idx=0)
     with pytest.raises(ValueError):
         sk.ScaleKVCluster([[1]], pooling="median")
+
+
+def test_reciprocal_of_sqrt_d_rounds_like_the_quotient():
+    """The device multiplies a bf16 logit by 1/sqrt(D); every bf16 value gives the bf16 value of the quotient."""
+    x = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).float()
+    x = x[~torch.isnan(x)]
+    for D, inv in ((64, 0.125), (128, 0.08838834764831845)):
+        root = torch.tensor(D, dtype=torch.float32).sqrt()
+        r = torch.tensor(inv, dtype=torch.float32)
+        assert torch.equal((x / root).bfloat16().view(torch.int16), (x * r).bfloat16().view(torch.int16))
