@@ -93,8 +93,9 @@ typedef struct lvar_attn_args {
    * Lq).  work_order (optional, device int32[B * H * pairs per head]) is a permutation of the pair ids: the
    * pair at position i is handed out i-th, e.g. heaviest first for a ragged block mask.  When the last wave
    * of pairs fills at most half of the SMs, the pairs at the END of the order are handed out as single
-   * tiles; dense and block-sparse attention run such a tile on both halves of the CTA, each half taking
-   * half of the tile's KV blocks, and merge the two partial results in the epilogue. */
+   * tiles; such a tile runs on both halves of the CTA, each half taking half of the tile's KV blocks, and
+   * the two partial results are merged (lvar_dense_colsum_attn and lvar_colsum_tiles without given
+   * statistics: only when there is more than one wave of pairs). */
   int32_t* sched_scratch;
   const int32_t* work_order;
   /* plumbing */

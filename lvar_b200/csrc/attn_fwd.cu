@@ -167,6 +167,7 @@ struct Bars {
   SchedEntry sched[kSchedStages];
   uint32_t tmem_base;
   int abort_flag;
+  uint64_t xchg_back;  // split tile, column-sum sweep to follow: slot 1's merged row constants are in place (128 arrivals)
 };
 static_assert(sizeof(Bars) <= 512, "barrier block too large");
 
@@ -230,6 +231,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     mbar_init(&bars->mma_done, 1);
     mbar_init(&bars->xchg_full[0], 128);
     mbar_init(&bars->xchg_full[1], 128);
+    if (kHasCs) mbar_init(&bars->xchg_back, 128);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&bars->part_full[s][0], 128);
       mbar_init(&bars->part_full[s][1], 128);
@@ -338,6 +340,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     int n_o = 0;  // items in which this slot produced an output (parity of o_full)
     int n_cs[2] = {0, 0};  // column-sum sweep: S^T tiles read per buffer (parity of cs_full)
     int n_xc[2] = {0, 0};  // split tiles merged so far, by item parity (parity of xchg_full)
+    int n_back = 0;        // split tiles whose constants came back (parity of xchg_back)
     int n_part[2] = {0, 0};  // MODE_DENSE_CS1: tiles reduced per buffer (parity of part_full)
     int n_rowl = 0;          // MODE_DENSE_CS1: items with tiles (parity of rowl_full)
     bool ok = true;
@@ -353,6 +356,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const int cnt_total = (MODE == MODE_CSP) ? e.aux : 0;
       const int n_mine = s == 0 ? e.n0 : e.n1;
 
+      // the keys from this slot's first KV tile on (slot 1 of a split tile starts in the middle of the list)
+      const int key0 = (MODE != MODE_BLOCK && s == 1) ? e.off1 * 128 : 0, n_keys = p.Lkv - key0;
       float m_ref = -INFINITY, m_true = -INFINITY, l = 0.f;
       int it = 0;
       if (MODE == MODE_DENSE_CS1 && n_mine > 0) {
@@ -379,7 +384,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         uint64_t rs2[4] = {0ull, 0ull, 0ull, 0ull};  // packed partial sums of p over this thread's columns, per row
         const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2);
         const int tile = im.row0[s] >> 7;
-        float* cs_row = p.cs + im.b * p.cs_sb + im.h * p.cs_sh + (int64_t)(p.cs_pair ? tile >> 1 : tile) * p.cs_st;
+        float* cs_row = p.cs + im.b * p.cs_sb + im.h * p.cs_sh + (int64_t)(p.cs_pair ? tile >> 1 : tile) * p.cs_st + key0;
         const uint32_t b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
         const int col0 = 8 * ((b4 ? 8 : 0) + (b3 ? 4 : 0) + (b2 ? 2 : 0)) + 2 * tc;  // this thread's first result column
         for (int j = 0; j < n_mine; ++j) {
@@ -391,7 +396,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tmem_ld_16x256b_x16(tS, ra);
           tmem_ld_16x256b_x16(tS + (16u << 16), rb);
           tmem_wait_ld();
-          const int valid = p.Lkv - j * 128;
+          const int valid = n_keys - j * 128;
           uint64_t acc2[16];
           auto half_tile = [&](const uint32_t (&r)[64], int h, auto masked_tag) {
             constexpr bool MASKED = decltype(masked_tag)::value;
@@ -455,7 +460,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           const float* pr = part + (s * 2 + buf) * 4 * 128 + r_in_tile;
           const float colsum = ((pr[0] + pr[128]) + pr[256]) + pr[384];
           const int key = j * 128 + r_in_tile;
-          if (key < p.Lkv) {
+          if (key < n_keys) {
             if (p.cs_pair) atomicAdd(cs_row + key, colsum);  // two addends onto zero: the same bits in either order
             else cs_row[key] = colsum;
           }
@@ -589,7 +594,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (!ok) break;
 
       // ---- epilogue: O / l -> bf16 -> global; row statistics
-      const bool split = (MODE == MODE_DENSE || MODE == MODE_BLOCK) && im.split;
+      const bool split = MODE != MODE_CSP && im.split;
       float m_stat = m_true, l_stat = (it > 0 && l > 0.f) ? l * fast_exp2(m_ref - m_true) : 0.f;
       if (MODE == MODE_CSP && row_ok) {
         // Column-sparse: the epilogue adds this row of the accumulate input (or the four rows of the coarser grid
@@ -608,6 +613,33 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
           for (int b128 = 0; b128 < D * 2; b128 += 128)
             prefetch_l1(reinterpret_cast<const char*>(ib + (int64_t)row * p.oi_sl) + b128);
+        }
+      }
+      if (MODE == MODE_CS_ONLY && split && !stats_given) {
+        // The exchange below without an output: slot 1 hands its half's statistics to slot 0 and gets the row
+        // constants of the whole tile back.
+        float* x = xchg + (n & 1) * 3 * 128;
+        if (s == 1) {
+          x[r_in_tile] = (it > 0) ? m_ref : -INFINITY;
+          x[128 + r_in_tile] = (it > 0) ? l : 0.f;
+          x[256 + r_in_tile] = m_true;
+          mbar_arrive(&bars->xchg_full[n & 1]);
+        } else {
+          ok = __all_sync(0xffffffffu, mbar_wait(&bars->xchg_full[n & 1], n_xc[n & 1] & 1, wc, DEV_TIMEOUT_SOFTMAX));
+          if (!ok) break;
+          ++n_xc[n & 1];
+          const float m1 = x[r_in_tile], l1 = x[128 + r_in_tile];
+          const float mm = fmaxf(m_ref, m1);
+          const float a0 = (m_ref == -INFINITY) ? 0.f : fast_exp2(m_ref - mm);
+          const float a1 = (m1 == -INFINITY) ? 0.f : fast_exp2(m1 - mm);
+          l = a0 * l + a1 * l1;
+          m_ref = mm;
+          m_stat = fmaxf(m_true, x[256 + r_in_tile]);
+          l_stat = l > 0.f ? l * fast_exp2(mm - m_stat) : 0.f;
+          if (e.n1 > 0) {
+            negc[128 + r_in_tile] = (row_ok && l > 0.f) ? -(mm + log2f(l)) : -INFINITY;
+            mbar_arrive(&bars->xchg_back);
+          }
         }
       }
       if (MODE != MODE_CS_ONLY) {
@@ -647,6 +679,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             w1 = a1 * inv;
             m_stat = fmaxf(m_true, mt1);
             l_stat = lt > 0.f ? lt * fast_exp2(mm - m_stat) : 0.f;
+            if (kHasCs) {
+              // the column-sum sweep of both slots needs the merged constants; slot 1 gets its copy before this
+              // warpgroup goes on with the output
+              m_ref = mm;
+              l = lt;
+              if (other) {
+                negc[128 + r_in_tile] = (row_ok && lt > 0.f) ? -(mm + log2f(lt)) : -INFINITY;
+                mbar_arrive(&bars->xchg_back);
+              }
+            }
           }
           const uint32_t tO1 = tmem_base + lane_off + TM_O + (uint32_t)D;  // slot 1's accumulator (split tiles)
           __nv_bfloat16* orow = p.o + im.b * p.o_sb + im.h * p.o_sh + (int64_t)row * p.o_sl;
@@ -784,10 +826,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       } else if (MODE == MODE_DENSE_CS1) {
         // statistics out: the given pair with L corrected by the measured row sum, so that 2^M * L is this
         // attention's true normaliser even when the given constants were another pass's
-        if (row_ok && p.L) {
+        if (row_ok && p.L && !(split && s == 1)) {
           const int64_t si = (int64_t)im.bh * p.Lq + row;
           if (p.M) p.M[si] = p.M_in[si];
-          p.L[si] = p.L_in[si] * l;
+          p.L[si] = p.L_in[si] * (split ? l_stat : l);
         }
       } else if (row_ok && MODE != MODE_CSP && !(split && s == 1)) {
         const int64_t si = (int64_t)im.bh * p.Lq + row;
@@ -798,14 +840,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         // ---- second sweep: column sums of this slot's query tile.  S^T = K Q^T lands in S_s with one KEY per
         // TMEM lane, so this thread owns key column j*128 + r_in_tile and sums the 128 probabilities
         // p_i = exp2(s_i * scale - (M_i + log2 L_i)) of the tile's queries in registers.
-        negc[s * 128 + r_in_tile] = (row_ok && l > 0.f) ? -(m_ref + log2f(l)) : -INFINITY;
-        wg_sync(s);  // the warpgroup's 128 constants are in place
+        // A split tile's sweep covers this slot's KV tiles only; slot 0 has written slot 1's constants.
+        if (split && s == 1 && !stats_given) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&bars->xchg_back, n_back & 1, wc, DEV_TIMEOUT_SOFTMAX));
+          if (!ok) break;
+          ++n_back;
+        } else {
+          negc[s * 128 + r_in_tile] = (row_ok && l > 0.f) ? -(m_ref + log2f(l)) : -INFINITY;
+          wg_sync(s);  // the warpgroup's 128 constants are in place
+        }
         const float4* nc4 = reinterpret_cast<const float4*>(negc + s * 128);
         // a tile with fewer than 128 queries carries -inf constants, which the polynomial cannot take
         const bool full_tile = im.row_end[s] - im.row0[s] >= 128;
         const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2);
         const int tile = im.row0[s] >> 7;
-        float* cs_row = p.cs + im.b * p.cs_sb + im.h * p.cs_sh + (int64_t)(p.cs_pair ? tile >> 1 : tile) * p.cs_st;
+        float* cs_row = p.cs + im.b * p.cs_sb + im.h * p.cs_sh + (int64_t)(p.cs_pair ? tile >> 1 : tile) * p.cs_st + key0;
         // the sweep over the KV tiles, compiled twice: the exponential mix is a compile-time choice (a run-time
         // choice per chunk measured 20 % slower)
         auto cs_sweep = [&](auto poly_tag) -> bool {
@@ -830,7 +879,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             tc_fence_before();
             mbar_arrive(&bars->cs_empty[s][buf]);
             const int key = j * 128 + r_in_tile;
-            if (key < p.Lkv) {
+            if (key < n_keys) {
               // two addends onto zero give the same bits in either order
               if (p.cs_pair) atomicAdd(cs_row + key, acc);
               else cs_row[key] = acc;
@@ -1158,6 +1207,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                   if (t == s || D == 64) ok = mbar_wait(&bars->o_empty[t], (n_o[t] & 1) ^ 1, wc, DEV_TIMEOUT_MMA);
                 if (!ok) break;
               }
+              if (s == 1 && im.split) {  // the slots of a split tile have a K tile each
+                ks = kc % kStages;
+                kp = (kc / kStages) & 1;
+                ++kc;
+                waited = false;
+              }
               if (!waited) {
                 ok = mbar_wait(&bars->k_full[ks], kp, wc, DEV_TIMEOUT_MMA);
                 if (!ok) break;
@@ -1173,7 +1228,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               }
               umma_commit_if(leader, &bars->cs_full[s][buf]);
               ++n_cst[s][buf];
-              if (s == 1 || !cur.has[1]) umma_commit_if(leader, &bars->k_empty[ks]);  // last reader of the K stage
+              if (s == 1 || !cur.has[1] || im.split) umma_commit_if(leader, &bars->k_empty[ks]);  // last reader of the K stage
             }
           }
           // the next item's attention sweep writes S_s and O_s again: the softmax warps' last reads first
@@ -1517,18 +1572,32 @@ int launch_attention(const lvar_attn_args* a, int mode, cudaStream_t stream) {
   LVAR_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   p.n_pair_items = (int)total;
   p.total_items = (int)total;
-  // A single tile of the attention modes runs on both slots, each taking half of the tile's KV list
-  // (see the kernel's decode); the column-sum modes keep one slot idle instead.
-  p.split_singles = ((mode == MODE_DENSE || mode == MODE_BLOCK) && !(a->sched_flags & LVAR_SCHED_SINGLE_ONE_SLOT)) ? 1 : 0;
+  // A single tile runs on both slots, each taking half of the tile's KV list (see the kernel's decode).  The modes that
+  // take statistics for a column-sum sweep of their own do so only when there is more than one wave of pairs: within
+  // one wave their output stays the bits of the dense kernel's one-slot schedule.
+  const bool sums = mode == MODE_DENSE_CS || (mode == MODE_CS_ONLY && !stats_given);
+  p.split_singles = (mode != MODE_CSP && !(a->sched_flags & LVAR_SCHED_SINGLE_ONE_SLOT) && (!sums || total > sms)) ? 1 : 0;
   if (mode != MODE_CSP && (total > sms || p.split_singles) && !(a->sched_flags & LVAR_SCHED_PAIRS_ONLY)) {
-    // Wave quantisation: the pairs left over after the last full wave of CTAs are handed out as single
-    // query tiles when those fit in one wave, so that the tail costs one short item per CTA instead of
-    // one full pair on a few CTAs.  With work_order the tail is the end of the caller's order.
-    const int64_t rem = total % sms;
-    if (rem > 0 && 2 * rem <= sms) {
-      p.n_pair_items = (int)(total - rem);
-      p.total_items = (int)(total + rem);
+    // Wave quantisation: the query tiles left over after the last full wave of CTAs are handed out as single tiles
+    // when those fit in one wave, so that the tail costs one short item per CTA instead of one full pair on a few CTAs.
+    // With work_order the tail is the end of the caller's order.  A split tile takes 0.62 of a pair's time (52 against
+    // 82 us for one wave at 33 KV tiles); left with one half of the CTA idle it takes all of it, since a slot's chain of
+    // dependent steps per KV tile is the same.  Column sums with an output, 4096 x 10521 x 32: 1.15 -> 1.08 ms, without
+    // 0.91 -> 0.88 ms, one sweep on 1000 x 2999 x 16 (64 pairs on 148 SMs) 63 -> 42 us; block-sparse on 1600 x 4121 x
+    // 32, whose heads end in half a pair: 46 -> 42 us.
+    int64_t singles = 0;  // pairs at the end of the order that are handed out as single tiles
+    if (p.split_singles) {
+      // counted in tiles: the last pair of a head with an odd number of tiles is half a pair's work
+      const int64_t per_head = (a->Lq + 127) / 128, left = per_head * a->B * a->H % (2 * sms);
+      if (left > 0 && left <= sms) {
+        const int64_t part = left % per_head, odd = per_head & 1;
+        singles = left / per_head * p.n_x + (part ? odd + (part - odd + 1) / 2 : 0);
+      }
+    } else if (2 * (total % sms) <= sms) {
+      singles = total % sms;
     }
+    p.n_pair_items = (int)(total - singles);
+    p.total_items = (int)(total + singles);
   }
   dim3 grid((unsigned)(p.total_items < sms ? p.total_items : sms), 1, 1);
 

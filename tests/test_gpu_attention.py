@@ -744,3 +744,31 @@ def test_overlapped_launches_keep_stream_order_for_data(K):
         torch.cuda.synchronize()
         return outs[-1]
     assert torch.equal(chain2(0), chain2(_lib.SCHED_SERIALIZE_LAUNCH))
+
+
+@pytest.mark.parametrize("B,H,Lq,Lkv,D", [(2, 40, 640, 300, 128), (1, 75, 300, 100, 64), (1, 150, 129, 129, 64),
+                                          (2, 37, 384, 257, 128), (1, 50, 641, 520, 128), (1, 2, 300, 130, 128), (1, 3, 129, 90, 64)])
+def test_column_sum_modes_with_split_tiles(K, B, H, Lq, Lkv, D):
+    """More than one wave of work items: the last tiles run on both halves of a CTA, each with its own part of the KV
+    list (odd and even tile counts per head, one KV tile only, ragged last tiles).  The modes with and without an
+    output agree bit for bit, and with the one-half schedule and the stand-alone kernel to rounding.  The one-sweep mode
+    splits within one wave too (last two shapes)."""
+    q, k, v = (t.cuda() for t in _qkv(B, H, Lq, Lkv, D, seed=Lq + H, peaked=True))
+    st = K.new_status("cuda")
+    o, cs, M, L = K.dense_colsum_attn_fwd(q, k, v, return_stats=True, status=st)
+    dense, M0, L0 = K.dense_attn_fwd(q, k, v, sched_flags=SCHED_SINGLE_ONE_SLOT)
+    _same_to_rounding(o, dense)
+    # maxima are selections; denominators differ by the merge of two partial sums (a few roundings and exp2 errors)
+    assert torch.allclose(M, M0, rtol=1e-6, atol=1e-6) and torch.allclose(L, L0, rtol=1e-5)
+    sep = K.colsum_fwd(q, k, M0, L0, 128)
+    assert ((cs - sep).abs() <= 1e-5 * sep.abs().max()).all()
+    cs2, M2, L2 = K.colsum_tiles_fwd(q, k, return_stats=True, status=st)
+    assert torch.equal(cs2, cs) and torch.equal(M2, M) and torch.equal(L2, L)
+    cs3 = K.colsum_tiles_fwd(q, k, stats=(M0, L0), status=st)
+    assert ((cs3 - sep).abs() <= 1e-5 * sep.abs().max()).all()
+    o4, cs4, _, L4 = K.dense_colsum_attn_given_fwd(q, k, v, M0, L0, return_stats=True, status=st)
+    _same_to_rounding(o4, dense)
+    assert ((cs4 - sep).abs() <= 1e-4 * sep.abs() + 1e-30).all() and torch.allclose(L4, L0, rtol=2e-3)
+    _, pair = K.dense_colsum_attn_fwd(q, k, v, group_tiles=2, status=st)
+    assert torch.equal(pair, K.sum_tiles(cs, 2))
+    _ok_status(K, st)
