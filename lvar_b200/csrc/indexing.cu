@@ -181,56 +181,119 @@ block_mask_from_colsums_kernel(const float* __restrict__ cs, int64_t cs_row_stri
 // ------------------------------------------------------------------------------------------------
 // exact top-k
 // ------------------------------------------------------------------------------------------------
-constexpr int kTopkThreads = 1024;
 constexpr int kHistCopies = 8, kHistStride = 257;
+constexpr int kRankCap = 256;   // candidates that are ranked against each other instead of another histogram pass
+constexpr int kSortRun = 64;    // pairs a warp sorts in registers, two per lane
 
-// One CTA per row.  Shared: keys[n] | pairs[K2] (descending-value order only) | hist[8][257] | scan[64].
-__global__ void __launch_bounds__(kTopkThreads)
+// One merge step of the bitonic network on a run of 64 pairs held by a warp (element lane in x, lane + 32 in y): all
+// exchanges at distances first, first / 2, ..., 1.
+__device__ __forceinline__ void bitonic_run(unsigned long long& x, unsigned long long& y, int lane, int base, int size,
+                                            int first) {
+  for (int d = first; d >= 1; d >>= 1) {
+    if (d == 32) {
+      const bool desc = ((base + lane) & size) == 0;
+      if ((x < y) == desc) {
+        const unsigned long long t = x;
+        x = y;
+        y = t;
+      }
+    } else {
+      const bool low = (lane & d) == 0;
+      const unsigned long long ox = __shfl_xor_sync(0xffffffffu, x, d), oy = __shfl_xor_sync(0xffffffffu, y, d);
+      const bool dx = (((base + lane) & size) == 0) == low, dy = (((base + lane + 32) & size) == 0) == low;
+      x = dx ? (x > ox ? x : ox) : (x < ox ? x : ox);
+      y = dy ? (y > oy ? y : oy) : (y < oy ? y : oy);
+    }
+  }
+}
+
+// One CTA per row.  Shared: keys[n] | pairs[K2] (descending-value order only).
+// A row of a few thousand scores is bound by latency: block-wide steps (histogram passes, sorting steps) and the rows
+// in flight per SM, not by the 40 KB it reads.
+//  * Radix select starts below the leading bits that all keys share and stops as soon as the bin that holds the k-th
+//    largest key has few enough members to rank them against each other: one or two passes instead of four.
+//    Scores of one row share most of their leading bits (attention column sums span a few binades), so a pass puts
+//    most keys into a handful of bins: the histogram is kept in eight copies (one per lane modulo 8, 257 words apart so
+//    that equal bins of different copies sit in different banks), which cuts the serialisation of same-address atomics
+//    eightfold; the copies are added up when the bins are scanned.
+//  * Compaction by ballots over coalesced reads; a warp owns a contiguous range.
+//  * The sort of the descending order keeps the steps at distances up to 32 in a warp's registers: 28 block-wide steps
+//    for 4096 pairs instead of 78, 6 instead of 36 for 256.
+//  * 512 threads where the rows fill the chip (up to four rows per SM; 256 threads measured 10 to 20 % slower on long
+//    rows, 1024 leave one row per SM), 1024 for fewer rows.
+// rows x n, k: 224 x 4121, 256 descending 25.8 -> 15.1 us; 512 x 10521, 2176 descending 186 -> 135 us; 960 x 2500, 320
+// descending 94 -> 45 us; 32 x 10521, 1052 ascending 11.7 -> 10.8 us; 32 x 121, 12 ascending 6.1 -> 3.9 us (before: four
+// 8-bit passes always, every sorting step block-wide, 1024 threads always).
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == 512 ? 4 : 1)
 topk_kernel(const float* __restrict__ scores, int64_t row_stride, int n, int k, int ascending_index,
             int32_t* __restrict__ out, int64_t out_stride, int out_cols, int32_t* __restrict__ counts,
             int count_value, int K2) {
+  constexpr int WARPS = THREADS / 32;
   extern __shared__ __align__(16) uint8_t sh_raw[];
   uint32_t* keys = reinterpret_cast<uint32_t*>(sh_raw);
   unsigned long long* pairs = reinterpret_cast<unsigned long long*>(sh_raw + (((size_t)n * 4 + 15) & ~(size_t)15));
   __shared__ int hist[kHistCopies * kHistStride];
-  __shared__ int wsum_gt[32], wsum_eq[32];
+  __shared__ __align__(16) uint32_t cand[kRankCap];
+  __shared__ int wsum_gt[WARPS], wsum_eq[WARPS];
+  __shared__ uint32_t wmin[WARPS], wmax[WARPS];
   __shared__ uint32_t sh_prefix;
-  __shared__ int sh_remaining;
+  __shared__ int sh_remaining, sh_bin, n_cand;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t row = blockIdx.x;
   const float* src = scores + row * row_stride;
   int32_t* dst = out + row * out_stride;
 
-  for (int i = tid; i < n; i += kTopkThreads) keys[i] = ordered_key(src[i]);
-  if (tid == 0) {
-    sh_prefix = 0;
-    sh_remaining = k;
+  uint32_t kmin = 0xffffffffu, kmax = 0u;
+#pragma unroll 4
+  for (int i = tid; i < n; i += THREADS) {
+    const uint32_t key = ordered_key(src[i]);
+    keys[i] = key;
+    kmin = min(kmin, key);
+    kmax = max(kmax, key);
   }
-  __syncthreads();
+  // the tail of the output row: zeros, 16 bytes at a time from the first aligned column on
+  {
+    const int first = min(out_cols, k + (int)((4 - ((reinterpret_cast<uintptr_t>(dst + k) >> 2) & 3)) & 3));
+    const int quads = (out_cols - first) >> 2, rest = first + 4 * quads;
+    int4* d4 = reinterpret_cast<int4*>(dst + first);
+    for (int i = tid; i < quads; i += THREADS) d4[i] = make_int4(0, 0, 0, 0);
+    if (tid < first - k) dst[k + tid] = 0;
+    if (tid < out_cols - rest) dst[rest + tid] = 0;
+  }
+  if (counts != nullptr && tid == 0) counts[row] = count_value;
+  if (k <= 0) return;
 
-  if (k > 0) {
-    // radix select, most significant byte first: after 4 passes sh_prefix is the k-th largest key and
-    // sh_remaining the number of elements equal to it that belong to the selection.
-    // Scores of one row share most of their leading bits (attention column sums span a few binades), so most
-    // keys of a pass fall into a handful of histogram bins: the histogram is kept in eight copies (one per lane
-    // modulo 8, 257 words apart so that equal bins of different copies sit in different banks), which cuts the
-    // serialisation of same-address atomics eightfold; the copies are added up when the bins are scanned.
-    uint32_t maskbits = 0;
-    for (int pass = 3; pass >= 0; --pass) {
-      for (int i = tid; i < kHistCopies * kHistStride; i += kTopkThreads) hist[i] = 0;
-      __syncthreads();
-      const uint32_t prefix = sh_prefix;
-      const int shift = pass * 8;
+  kmin = __reduce_min_sync(0xffffffffu, kmin);
+  kmax = __reduce_max_sync(0xffffffffu, kmax);
+  if (lane == 0) {
+    wmin[warp] = kmin;
+    wmax[warp] = kmax;
+  }
+  for (int i = tid; i < kHistCopies * kHistStride; i += THREADS) hist[i] = 0;
+  __syncthreads();
+  kmin = __reduce_min_sync(0xffffffffu, wmin[lane & (WARPS - 1)]);
+  kmax = __reduce_max_sync(0xffffffffu, wmax[lane & (WARPS - 1)]);
+
+  uint32_t T = kmin;  // the k-th largest key
+  int need_eq = k;    // keys equal to it that belong to the selection
+  if (kmin != kmax) {
+    // digits of 8 bits, the first one right below the common leading bits
+    int top = 32 - __clz(kmin ^ kmax);          // bits [0, top) are still open
+    uint32_t prefix = top < 32 ? (kmin >> top) << top : 0u;
+    while (true) {
+      const int shift = max(0, top - 8);
+      const uint32_t dmask = (1u << (top - shift)) - 1u;
+      const uint32_t above = top < 32 ? ~0u << top : 0u;
       int* myhist = hist + (lane & (kHistCopies - 1)) * kHistStride;
-      for (int i = tid; i < n; i += kTopkThreads) {
+      for (int i = tid; i < n; i += THREADS) {
         const uint32_t key = keys[i];
-        if ((key & maskbits) == prefix) atomicAdd(&myhist[(key >> shift) & 255u], 1);
+        if ((key & above) == prefix) atomicAdd(&myhist[(key >> shift) & dmask], 1);
       }
       __syncthreads();
       if (warp == 0) {
-        // bins from the top: the bin that holds the rem-th largest candidate.  Lane l owns bins 8l .. 8l+7.
-        const int rem = sh_remaining;
+        // bins from the top: the bin that holds the need_eq-th largest candidate.  Lane l owns bins 8l .. 8l+7.
         int binc[8];  // this lane's eight bins, summed over the copies
         int own = 0;
 #pragma unroll
@@ -247,99 +310,155 @@ topk_kernel(const float* __restrict__ scores, int64_t row_stride, int n, int k, 
           const int t = __shfl_down_sync(0xffffffffu, suffix, d);
           if (lane + d < 32) suffix += t;
         }
-        const uint32_t reach = __ballot_sync(0xffffffffu, suffix >= rem);  // never empty: all candidates >= rem
+        const uint32_t reach = __ballot_sync(0xffffffffu, suffix >= need_eq);  // never empty: all candidates >= need_eq
         const int L = 31 - __clz(reach);
         if (lane == L) {
-          int r = rem - (suffix - own);  // still to find inside this lane's bins
-          int j = 7;
+          int r = need_eq - (suffix - own);  // still to find inside this lane's bins
+          int j = 7, size = binc[7];
 #pragma unroll
           for (int t = 7; t > 0; --t) {
             if (j == t && binc[t] < r) {
               r -= binc[t];
               j = t - 1;
+              size = binc[t - 1];
             }
           }
-          const int d = 8 * lane + j;
-          sh_prefix = prefix | ((uint32_t)d << shift);
+          sh_prefix = prefix | ((uint32_t)(8 * lane + j) << shift);
           sh_remaining = r;
+          sh_bin = size;
+          n_cand = 0;
         }
+      } else {
+        for (int i = tid - 32; i < kRankCap; i += THREADS - 32) cand[i] = 0u;
       }
-      maskbits |= 0xFFu << shift;
+      __syncthreads();
+      prefix = sh_prefix;
+      need_eq = sh_remaining;
+      top = shift;
+      const int size = sh_bin;
+      if (top == 0 || size == need_eq) break;
+      if (size <= kRankCap) break;
+      for (int i = tid; i < kHistCopies * kHistStride; i += THREADS) hist[i] = 0;
       __syncthreads();
     }
-  }
-  const uint32_t T = sh_prefix;
-  const int need_eq = (k > 0) ? sh_remaining : 0;
-
-  // ordered compaction: thread t owns the contiguous range [t*per, (t+1)*per)
-  const int per = (n + kTopkThreads - 1) / kTopkThreads;
-  const int lo = min(n, tid * per), hi = min(n, lo + per);
-  int gt = 0, eq = 0;
-  if (k > 0) {
-    for (int i = lo; i < hi; ++i) {
-      const uint32_t key = keys[i];
-      gt += key > T;
-      eq += key == T;
-    }
-  }
-  int gt_inc = warp_incl_scan(gt, lane), eq_inc = warp_incl_scan(eq, lane);
-  if (lane == 31) {
-    wsum_gt[warp] = gt_inc;
-    wsum_eq[warp] = eq_inc;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    int a = wsum_gt[lane], b = wsum_eq[lane];
-    const int ai = warp_incl_scan(a, lane), bi = warp_incl_scan(b, lane);
-    wsum_gt[lane] = ai - a;
-    wsum_eq[lane] = bi - b;
-  }
-  __syncthreads();
-  int gt_b = wsum_gt[warp] + gt_inc - gt;  // selected-by-value elements before this thread's range
-  int eq_b = wsum_eq[warp] + eq_inc - eq;  // elements equal to T before this thread's range
-  if (k > 0) {
-    for (int i = lo; i < hi; ++i) {
-      const uint32_t key = keys[i];
-      int pos = -1;
-      if (key > T) {
-        pos = gt_b + min(eq_b, need_eq);
-        ++gt_b;
-      } else if (key == T) {
-        if (eq_b < need_eq) pos = gt_b + eq_b;
-        ++eq_b;
-      }
-      if (pos >= 0) {
-        if (ascending_index) {
-          dst[pos] = i;
-        } else {
-          pairs[pos] = ((unsigned long long)key << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)i);
+    T = prefix;
+    if (top > 0) {
+      // the bin's members in shared memory, in any order: the k-th largest has fewer than need_eq greater ones and at
+      // least need_eq not smaller ones
+      const uint32_t above = ~0u << top;
+      const int size = sh_bin;
+      if (size > kRankCap) {
+        // all of a large bin is selected: its smallest member
+        uint32_t least = 0xffffffffu;
+        for (int i = tid; i < n; i += THREADS) {
+          const uint32_t key = keys[i];
+          if ((key & above) == prefix) least = min(least, key);
         }
-      }
-    }
-  }
-  if (!ascending_index && k > 0) {
-    for (int i = k + tid; i < K2; i += kTopkThreads) pairs[i] = 0ull;  // sorts last
-    __syncthreads();
-    // bitonic sort, descending on (key, ~index): equal keys come out in ascending index order
-    for (int size = 2; size <= K2; size <<= 1) {
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        for (int t = tid; t < (K2 >> 1); t += kTopkThreads) {
-          const int i = 2 * t - (t & (stride - 1));
-          const int j = i + stride;
-          const bool desc = ((i & size) == 0);
-          const unsigned long long a = pairs[i], b = pairs[j];
-          if ((a < b) == desc) {
-            pairs[i] = b;
-            pairs[j] = a;
+        least = __reduce_min_sync(0xffffffffu, least);
+        if (lane == 0) wmin[warp] = least;
+        __syncthreads();
+        T = __reduce_min_sync(0xffffffffu, wmin[lane & (WARPS - 1)]);
+        // how many equal ones: all of them
+        need_eq = n;
+      } else {
+        for (int i = tid; i < n; i += THREADS) {
+          const uint32_t key = keys[i];
+          if ((key & above) == prefix) cand[atomicAdd(&n_cand, 1)] = key;
+        }
+        __syncthreads();
+        if (tid < size) {
+          const uint32_t mine = cand[tid];
+          // four at a time; the zeros behind the last one are never greater, and equal only to the smallest key there
+          // is, for which the test below holds either way
+          int greater = 0, equal = 0;
+#pragma unroll 4
+          for (int i = 0; i < size; i += 4) {
+            const uint4 c = *reinterpret_cast<const uint4*>(cand + i);
+            greater += (c.x > mine) + (c.y > mine) + (c.z > mine) + (c.w > mine);
+            equal += (c.x == mine) + (c.y == mine) + (c.z == mine) + (c.w == mine);
+          }
+          if (greater < need_eq && greater + equal >= need_eq) {  // equal members write equal values
+            sh_prefix = mine;
+            sh_remaining = need_eq - greater;
           }
         }
         __syncthreads();
+        T = sh_prefix;
+        need_eq = sh_remaining;
       }
     }
-    for (int i = tid; i < k; i += kTopkThreads) dst[i] = (int32_t)(0xFFFFFFFFu - (uint32_t)(pairs[i] & 0xFFFFFFFFull));
   }
-  for (int i = k + tid; i < out_cols; i += kTopkThreads) dst[i] = 0;
-  if (counts != nullptr && tid == 0) counts[row] = count_value;
+
+  // ordered compaction: warp w owns the contiguous range [w*per, (w+1)*per), 32 keys at a time
+  const int per = (((n + 31) / 32 + WARPS - 1) / WARPS) * 32;
+  const int lo = min(n, warp * per), hi = min(n, lo + per);
+  int gt = 0, eq = 0;
+  for (int i = lo; i < hi; i += 32) {
+    const uint32_t key = i + lane < hi ? keys[i + lane] : 0u;
+    const bool in = i + lane < hi;
+    gt += __popc(__ballot_sync(0xffffffffu, in && key > T));
+    eq += __popc(__ballot_sync(0xffffffffu, in && key == T));
+  }
+  if (lane == 0) {
+    wsum_gt[warp] = gt;
+    wsum_eq[warp] = eq;
+  }
+  __syncthreads();
+  int gt_b = 0, eq_b = 0;  // keys above T / equal to T before this warp's range
+  {
+    const int a = lane < warp ? wsum_gt[lane & (WARPS - 1)] : 0, b = lane < warp ? wsum_eq[lane & (WARPS - 1)] : 0;
+    gt_b = __reduce_add_sync(0xffffffffu, a);
+    eq_b = __reduce_add_sync(0xffffffffu, b);
+  }
+  const uint32_t lt = (1u << lane) - 1u;
+  for (int i = lo; i < hi; i += 32) {
+    const bool in = i + lane < hi;
+    const uint32_t key = in ? keys[i + lane] : 0u;
+    const uint32_t vg = __ballot_sync(0xffffffffu, in && key > T), ve = __ballot_sync(0xffffffffu, in && key == T);
+    const int g_before = gt_b + __popc(vg & lt), e_before = eq_b + __popc(ve & lt);
+    if (in && (key > T || (key == T && e_before < need_eq))) {
+      const int pos = g_before + min(e_before, need_eq);
+      if (ascending_index) dst[pos] = i + lane;
+      else pairs[pos] = ((unsigned long long)key << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)(i + lane));
+    }
+    gt_b += __popc(vg);
+    eq_b += __popc(ve);
+  }
+  if (ascending_index) return;
+
+  for (int i = k + tid; i < K2; i += THREADS) pairs[i] = 0ull;  // sorts last
+  __syncthreads();
+  // bitonic sort, descending on (key, ~index): equal keys come out in ascending index order
+  for (int run = warp * kSortRun; run < K2; run += WARPS * kSortRun) {
+    unsigned long long x = pairs[run + lane], y = pairs[run + lane + 32];
+    for (int size = 2; size <= kSortRun; size <<= 1) bitonic_run(x, y, lane, run, size, size >> 1);
+    pairs[run + lane] = x;
+    pairs[run + lane + 32] = y;
+  }
+  for (int size = 2 * kSortRun; size <= K2; size <<= 1) {
+    __syncthreads();
+    for (int stride = size >> 1; stride >= kSortRun; stride >>= 1) {
+      for (int t = tid; t < (K2 >> 1); t += THREADS) {
+        const int i = 2 * t - (t & (stride - 1));
+        const int j = i + stride;
+        const bool desc = ((i & size) == 0);
+        const unsigned long long a = pairs[i], b = pairs[j];
+        if ((a < b) == desc) {
+          pairs[i] = b;
+          pairs[j] = a;
+        }
+      }
+      __syncthreads();
+    }
+    for (int run = warp * kSortRun; run < K2; run += WARPS * kSortRun) {
+      unsigned long long x = pairs[run + lane], y = pairs[run + lane + 32];
+      bitonic_run(x, y, lane, run, size, kSortRun >> 1);
+      pairs[run + lane] = x;
+      pairs[run + lane + 32] = y;
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < k; i += THREADS) dst[i] = (int32_t)(0xFFFFFFFFu - (uint32_t)(pairs[i] & 0xFFFFFFFFull));
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -506,17 +625,25 @@ int launch_topk(const float* scores, int64_t rows, int n, int64_t row_stride, in
   LVAR_REQUIRE(k >= 0 && k <= n, LVAR_ERR_ARG, "k must be in [0, n] (k=%d, n=%d)", k, n);
   LVAR_REQUIRE(out_cols >= k && out_stride >= out_cols, LVAR_ERR_ARG, "output row too short for k entries");
   LVAR_REQUIRE(rows < (1ll << 31), LVAR_ERR_LIMIT, "too many rows");
+  size_t smem = (((size_t)n * 4 + 15) & ~(size_t)15);
   int K2 = 0;
   if (!ascending_index && k > 0) {
     K2 = 2;
     while (K2 < k) K2 <<= 1;
+    LVAR_REQUIRE(smem + (size_t)K2 * 8 <= 200 * 1024, LVAR_ERR_LIMIT,
+                 "row of %d scores with k=%d needs %zu bytes of shared memory (limit 204800)", n, k, smem + (size_t)K2 * 8);
+    if (K2 < kSortRun) K2 = kSortRun;
   }
-  const size_t smem = (((size_t)n * 4 + 15) & ~(size_t)15) + (size_t)K2 * 8;
   LVAR_REQUIRE(smem <= 200 * 1024, LVAR_ERR_LIMIT,
                "row of %d scores with k=%d needs %zu bytes of shared memory (limit 204800)", n, k, smem);
-  LVAR_CUDA_OK(cudaFuncSetAttribute(topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  topk_kernel<<<(unsigned)rows, kTopkThreads, smem, stream>>>(scores, row_stride, n, k, ascending_index, out,
-                                                              out_stride, out_cols, counts, count_value, K2);
+  smem += (size_t)K2 * 8;
+  int dev = 0, sms = 0;
+  LVAR_CUDA_OK(cudaGetDevice(&dev));
+  LVAR_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  auto kern = rows > sms ? topk_kernel<512> : topk_kernel<1024>;
+  LVAR_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024 + kSortRun * 8));
+  kern<<<(unsigned)rows, rows > sms ? 512 : 1024, smem, stream>>>(scores, row_stride, n, k, ascending_index, out,
+                                                                  out_stride, out_cols, counts, count_value, K2);
   LVAR_CUDA_OK(cudaGetLastError());
   return LVAR_OK;
 }

@@ -466,7 +466,11 @@ def topk_indices(scores: torch.Tensor, k: int, *, ascending_index=False, out_col
     rows = flat.shape[0]
     cols = int(k if out_cols is None else out_cols)
     out = torch.empty((rows, cols), dtype=torch.int32, device=scores.device)
-    counts = torch.full((rows,), int(k), dtype=torch.int32, device=scores.device) if with_counts else None
+    # the kernel writes the counts; without output columns there is no launch
+    counts = None
+    if with_counts:
+        counts = (torch.empty((rows,), dtype=torch.int32, device=scores.device) if cols > 0 else
+                  torch.full((rows,), int(k), dtype=torch.int32, device=scores.device))
     if cols > 0:
         check(lib.lvar_topk_indices(flat.data_ptr(), rows, n, flat.stride(0), int(k),
                                     int(bool(ascending_index)),

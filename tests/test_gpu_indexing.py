@@ -219,3 +219,33 @@ def test_sparse_step_lists_row_edges(K, k_len, src_cols, cnt, band_count):
     src = inds.cuda()
     got, counts = K.sparse_step_lists(src, remap.cuda(), band.cuda() if band_count else None, cnt, k_len, count_value=9)
     assert torch.equal(got.cpu(), want) and (counts == 9).all()
+
+
+@pytest.mark.parametrize("rows", [3, 200])          # 1024 threads per row up to one row per SM, 512 beyond
+@pytest.mark.parametrize("n,k", [(1, 1), (31, 5), (33, 33), (64, 64), (65, 64), (127, 128 - 63), (513, 512), (1000, 1), (4121, 256),
+                                 (6001, 2049), (10521, 1052)])
+def test_topk_value_distributions(K, rows, n, k):
+    """Rows of one value, of few values (bins larger than the ranking step takes), of values in one binade, of all bit
+    patterns of numbers with infinities and both zeros, with a bin that is selected as a whole; strided rows, odd output
+    widths: against a stable sort of the keys."""
+    g = torch.Generator().manual_seed(n + k + rows)
+    s = torch.rand(rows, n, generator=g) + 1.0                                        # one binade
+    s[0] = 0.25                                                                       # one value
+    s[1] = torch.randint(0, 3, (n,), generator=g).float()                             # three values
+    bits = torch.randint(-2 ** 31, 2 ** 31, (n,), generator=g, dtype=torch.int64).to(torch.int32).view(torch.float32)
+    s[2] = torch.where(torch.isnan(bits), torch.ones_like(bits), bits)                # any number
+    s[2, : min(n, 4)] = torch.tensor([float("inf"), -float("inf"), -0.0, 0.0])[: min(n, 4)]
+    if rows > 4:
+        s[3] = 1.0 + (torch.arange(n) < k).float() * 2.0 ** -9 * (1 + torch.rand(n, generator=g))  # k above the rest
+        s[4] = torch.exp2(torch.randn(n, generator=g) * 10)
+    wide = torch.zeros(rows, n + 3)
+    wide[:, :n] = s
+    u = (s + 0.0).view(torch.int32).long() & 0xFFFFFFFF
+    key = torch.where(u >= 2 ** 31, (~u) & 0xFFFFFFFF, u | 2 ** 31)
+    order = torch.sort(key, dim=-1, descending=True, stable=True).indices[:, :k].int()
+    dev = wide.cuda()[:, :n]
+    for cols in (k, k + 1, k + 6):
+        got, counts = K.topk_indices(dev, k, out_cols=cols, with_counts=True)
+        assert torch.equal(got[:, :k].cpu(), order) and (got[:, k:] == 0).all() and (counts == k).all()
+        asc = K.topk_indices(dev, k, ascending_index=True, out_cols=cols)
+        assert torch.equal(asc[:, :k].cpu(), order.sort(-1).values) and (asc[:, k:] == 0).all()
