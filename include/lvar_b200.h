@@ -143,6 +143,11 @@ int lvar_dense_colsum_attn(const lvar_attn_args* args, lvar_stream_t stream);
  * dense_colsum_attn_s calls after dense_attn (kernels/sparse_attn/sparse_attn_ops.py:65-113). */
 int lvar_dense_colsum_attn_given(const lvar_attn_args* args, lvar_stream_t stream);
 
+/* The same with the normalisers in the reference operator's own form: args->M_in holds p_i = 1 / sum_j exp(s_ij) (fp32
+ * [B,H,Lq]; values below the smallest normal number count as that), args->L_in and args->M are not read, and args->L, when
+ * non-null, receives this attention's own p.  No launch before or after it to convert them. */
+int lvar_dense_colsum_attn_p(const lvar_attn_args* args, lvar_stream_t stream);
+
 /* The attention column sums alone, per 128-row query tile (cs as in lvar_dense_colsum_attn); v, o and their
  * strides are not read and may be null / 0.  stats_given = 0: one launch takes the row statistics in a first
  * sweep that does everything but P and PV (M and L are written when non-null) and the sums in a second one.

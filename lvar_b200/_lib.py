@@ -66,6 +66,7 @@ _SIGNATURES = {
     "lvar_dense_attn": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
     "lvar_dense_colsum_attn": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
     "lvar_dense_colsum_attn_given": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
+    "lvar_dense_colsum_attn_p": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
     "lvar_colsum_tiles": (C.c_int, [C.POINTER(AttnArgs), C.c_int32, C.c_void_p]),
     "lvar_block_sparse_attn": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
     "lvar_csp_attn": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),

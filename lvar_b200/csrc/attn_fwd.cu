@@ -26,6 +26,7 @@
 //
 // Every wait is bounded (ptx.cuh: mbar_wait); a wait that runs out records a status code, raises a
 // CTA-wide abort flag, lets the loaders drain their copies, frees TMEM and returns.
+#include <float.h>
 #include <math.h>
 
 #include <type_traits>
@@ -81,7 +82,8 @@ struct AttnParams {
   int64_t cs_sb, cs_sh, cs_st;
   int cs_pair;  // 1: the two 128-row tiles of a 256-row group add into ONE zero-initialised row of cs
   const float* M_in;  // MODE_CS_ONLY: row statistics supplied by the caller (both or neither); the
-  const float* L_in;  // statistics sweep is then skipped
+  const float* L_in;  // statistics sweep is then skipped.  MODE_DENSE_CS1: L_in null = M_in holds p = 1 / sum exp(s),
+                      // and L receives this attention's own p
   // block mask (MODE_BLOCK): uint8 [*,*,nqb,nkb], broadcast over batch/head when the stride is 0
   const uint8_t* mask;
   int64_t m_sb, m_sh, m_sq;
@@ -143,6 +145,9 @@ struct SchedEntry {
   int aux;   // csp: length of the item's index list
   int off1;  // dense, split tile: slot 1 starts at this KV tile (slot 0 takes the tiles before it)
 };
+
+// A supplied normaliser that underflowed counts as the smallest normal number; NaN stays NaN.
+__device__ __forceinline__ float at_least_tiny(float x) { return x < FLT_MIN ? FLT_MIN : x; }
 
 // One round of the two slots' tile streams: slot s works on KV tile kvb[s] if has[s]; when both want
 // the same tile it is loaded once and shared.
@@ -376,8 +381,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           float c = -INFINITY;
           if (rr < im.row_end[s]) {
             const int64_t si = (int64_t)im.bh * p.Lq + rr;
-            const float Lr = p.L_in[si];
-            if (Lr > 0.f) c = -(p.M_in[si] + log2f(Lr));
+            if (p.L_in == nullptr) {
+              c = log2f(at_least_tiny(p.M_in[si]));
+            } else {
+              const float Lr = p.L_in[si];
+              if (Lr > 0.f) c = -(p.M_in[si] + log2f(Lr));
+            }
           }
           ncst[i] = c;
         }
@@ -828,8 +837,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         // attention's true normaliser even when the given constants were another pass's
         if (row_ok && p.L && !(split && s == 1)) {
           const int64_t si = (int64_t)im.bh * p.Lq + row;
-          if (p.M) p.M[si] = p.M_in[si];
-          p.L[si] = p.L_in[si] * (split ? l_stat : l);
+          const float sum = split ? l_stat : l;
+          if (p.L_in == nullptr) {
+            p.L[si] = at_least_tiny(p.M_in[si]) / sum;
+          } else {
+            if (p.M) p.M[si] = p.M_in[si];
+            p.L[si] = p.L_in[si] * sum;
+          }
         }
       } else if (row_ok && MODE != MODE_CSP && !(split && s == 1)) {
         const int64_t si = (int64_t)im.bh * p.Lq + row;
@@ -1437,11 +1451,14 @@ int launch_d(int mode, const CUtensorMap& tq, const CUtensorMap& tk, const CUten
 }  // namespace
 
 // mode: an AttnMode, or MODE_CS_ONLY + 1 for the column sums from row statistics the caller supplies in
-// a->M / a->L.  MODE_DENSE_CS1 reads its row statistics from a->M_in / a->L_in.
+// a->M / a->L.  MODE_DENSE_CS1 reads its row statistics from a->M_in / a->L_in; MODE_DENSE_CS1 + 1 is the same from
+// p = 1 / sum exp(s) in a->M_in.
 int launch_attention(const lvar_attn_args* a, int mode, cudaStream_t stream) {
   LVAR_REQUIRE(a != nullptr, LVAR_ERR_ARG, "null argument block");
   const bool stats_given = mode == MODE_CS_ONLY + 1;
   if (stats_given) mode = MODE_CS_ONLY;
+  const bool p_given = mode == MODE_DENSE_CS1 + 1;
+  if (p_given) mode = MODE_DENSE_CS1;
   LVAR_REQUIRE(a->D == 64 || a->D == 128, LVAR_ERR_UNSUPPORTED, "Head dimension must be 64 or 128 (got %d)", a->D);
   LVAR_REQUIRE(a->B >= 1 && a->H >= 1 && a->Lq >= 1 && a->Lkv >= 1, LVAR_ERR_ARG,
                "B, H, Lq, Lkv must be >= 1 (got %d %d %d %d)", a->B, a->H, a->Lq, a->Lkv);
@@ -1482,11 +1499,11 @@ int launch_attention(const lvar_attn_args* a, int mode, cudaStream_t stream) {
     p.M = p.L = nullptr;
   }
   if (mode == MODE_DENSE_CS1) {
-    LVAR_REQUIRE(a->M_in && a->L_in, LVAR_ERR_ARG,
+    LVAR_REQUIRE(a->M_in && (a->L_in || p_given), LVAR_ERR_ARG,
                  "M_in and L_in (row statistics of this attention, fp32 [B,H,Lq]) must be non-null");
-    LVAR_REQUIRE((a->M == nullptr) == (a->L == nullptr), LVAR_ERR_ARG, "M and L (statistics out) go together");
+    LVAR_REQUIRE(p_given || (a->M == nullptr) == (a->L == nullptr), LVAR_ERR_ARG, "M and L (statistics out) go together");
     p.M_in = a->M_in;
-    p.L_in = a->L_in;
+    p.L_in = p_given ? nullptr : a->L_in;
   }
   if (mode == MODE_DENSE_CS || mode == MODE_CS_ONLY || mode == MODE_DENSE_CS1) {
     LVAR_REQUIRE(a->cs != nullptr, LVAR_ERR_ARG, "cs (column sums per 128-row query tile) is null");

@@ -265,3 +265,32 @@ def test_sparse_flex_attn_class(ops):
     mask = oi.csla_block_mask(sched, win, 4, 2, 128)
     assert torch.equal(mod.block_mask.cpu(), mask)
     assert (out.float().cpu() - oa.block_sparse_attn(q, k, v, mask, 0.125)).abs().max() <= 2e-2
+
+
+@pytest.mark.parametrize("B,H,Lq,Lkv,D", [(1, 2, 1, 130, 128), (1, 2, 300, 257, 64), (2, 80, 300, 129, 64), (1, 3, 1000, 520, 128)])
+def test_dense_colsum_attn_takes_p_as_it_is(B, H, Lq, Lkv, D):
+    """The operator's p = 1 / sum exp(s) goes into the kernel unconverted and this attention's own p comes out: against
+    the form with base-2 statistics, for p of other types and strides, underflowed (0), subnormal and NaN entries."""
+    import lvar_b200.torch_ops  # noqa: F401
+    from lvar_b200 import kernels as K
+    g = torch.Generator().manual_seed(Lq + Lkv)
+    q, k, v = (torch.randn(B, H, n, D, generator=g).bfloat16().cuda() for n in (Lq, Lkv, Lkv))
+    scale = D ** -0.5
+    _, M, L = K.dense_attn_fwd(q, k, v, scale)
+    p = (torch.exp2(-M) / L).unsqueeze(-1)
+    if Lq > 8:
+        p[0, 0, 3], p[0, 0, 4], p[0, 0, 5] = 0.0, 1e-40, float("nan")
+    tiny = torch.finfo(torch.float32).tiny
+    wide = torch.empty(B, H, Lq, 2, dtype=torch.float64, device="cuda")
+    wide[..., :1] = p
+    for given in (p, wide[..., :1], p.bfloat16()):
+        Mp = -torch.log2(given.reshape(B, H, Lq).float().clamp_min(tiny)).contiguous()
+        o0, cs0, M0, L0 = K.dense_colsum_attn_given_fwd(q, k, v, Mp, torch.ones_like(Mp), scale, return_stats=True,
+                                                        group_tiles=2)
+        o, cs, own = torch.ops.chipmunk.dense_colsum_attn_scaled(q, k, v, given, scale)
+        assert own.shape == (B, H, Lq, 1)
+        # log2 of p is taken by two implementations that may differ in the last bit of a value up to 2^7: 2^-17 in exp2
+        for a, b, tol in ((o.float(), o0.float(), 2.0 ** -7), (cs, cs0, 1e-4), (own[..., 0], torch.exp2(-M0) / L0, 1e-4)):
+            assert torch.equal(torch.isnan(a), torch.isnan(b))
+            a, b = a.nan_to_num(0.0, 0.0, 0.0), b.nan_to_num(0.0, 0.0, 0.0)
+            assert ((a - b).abs() <= tol * b.abs() + 1e-3 * tol).all()
