@@ -441,7 +441,9 @@ def build_block_mask(scores: torch.Tensor, always: Optional[torch.Tensor], k_tot
     a_ptr = None
     if always is not None:
         _require(always.is_cuda and tuple(always.shape) == (nq, nk), f"always must be a CUDA [{nq},{nk}] tensor")
-        always = always.to(torch.uint8).contiguous() if always.dtype != torch.uint8 else always.contiguous()
+        always = always.contiguous()
+        if always.dtype != torch.uint8:
+            always = always.view(torch.uint8) if always.dtype == torch.bool else always.to(torch.uint8)
         a_ptr = always.data_ptr()
     mask = torch.empty((B, H, nq, nk), dtype=torch.uint8, device=scores.device)
     lists = counts = None
@@ -470,7 +472,9 @@ def block_mask_from_colsums(cs: torch.Tensor, always: Optional[torch.Tensor], k_
     a_ptr = None
     if always is not None:
         _require(always.is_cuda and tuple(always.shape) == (G, nk), f"always must be a CUDA [{G},{nk}] tensor")
-        always = always.to(torch.uint8).contiguous() if always.dtype != torch.uint8 else always.contiguous()
+        always = always.contiguous()
+        if always.dtype != torch.uint8:
+            always = always.view(torch.uint8) if always.dtype == torch.bool else always.to(torch.uint8)
         a_ptr = always.data_ptr()
     mask = torch.empty((B, H, G, nk), dtype=torch.uint8, device=cs.device)
     scores = torch.empty((B, H, G, nk), dtype=torch.float32, device=cs.device) if return_scores else None
