@@ -12,7 +12,7 @@ from __future__ import annotations
 
 import math
 import warnings
-from typing import List, Sequence
+from typing import Dict, List, Sequence, Tuple
 
 import torch
 
@@ -37,6 +37,24 @@ def window_indices(current_scale_size: int, current_scale_start: int, key_len: i
             wc = max(0, min(side - 1, j * wp + (wp - 1) // 2))
             out.append(min(max(hc * side + wc + current_scale_start, 0), key_len - 1))
     return sorted(set(out))[:window_size]
+
+
+_WINDOWS: Dict[tuple, torch.Tensor] = {}
+
+
+def _window_on(win: Tuple[int, ...], device: torch.device) -> torch.Tensor:
+    """The window's key indices on the device.  The same few windows (one per scale) come back for every layer and image;
+    uploading them from pageable memory on each call stalled the host until the stream had drained.  Bounded, and never
+    dropped (a captured graph may read them); a tensor made during a capture belongs to that graph and is not kept."""
+    key = (win, str(device))
+    window = _WINDOWS.get(key)
+    if window is None:
+        window = torch.tensor(win, dtype=torch.int32, device=device)
+        if len(_WINDOWS) < 256 and not (device.type == "cuda" and torch.cuda.is_current_stream_capturing()):
+            if device.type == "cuda":
+                torch.cuda.current_stream(device).synchronize()  # once: any stream may read it from here on
+            _WINDOWS[key] = window
+    return window
 
 
 class ScaleKVCluster:
@@ -87,9 +105,9 @@ class ScaleKVCluster:
             warnings.warn(f"Layer {self.layer_idx}: max_capacity ({self.max_capacity}) is less than the window "
                           f"({len(win)}). Will only keep the window tokens.", UserWarning)
             self.max_capacity = len(win)
-        window = torch.tensor(win, dtype=torch.int32, device=key_states.device)
+        window = _window_on(tuple(win), key_states.device)
         if self.max_capacity == len(win):
-            return window.view(1, 1, -1).expand(B, H, -1).contiguous()
+            return window.view(1, 1, -1).expand(B, H, -1).clone(memory_format=torch.contiguous_format)
         offset = key_len - query_states.shape[2]
         scores = K.scalekv_scores(query_states, key_states, window, offset)
         pooled = K.scalekv_pool(scores, window, self.kernel_size, self.pooling)

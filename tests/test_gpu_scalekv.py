@@ -110,3 +110,18 @@ def test_scores_bits_follow_the_stated_order(K, D, Lkv, w):
     inside = window[window < Lkv].long()
     total[..., inside] = float("-inf")
     assert torch.equal(got, total)
+
+
+def test_window_only_selection_is_the_callers_own(K):
+    """With a budget of the window alone the returned indices are a fresh tensor, not the shared window, and several
+    scales and repeated calls keep their own windows."""
+    from lvar_b200.scalekv import ScaleKVCluster, window_indices
+    q = torch.randn(1, 1, 1600, 64).bfloat16().cuda()
+    for _ in range(2):
+        for lq, lkv, scale in ((1600, 4121, 10), (1024, 2521, 9), (1600, 4121, 10)):
+            c = ScaleKVCluster([[16]] * 13, window_size=16)
+            c.max_capacity = 16
+            k = torch.randn(1, 1, lkv, 64).bfloat16().cuda()
+            idx = c.select_indices(k, q[:, :, :lq], scale)
+            assert idx[0, 0].tolist() == window_indices(lq, lkv - lq, lkv, 16)
+            idx.fill_(-1)
