@@ -41,9 +41,10 @@ constexpr size_t scores_smem_bytes(int w) {
 // in ascending order, then a pairwise tree over the partial sums p and p + D/16, p + D/32, ...  A thread owns two
 // whole keys and a group of 8 queries, so that one 16-byte shared-memory read of queries feeds four packed
 // multiply-adds; the tree is walked in the order that closes its pairs at once (a binary counter), which keeps at most
-// log2(D/8) + 1 partial sums per logit alive.  Nothing crosses lanes.  32 heads x 6425
-// keys x 16 queries, D = 128: 43 us; 103 us with a key shared by as many lanes as it has 16-byte pieces, which
-// spends four shuffles and sixteen lanes' rounding arithmetic on every logit.
+// log2(D/8) + 1 partial sums per logit alive.  Nothing crosses lanes.  Only four of the D/8 leaves are unrolled: all of
+// them together miss the instruction caches (two stalled cycles per issue).  32 heads x 6425 keys x 16 queries, D = 128:
+// 38 us; 42 us with every leaf unrolled; 103 us with a key shared by as many lanes as it has 16-byte pieces, which spends
+// four shuffles and sixteen lanes' rounding arithmetic on every logit.
 template <int D>
 __global__ void __launch_bounds__(kScoreThreads, 5)
 scalekv_scores_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
@@ -89,57 +90,63 @@ scalekv_scores_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* 
 
   float total[2] = {0.f, 0.f};
   for (int g = 0; g < groups; ++g) {
-    uint64_t stack[LEVELS + 1][2][4];  // [tree level][key][query pair]; compile-time indices only
+    uint64_t node[2][4], pair[2][4], hold[2][4], left[2][4];  // [key][query pair]; node: the subtree just closed
+#pragma unroll 1
+    for (int m = 0; m < NP / 4; ++m) {
+      // leaf n of the walk is the piece whose number is n with its bits reversed; leaves 4m .. 4m + 3 close a subtree of
+      // four (unrolled), the subtrees close in the same manner in the outer loop
+      const int mrev = LEVELS == 4 ? ((m & 1) << 1) | (m >> 1) : m;
+      uint64_t first[2][4];
 #pragma unroll
-    for (int n = 0; n < NP; ++n) {
-      // leaf n of the walk is the piece whose number is n with its bits reversed
-      int piece = 0;
+      for (int n = 0; n < 4; ++n) {
+        const int piece = (((n & 1) << 1 | n >> 1) << (LEVELS - 2)) | mrev;
+        asm volatile("" ::: "memory");  // a piece's shared-memory reads stay with it: hoisted, they would spill
+        uint64_t acc[2][4];
 #pragma unroll
-      for (int bit = 0; bit < LEVELS; ++bit) piece |= ((n >> bit) & 1) << (LEVELS - 1 - bit);
-      asm volatile("" ::: "memory");  // a piece's shared-memory reads stay with it: hoisted, they would spill
-      uint64_t acc[2][4];
+        for (int x = 0; x < 2; ++x)
 #pragma unroll
-      for (int x = 0; x < 2; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) acc[x][y] = 0ull;
-      uint32_t ku[2][4];
-#pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(sh_keys + (threadIdx.x + x * kScoreThreads) * ROW + piece * 16);
-        ku[x][0] = raw.x; ku[x][1] = raw.y; ku[x][2] = raw.z; ku[x][3] = raw.w;
-      }
-      const ulonglong2* qp = reinterpret_cast<const ulonglong2*>(qf + (g * D + piece * 8) * kQGroup);
-#pragma unroll
-      for (int d = 0; d < 8; ++d) {
-        const ulonglong2 qa = qp[2 * d], qc = qp[2 * d + 1];
+          for (int y = 0; y < 4; ++y) acc[x][y] = 0ull;
+        uint32_t ku[2][4];
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
-          const uint32_t u = ku[x][d >> 1];
-          const float kv = __uint_as_float((d & 1) ? (u & 0xffff0000u) : (u << 16));
-          const uint64_t kk = pack_f32x2(kv, kv);
-          acc[x][0] = ffma2(qa.x, kk, acc[x][0]);
-          acc[x][1] = ffma2(qa.y, kk, acc[x][1]);
-          acc[x][2] = ffma2(qc.x, kk, acc[x][2]);
-          acc[x][3] = ffma2(qc.y, kk, acc[x][3]);
+          const uint4 raw = *reinterpret_cast<const uint4*>(sh_keys + (threadIdx.x + x * kScoreThreads) * ROW + piece * 16);
+          ku[x][0] = raw.x; ku[x][1] = raw.y; ku[x][2] = raw.z; ku[x][3] = raw.w;
         }
-      }
-      // binary counter: every trailing one bit of n closes a pair of the tree
+        const ulonglong2* qp = reinterpret_cast<const ulonglong2*>(qf + (g * D + piece * 8) * kQGroup);
 #pragma unroll
-      for (int lev = 0; lev <= LEVELS; ++lev) {
-        if (((n + 1) & ((1 << lev) - 1)) != 0) break;
+        for (int d = 0; d < 8; ++d) {
+          const ulonglong2 qa = qp[2 * d], qc = qp[2 * d + 1];
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const uint32_t u = ku[x][d >> 1];
+            const float kv = __uint_as_float((d & 1) ? (u & 0xffff0000u) : (u << 16));
+            const uint64_t kk = pack_f32x2(kv, kv);
+            acc[x][0] = ffma2(qa.x, kk, acc[x][0]);
+            acc[x][1] = ffma2(qa.y, kk, acc[x][1]);
+            acc[x][2] = ffma2(qc.x, kk, acc[x][2]);
+            acc[x][3] = ffma2(qc.y, kk, acc[x][3]);
+          }
+        }
 #pragma unroll
         for (int x = 0; x < 2; ++x)
 #pragma unroll
           for (int y = 0; y < 4; ++y) {
-            if (lev > 0) acc[x][y] = fadd2(stack[lev - 1][x][y], acc[x][y]);
+            if (n == 0 || n == 2) first[x][y] = acc[x][y];
+            else if (n == 1) pair[x][y] = fadd2(first[x][y], acc[x][y]);
+            else node[x][y] = fadd2(pair[x][y], fadd2(first[x][y], acc[x][y]));
           }
-        if (((n >> lev) & 1) == 0) {
-#pragma unroll
-          for (int x = 0; x < 2; ++x)
-#pragma unroll
-            for (int y = 0; y < 4; ++y) stack[lev][x][y] = acc[x][y];
-        }
       }
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+          if (m & 1) node[x][y] = fadd2(hold[x][y], node[x][y]);
+          else hold[x][y] = node[x][y];
+          if (LEVELS == 4) {
+            if (m == 1) left[x][y] = node[x][y];
+            if (m == 3) node[x][y] = fadd2(left[x][y], node[x][y]);
+          }
+        }
     }
     // the closed tree: logit rounded to bf16 (matmul output), divided by sqrt(D) and rounded again (bf16 / scalar)
 #pragma unroll
@@ -147,7 +154,7 @@ scalekv_scores_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* 
 #pragma unroll
       for (int y = 0; y < 4; ++y) {
         float lo, hi;
-        unpack_f32x2(stack[LEVELS][x][y], lo, hi);
+        unpack_f32x2(node[x][y], lo, hi);
         if (g * kQGroup + 2 * y < w) total[x] += bf16_round(bf16_round(lo) * inv_sqrt_d<D>());
         if (g * kQGroup + 2 * y + 1 < w) total[x] += bf16_round(bf16_round(hi) * inv_sqrt_d<D>());
       }
