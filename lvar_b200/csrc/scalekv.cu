@@ -193,21 +193,41 @@ __global__ void scalekv_pool_kernel(const float* __restrict__ scores, const int3
   }
 }
 
-// One 16-byte piece per thread.
-__global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__ idx,
-                                   __nv_bfloat16* __restrict__ dst, int H, int L, int n, int D, int64_t s_sb,
-                                   int64_t s_sh, int64_t s_sl, int64_t idx_row_stride, int64_t total_pieces) {
+// Bound by HBM once the index arithmetic is out of the way: D/8 threads copy a row in 16-byte pieces, a thread keeps its
+// piece number and walks rows (four in flight), a (batch, head) per grid row.  2000 of 6425 rows of 256 bytes, 32 heads:
+// 7.3 us; 8.7 us with 64-bit divisions and remainders for every piece.
+constexpr int kGatherThreads = 256, kGatherRows = 4;
+__global__ void __launch_bounds__(kGatherThreads)
+gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__ idx, __nv_bfloat16* __restrict__ dst,
+                   int H, int L, int n, int D, int64_t s_sb, int64_t s_sh, int64_t s_sl, int64_t idx_row_stride, int BH) {
   const int ppr = D / 8;  // pieces per row
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total_pieces;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(t % ppr);
-    const int64_t ri = t / ppr;      // (bh, i)
-    const int i = (int)(ri % n);
-    const int64_t bh = ri / n;
-    const int b = (int)(bh / H), h = (int)(bh % H);
-    const int row = min(max(idx[bh * idx_row_stride + i], 0), L - 1);
-    const uint4 v = *reinterpret_cast<const uint4*>(src + b * s_sb + h * s_sh + (int64_t)row * s_sl + c * 8);
-    reinterpret_cast<uint4*>(dst)[t] = v;
+  const int rpb = max(1, kGatherThreads / ppr);
+  const int r = (int)threadIdx.x / ppr;
+  if (r >= rpb) return;
+  const int c0 = (int)threadIdx.x - r * ppr;
+  for (int bh = blockIdx.y; bh < BH; bh += gridDim.y) {
+    const int b = bh / H, h = bh - b * H;
+    const __nv_bfloat16* s = src + b * s_sb + h * s_sh;
+    const int32_t* ix = idx + bh * idx_row_stride;
+    uint4* d = reinterpret_cast<uint4*>(dst) + (int64_t)bh * n * ppr;
+    for (int64_t i0 = (int64_t)blockIdx.x * rpb + r; i0 < n; i0 += (int64_t)gridDim.x * rpb * kGatherRows) {
+      int row[kGatherRows];
+#pragma unroll
+      for (int u = 0; u < kGatherRows; ++u) {
+        const int64_t i = i0 + (int64_t)u * gridDim.x * rpb;
+        row[u] = i < n ? min(max(ix[i], 0), L - 1) : 0;
+      }
+      for (int c = c0; c < ppr; c += kGatherThreads) {  // more than one pass only for rows above 4 KB
+        uint4 v[kGatherRows];
+#pragma unroll
+        for (int u = 0; u < kGatherRows; ++u) v[u] = *reinterpret_cast<const uint4*>(s + row[u] * s_sl + c * 8);
+#pragma unroll
+        for (int u = 0; u < kGatherRows; ++u) {
+          const int64_t i = i0 + (int64_t)u * gridDim.x * rpb;
+          if (i < n) d[i * ppr + c] = v[u];
+        }
+      }
+    }
   }
 }
 
@@ -264,12 +284,13 @@ int launch_gather_rows(const void* src, const int32_t* idx, void* dst, int B, in
   LVAR_REQUIRE(s_sb % 8 == 0 && s_sh % 8 == 0 && s_sl % 8 == 0, LVAR_ERR_ARG,
                "tensor strides must be multiples of 8 elements");
   LVAR_REQUIRE(idx_row_stride >= n, LVAR_ERR_ARG, "index rows shorter than n");
-  const int64_t total = (int64_t)B * H * n * (D / 8);
-  int64_t blocks = (total + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  gather_rows_kernel<<<(unsigned)blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(src), idx,
-                                                           static_cast<__nv_bfloat16*>(dst), H, L, n, D, s_sb, s_sh,
-                                                           s_sl, idx_row_stride, total);
+  LVAR_REQUIRE((int64_t)B * H < (1ll << 31), LVAR_ERR_LIMIT, "too many rows");
+  const int bh = B * H, rpb = D / 8 < kGatherThreads ? kGatherThreads / (D / 8) : 1;
+  const int64_t bx = ((int64_t)n + (int64_t)rpb * kGatherRows - 1) / ((int64_t)rpb * kGatherRows);
+  const dim3 grid((unsigned)(bx < (1ll << 30) ? bx : (1ll << 30)), (unsigned)(bh < 65535 ? bh : 65535));
+  gather_rows_kernel<<<grid, kGatherThreads, 0, stream>>>(static_cast<const __nv_bfloat16*>(src), idx,
+                                                          static_cast<__nv_bfloat16*>(dst), H, L, n, D, s_sb, s_sh, s_sl,
+                                                          idx_row_stride, bh);
   LVAR_CUDA_OK(cudaGetLastError());
   return LVAR_OK;
 }

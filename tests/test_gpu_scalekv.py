@@ -125,3 +125,15 @@ def test_window_only_selection_is_the_callers_own(K):
             idx = c.select_indices(k, q[:, :, :lq], scale)
             assert idx[0, 0].tolist() == window_indices(lq, lkv - lq, lkv, 16)
             idx.fill_(-1)
+
+
+@pytest.mark.parametrize("B,H,L,n,D", [(1, 1, 1, 1, 8), (2, 3, 70, 129, 128), (1, 2, 40, 33, 24), (1, 1, 9, 5, 2056), (3, 5, 200, 64, 64),
+                                       (2, 40000, 3, 2, 8)])
+def test_gather_rows_shapes(K, B, H, L, n, D):
+    """Rows shorter and longer than a block's pieces, piece counts that do not divide it, counts off the rows a thread
+    takes, more (batch, head) pairs than a grid row count allows, indices out of range on both sides."""
+    g = torch.Generator().manual_seed(n)
+    src = torch.randn(B, H, L, D, generator=g).bfloat16().cuda()
+    idx = torch.randint(-2, L + 2, (B, H, n), generator=g, dtype=torch.int32).cuda()
+    want = torch.gather(src, 2, idx.clamp(0, L - 1).long().unsqueeze(-1).expand(-1, -1, -1, D))
+    assert torch.equal(K.gather_rows(src, idx), want)
