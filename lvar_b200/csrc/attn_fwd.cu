@@ -1595,26 +1595,19 @@ int launch_attention(const lvar_attn_args* a, int mode, cudaStream_t stream) {
   const bool sums = mode == MODE_DENSE_CS || (mode == MODE_CS_ONLY && !stats_given);
   p.split_singles = (mode != MODE_CSP && !(a->sched_flags & LVAR_SCHED_SINGLE_ONE_SLOT) && (!sums || total > sms)) ? 1 : 0;
   if (mode != MODE_CSP && (total > sms || p.split_singles) && !(a->sched_flags & LVAR_SCHED_PAIRS_ONLY)) {
-    // Wave quantisation: the query tiles left over after the last full wave of CTAs are handed out as single tiles
-    // when those fit in one wave, so that the tail costs one short item per CTA instead of one full pair on a few CTAs.
-    // With work_order the tail is the end of the caller's order.  A split tile takes 0.62 of a pair's time (52 against
-    // 82 us for one wave at 33 KV tiles); left with one half of the CTA idle it takes all of it, since a slot's chain of
-    // dependent steps per KV tile is the same.  Column sums with an output, 4096 x 10521 x 32: 1.15 -> 1.08 ms, without
-    // 0.91 -> 0.88 ms, one sweep on 1000 x 2999 x 16 (64 pairs on 148 SMs) 63 -> 42 us; block-sparse on 1600 x 4121 x
-    // 32, whose heads end in half a pair: 46 -> 42 us.
-    int64_t singles = 0;  // pairs at the end of the order that are handed out as single tiles
-    if (p.split_singles) {
-      // counted in tiles: the last pair of a head with an odd number of tiles is half a pair's work
-      const int64_t per_head = (a->Lq + 127) / 128, left = per_head * a->B * a->H % (2 * sms);
-      if (left > 0 && left <= sms) {
-        const int64_t part = left % per_head, odd = per_head & 1;
-        singles = left / per_head * p.n_x + (part ? odd + (part - odd + 1) / 2 : 0);
-      }
-    } else if (2 * (total % sms) <= sms) {
-      singles = total % sms;
+    // Wave quantisation: the pairs left over after the last full wave of CTAs are handed out as single query tiles when
+    // those fit in one wave, so that the tail costs one short item per CTA instead of one full pair on a few CTAs.
+    // With work_order the tail is the end of the caller's order.  Column sums with an output, 4096 x 10521 x 32: 1.15 ->
+    // 1.08 ms, without 0.91 -> 0.88 ms; one sweep on 1000 x 2999 x 16 (64 pairs on 148 SMs) 63 -> 42 us.
+    // Pairs are what is counted, also where the last pair of a head holds one tile: a tile on one half of a CTA takes
+    // 0.8 of a pair's time (69 against 87 us for one wave at 33 KV tiles), not half of it.  Counting the left-over in
+    // tiles instead hands out too few or too many singles: dense attention with 13 tiles a
+    // head 192 -> 220 us at 48 heads and 265 -> 274 at 64, 5 tiles 122 -> 151 at 60, 9 tiles 117 -> 142 at 32.
+    const int64_t rem = total % sms;
+    if (rem > 0 && 2 * rem <= sms) {
+      p.n_pair_items = (int)(total - rem);
+      p.total_items = (int)(total + rem);
     }
-    p.n_pair_items = (int)(total - singles);
-    p.total_items = (int)(total + singles);
   }
   dim3 grid((unsigned)(p.total_items < sms ? p.total_items : sms), 1, 1);
 

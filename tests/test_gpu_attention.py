@@ -772,3 +772,21 @@ def test_column_sum_modes_with_split_tiles(K, B, H, Lq, Lkv, D):
     _, pair = K.dense_colsum_attn_fwd(q, k, v, group_tiles=2, status=st)
     assert torch.equal(pair, K.sum_tiles(cs, 2))
     _ok_status(K, st)
+
+
+@pytest.mark.parametrize("U,Lq,D", [(64, 1600, 128), (32, 1600, 128), (60, 576, 128), (160, 100, 64), (40, 576, 64), (30, 896, 128),
+                                    (80, 512, 128)])
+def test_tail_is_counted_in_pairs(K, U, Lq, D):
+    """The left-over pairs of the last wave, and no other tiles, run on both halves of a CTA: also where the last pair of
+    a head holds one tile.  A split tile adds two partial row sums where the one-half schedule keeps one running sum, so
+    the statistics of its 128 rows differ in their last bits; those of every other tile are the same bits."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    q, k, v = (t.cuda() for t in _qkv(1, U, Lq, 1100, D, seed=U))
+    _, M, L = K.dense_attn_fwd(q, k, v)
+    _, M1, L1 = K.dense_attn_fwd(q, k, v, sched_flags=SCHED_SINGLE_ONE_SLOT)
+    tiles, per_head = -(-Lq // 128), -(-Lq // 256)
+    total = U * per_head
+    rem = total % sms if 2 * (total % sms) <= sms else 0
+    want = {(p // per_head, t) for p in range(total - rem, total) for t in (2 * (p % per_head), 2 * (p % per_head) + 1) if t < tiles}
+    diff = torch.nn.functional.pad((L != L1)[0], (0, tiles * 128 - Lq)).view(U, tiles, 128).any(-1)
+    assert {tuple(x) for x in diff.nonzero().tolist()} == want
