@@ -688,12 +688,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             w1 = a1 * inv;
             m_stat = fmaxf(m_true, mt1);
             l_stat = lt > 0.f ? lt * fast_exp2(mm - m_stat) : 0.f;
-            if (kHasCs) {
+            if (kHasCs || MODE == MODE_DENSE_CS1) {
               // the column-sum sweep of both slots needs the merged constants; slot 1 gets its copy before this
-              // warpgroup goes on with the output
+              // warpgroup goes on with the output.  In the one-sweep mode lt is the row sum that the statistics take
+              // (a NaN stays one).
               m_ref = mm;
               l = lt;
-              if (other) {
+              if (kHasCs && other) {
                 negc[128 + r_in_tile] = (row_ok && lt > 0.f) ? -(mm + log2f(lt)) : -INFINITY;
                 mbar_arrive(&bars->xchg_back);
               }
@@ -837,12 +838,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         // attention's true normaliser even when the given constants were another pass's
         if (row_ok && p.L && !(split && s == 1)) {
           const int64_t si = (int64_t)im.bh * p.Lq + row;
-          const float sum = split ? l_stat : l;
           if (p.L_in == nullptr) {
-            p.L[si] = at_least_tiny(p.M_in[si]) / sum;
+            p.L[si] = at_least_tiny(p.M_in[si]) / l;
           } else {
             if (p.M) p.M[si] = p.M_in[si];
-            p.L[si] = p.L_in[si] * sum;
+            p.L[si] = p.L_in[si] * l;
           }
         }
       } else if (row_ok && MODE != MODE_CSP && !(split && s == 1)) {

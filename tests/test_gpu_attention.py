@@ -790,3 +790,25 @@ def test_tail_is_counted_in_pairs(K, U, Lq, D):
     want = {(p // per_head, t) for p in range(total - rem, total) for t in (2 * (p % per_head), 2 * (p % per_head) + 1) if t < tiles}
     diff = torch.nn.functional.pad((L != L1)[0], (0, tiles * 128 - Lq)).view(U, tiles, 128).any(-1)
     assert {tuple(x) for x in diff.nonzero().tolist()} == want
+
+
+@pytest.mark.parametrize("split", [True, False])
+@pytest.mark.parametrize("D", [64, 128])
+def test_one_sweep_statistics_keep_nan(K, D, split):
+    """A NaN in q makes its row's denominator NaN, a NaN key that of every row of its head, whether the row's tile runs on
+    one half of a CTA or on both (300 rows of two heads fit in one wave and split; one pair per SM does not)."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    H, Lq = (2, 300) if split else (sms, 256)
+    q, k, v = (t.cuda() for t in _qkv(1, H, Lq, 300, D, seed=3))
+    _, M, L = K.dense_attn_fwd(q, k, v)
+    q[0, 0, 5, 7] = float("nan")
+    q[0, 0, 200, 0] = float("nan")
+    k[0, 1, 290, 3] = float("nan")
+    want = torch.zeros(1, H, Lq, dtype=torch.bool, device="cuda")
+    want[0, 0, 5] = want[0, 0, 200] = True
+    want[0, 1] = True
+    o, _, _, Lo = K.dense_colsum_attn_given_fwd(q, k, v, M, L, return_stats=True)
+    op, _, own = K.dense_colsum_attn_p_fwd(q, k, v, (torch.exp2(-M) / L).contiguous())
+    for x in (Lo, own, o.float().sum(-1), op.float().sum(-1)):
+        assert torch.equal(torch.isnan(x), want)
+    assert torch.isfinite(own[~want]).all() and torch.isfinite(Lo[~want]).all()
