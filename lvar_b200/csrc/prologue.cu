@@ -44,10 +44,22 @@ struct PrologueParams {
 
 // a / b rounded to nearest, for r = 1 / b rounded to nearest: the residual of the first quotient is exact in a fused
 // multiply-add and corrects it (Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990).  Three instructions per element once the row's reciprocal is known.
+// processor", 1990).  Three instructions per element once the row's reciprocal is known.  Exact while the quotient is a
+// normal number and the residual does not fall below the subnormal step: for b in [1e-12, 2^64], a zero or |a| >= 2^-62.
+// The residual is formed with its sign reversed, so that a zero keeps its own.
 __device__ __forceinline__ float div_by(float a, float b, float r) {
   const float q = __fmul_rn(a, r);
-  return fmaf(fmaf(-q, b, a), r, q);
+  return fmaf(-fmaf(q, b, -a), r, q);
+}
+
+// Whether all eight bf16 elements are ones that div_by takes, where some are zeros or tiny.  Per 16-bit half: magnitude
+// + 0x7fff has no carry and, as a signed number, is largest for a zero and ascending for the others; 0x2080 is 2^-62.
+__device__ __forceinline__ bool div_by_takes(const uint32_t (&u)[4]) {
+  uint32_t least = 0x7fff7fffu;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) least = __vmins2(least, (u[i] & 0x7fff7fffu) + 0x7fff7fffu);
+  constexpr int kTiny = (int)(0xa07fu << 16);
+  return (int)(least << 16) >= kTiny && (int)(least & 0xffff0000u) >= kTiny;
 }
 
 template <bool WIDE>
@@ -99,7 +111,8 @@ __global__ void __launch_bounds__(256) qkv_prologue_kernel(const PrologueParams 
 #pragma unroll
       for (int which = 0; which < 3; ++which) raw[r][which] = load8<WIDE>(src + h * p.s_h + which * p.s_w);
     } else {
-      raw[r][0] = raw[r][1] = raw[r][2] = make_uint4(0, 0, 0, 0);
+      // ones: nothing that leaves the fast path of the division
+      raw[r][0] = raw[r][1] = raw[r][2] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
     }
   }
   float cs[4], sn[4];
@@ -141,12 +154,15 @@ __global__ void __launch_bounds__(256) qkv_prologue_kernel(const PrologueParams 
           for (int i = 0; i < d; ++i) ssq[i] += ssq[i + d];
         const float denom = fmaxf(sqrtf(ssq[0]), 1e-12f);
         const float mul = which == 0 && live ? p.scale_mul[h] : 1.0f;
-        if (ssq[0] < INFINITY) {
+        float least = fabsf(x[0]);
+#pragma unroll
+        for (int e = 1; e < 8; ++e) least = fminf(least, fabsf(x[e]));
+        if (ssq[0] < INFINITY && (least >= 0x1p-62f || div_by_takes(u))) {
           // denom lies in [1e-12, 2^64] and no quotient overflows
           const float inv = __frcp_rn(denom);
 #pragma unroll
           for (int e = 0; e < 8; ++e) x[e] = div_by(x[e], denom, inv);
-        } else {  // an infinite or NaN sum of squares
+        } else {  // an infinite or NaN sum of squares, a tiny element
 #pragma unroll
           for (int e = 0; e < 8; ++e) x[e] = __fdiv_rn(x[e], denom);
         }

@@ -120,3 +120,41 @@ def test_prologue_8_byte_rows_give_the_same_bits(K, B, L, H, c):
         fin = torch.isfinite(want)
         assert torch.equal(torch.isnan(got), torch.isnan(want))
         assert torch.equal(got[fin], want[fin])
+
+
+@pytest.mark.parametrize("c", [64, 128])
+@pytest.mark.parametrize("rope", [False, True])
+def test_prologue_division_bits(K, c, rope):
+    """Zeros of both signs, subnormal and tiny elements beside large ones, exponents over the whole range: bit for bit
+    plain fp32 division, rotation and one rounding to bf16.  The rows' sums of squares are exact here (one large power of
+    two, the rest far below its last bit, or rows so small that the norm is clamped), so any order of the sum gives them."""
+    g = torch.Generator().manual_seed(c)
+    B, L, H = 1, 64, 4
+    mant = torch.randint(128, 256, (B, L, 3, H, c), generator=g).float()
+    e = torch.randint(-140, -20, (B, L, 3, H, c), generator=g)
+    e[:, ::4] = torch.randint(-80, -60, (B, L // 4, 3, H, c), generator=g)
+    x = mant.double() * torch.exp2(e.double()) * (1 - 2 * torch.randint(0, 2, mant.shape, generator=g))
+    x[..., 0] = torch.exp2(torch.randint(20, 60, x.shape[:-1], generator=g).double())    # the norm
+    x[:, 1::4, ..., 0] = 1e-30                                                           # clamped norm, squares underflow
+    x[:, 1::4] = x[:, 1::4].clamp(-1e-30, 1e-30)
+    x[..., 3], x[..., 10], x[..., 11] = -0.0, 0.0, -0.0
+    x[:, 2::4, ..., 16:] = -0.0
+    qkv = x.float().bfloat16().cuda()
+    sm = torch.tensor([1.0, 0.37, 4.0, 2.5]).cuda()
+    ang = torch.rand(L, c // 2, generator=g) * 6
+    cos, sin = (ang.cos().cuda(), ang.sin().cuda()) if rope else (None, None)
+    kc = torch.zeros(B, H, L, c, dtype=torch.bfloat16, device="cuda")
+    vc = torch.zeros_like(kc)
+    q = K.qkv_prologue(qkv, sm, cos, sin, 0, kc, vc, 0)
+
+    def unit(y, mul):
+        y = y.permute(0, 2, 1, 3).float()
+        y = y / y.double().pow(2).sum(-1, keepdim=True).float().sqrt().clamp_min(1e-12)
+        if mul is not None:
+            y = y * mul.view(1, H, 1, 1)
+        if rope:
+            y0, y1 = y[..., 0::2], y[..., 1::2]
+            y = torch.stack([cos * y0 - sin * y1, sin * y0 + cos * y1], -1).flatten(-2)
+        return y.bfloat16()
+    for got, want in ((q, unit(qkv[:, :, 0], sm)), (kc, unit(qkv[:, :, 1], None))):
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16))
