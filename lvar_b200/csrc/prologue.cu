@@ -88,25 +88,30 @@ __device__ __forceinline__ void load4f(const float* p, float (&out)[4]) {
   }
 }
 
-// One warp: one token, ROWS * 32 / (C / 8) of its heads, all loads issued before any arithmetic.  WIDE: every base
-// and stride allows 16-byte accesses (else 8-byte ones, and single floats from the tables).
-template <int C, bool WIDE>
-__global__ void __launch_bounds__(256) qkv_prologue_kernel(const PrologueParams p, int units, int chunks) {
+// One warp: ROWS * 32 / (C / 8) rows, all loads issued before any arithmetic.  Its 32 / (C / 8) groups of C / 8 lanes
+// take 1 << hsh heads of as many tokens as that leaves (one token but for tensors with one or two heads).  WIDE: every
+// base and stride allows 16-byte accesses (else 8-byte ones, and single floats from the tables).
+template <int C, bool WIDE, int ROWS>
+__global__ void __launch_bounds__(256) qkv_prologue_kernel(const PrologueParams p, int units, int chunks, int hsh) {
   constexpr int LPR = C / 8;        // lanes per row
-  constexpr int RPW = 32 / LPR;     // rows per warp at a time
-  constexpr int ROWS = 2;           // rows per lane
+  constexpr int LOG_RPW = C == 128 ? 1 : 2;  // 32 / LPR rows per warp at a time
   const int lane = threadIdx.x & 31;
   const int unit = (int)blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
   if (unit >= units) return;
-  const int t = unit / chunks;      // token over the batch
+  const int g = lane / LPR;
+  const int sh = ROWS == 2 ? LOG_RPW : hsh;  // two rows per lane: one token per warp
+  const int tu = unit / chunks;
+  const int t = (tu << (LOG_RPW - sh)) + (g >> sh);  // token over the batch
   const int b = t / p.L, l = t - b * p.L;
-  const int h0 = (unit - t * chunks) * (ROWS * RPW) + lane / LPR;
+  const int hstep = 1 << sh;
+  // a lane past the last token takes part in the shuffles without a head
+  const int h0 = t < p.B * p.L ? (((unit - tu * chunks) * ROWS) << sh) + (g & (hstep - 1)) : p.H;
   const int e0 = (lane % LPR) * 8;  // this lane's first element
   const __nv_bfloat16* src = p.qkv + b * p.s_b + l * p.s_l + e0;
   uint4 raw[ROWS][3];
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
-    const int h = h0 + r * RPW;
+    const int h = h0 + r * hstep;
     if (h < p.H) {
 #pragma unroll
       for (int which = 0; which < 3; ++which) raw[r][which] = load8<WIDE>(src + h * p.s_h + which * p.s_w);
@@ -115,15 +120,18 @@ __global__ void __launch_bounds__(256) qkv_prologue_kernel(const PrologueParams 
       raw[r][0] = raw[r][1] = raw[r][2] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
     }
   }
+  float mul[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) mul[r] = p.scale_mul != nullptr && h0 + r * hstep < p.H ? p.scale_mul[h0 + r * hstep] : 1.0f;
   float cs[4], sn[4];
-  if (p.cos_t != nullptr) {
+  if (p.cos_t != nullptr && h0 < p.H) {
     const int64_t base = (int64_t)(p.rope_start + l) * (C / 2) + (e0 >> 1);
     load4f<WIDE>(p.cos_t + base, cs);
     load4f<WIDE>(p.sin_t + base, sn);
   }
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
-    const int h = h0 + r * RPW;
+    const int h = h0 + r * hstep;
     const bool live = h < p.H;  // lanes past the last head still take part in the shuffles
     uint4 out[2];
 #pragma unroll
@@ -153,7 +161,6 @@ __global__ void __launch_bounds__(256) qkv_prologue_kernel(const PrologueParams 
 #pragma unroll
           for (int i = 0; i < d; ++i) ssq[i] += ssq[i + d];
         const float denom = fmaxf(sqrtf(ssq[0]), 1e-12f);
-        const float mul = which == 0 && live ? p.scale_mul[h] : 1.0f;
         float least = fabsf(x[0]);
 #pragma unroll
         for (int e = 1; e < 8; ++e) least = fminf(least, fabsf(x[e]));
@@ -168,7 +175,7 @@ __global__ void __launch_bounds__(256) qkv_prologue_kernel(const PrologueParams 
         }
         if (which == 0) {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) x[e] = __fmul_rn(x[e], mul);
+          for (int e = 0; e < 8; ++e) x[e] = __fmul_rn(x[e], mul[r]);
         }
       }
       if (p.cos_t != nullptr) {
@@ -191,17 +198,34 @@ __global__ void __launch_bounds__(256) qkv_prologue_kernel(const PrologueParams 
   }
 }
 
-template <int C>
+template <int C, int ROWS>
 int launch_c(const PrologueParams& p, bool wide, cudaStream_t stream) {
-  constexpr int HEADS = 2 * 32 / (C / 8);  // heads per warp
-  const int chunks = (p.H + HEADS - 1) / HEADS;
-  const int64_t units = (int64_t)p.B * p.L * chunks;
-  LVAR_REQUIRE(units < (1ll << 31) - 8, LVAR_ERR_LIMIT, "too many rows");
+  constexpr int LOG_RPW = C == 128 ? 1 : 2;
+  int hsh = 0;
+  while (hsh < LOG_RPW && (ROWS == 2 || (1 << hsh) < p.H)) ++hsh;
+  const int chunks = (p.H + (ROWS << hsh) - 1) / (ROWS << hsh);
+  const int64_t tokens = (int64_t)p.B * p.L, per = 1 << (LOG_RPW - hsh);
+  const int64_t units = (tokens + per - 1) / per * chunks;
+  LVAR_REQUIRE(units < (1ll << 31) - 8 && tokens < (1ll << 31) - 8, LVAR_ERR_LIMIT, "too many rows");
   const unsigned blocks = (unsigned)((units + 7) / 8);
-  if (wide) qkv_prologue_kernel<C, true><<<blocks, 256, 0, stream>>>(p, (int)units, chunks);
-  else qkv_prologue_kernel<C, false><<<blocks, 256, 0, stream>>>(p, (int)units, chunks);
+  if (wide) qkv_prologue_kernel<C, true, ROWS><<<blocks, 256, 0, stream>>>(p, (int)units, chunks, hsh);
+  else qkv_prologue_kernel<C, false, ROWS><<<blocks, 256, 0, stream>>>(p, (int)units, chunks, hsh);
   LVAR_CUDA_OK(cudaGetLastError());
   return LVAR_OK;
+}
+
+// Two rows per lane once one row each would fill the chip twice over and the heads pad to the same number either way
+// (without normalisation, which is bound by memory alone, to at most a third more): 2 x 4096 x 16 x 128 36 against 41 us
+// with one.  One row otherwise: half the chain of dependent steps, which is all that a small call waits for (2 x 64 x 16 x
+// 128 2.8 against 3.8 us), and no idle lanes (2 x 4096 x 2 x 128 6.1 against 8.3, x 9 heads x 64 14.5 against 16.0).
+template <int C>
+int launch_rows(const PrologueParams& p, bool wide, cudaStream_t stream) {
+  constexpr int LOG_RPW = C == 128 ? 1 : 2;
+  const int64_t step = p.H > 1 << (LOG_RPW - 1) ? 1 << LOG_RPW : p.H;  // heads per warp with one row per lane
+  const int64_t chunks = (p.H + step - 1) / step, even = (chunks + 1) / 2 * 2;
+  const int64_t units = (int64_t)p.B * p.L * chunks;
+  const bool fits = even == chunks || (p.scale_mul == nullptr && 3 * even <= 4 * chunks);
+  return fits && units >= 2 * 148 * 40 ? launch_c<C, 2>(p, wide, stream) : launch_c<C, 1>(p, wide, stream);
 }
 
 }  // namespace
@@ -233,7 +257,7 @@ int launch_qkv_prologue(const void* qkv, int64_t s_b, int64_t s_l, int64_t s_w, 
   bool wide = (uintptr_t)rope_cos % 16 == 0 && (uintptr_t)rope_sin % 16 == 0;
   for (int64_t s : strides) wide = wide && s % 8 == 0;
   for (uintptr_t a : ptrs) wide = wide && a % 16 == 0;
-  return c == 128 ? launch_c<128>(p, wide, stream) : launch_c<64>(p, wide, stream);
+  return c == 128 ? launch_rows<128>(p, wide, stream) : launch_rows<64>(p, wide, stream);
 }
 
 }  // namespace lvar

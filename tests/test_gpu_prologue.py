@@ -158,3 +158,9 @@ def test_prologue_division_bits(K, c, rope):
         return y.bfloat16()
     for got, want in ((q, unit(qkv[:, :, 0], sm)), (kc, unit(qkv[:, :, 1], None))):
         assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("B,L,H,c", [(2, 7, 1, 128), (3, 3, 1, 64), (1, 5, 2, 64), (2, 130, 2, 128), (1, 1, 1, 64)])
+def test_prologue_tokens_that_share_a_warp(K, B, L, H, c):
+    """One and two heads: a warp takes several tokens (over the batch), the last warp fewer."""
+    test_prologue_8_byte_rows_give_the_same_bits(K, B, L, H, c)
