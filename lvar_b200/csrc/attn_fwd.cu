@@ -178,7 +178,12 @@ static_assert(sizeof(Bars) <= 512, "barrier block too large");
 
 }  // namespace
 
-template <int D, int MODE>
+// SPLIT: the launch may hold single tiles that run on both slots.  The column-sum modes with an output are built without
+// it too, for launches that hold none: the merge that such a launch never reaches cost the two-sweep mode 1 to 4 % (1600 x
+// 4121 x 32: 240 -> 244 us, 148 heads of one tile 104 -> 108) and the one-sweep mode 2 % (164 -> 167 us), in registers and
+// code.  What the schedule alone decides (decode, the loaders) is the same code either way: fewer run-time choices there
+// measured 2 % slower.  The other modes measured the same with and without.
+template <int D, int MODE, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const AttnParams p) {
@@ -362,7 +367,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const int n_mine = s == 0 ? e.n0 : e.n1;
 
       // the keys from this slot's first KV tile on (slot 1 of a split tile starts in the middle of the list)
-      const int key0 = (MODE != MODE_BLOCK && s == 1) ? e.off1 * 128 : 0, n_keys = p.Lkv - key0;
+      const int key0 = (SPLIT && MODE != MODE_BLOCK && s == 1) ? e.off1 * 128 : 0, n_keys = p.Lkv - key0;
       float m_ref = -INFINITY, m_true = -INFINITY, l = 0.f;
       int it = 0;
       if (MODE == MODE_DENSE_CS1 && n_mine > 0) {
@@ -603,7 +608,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (!ok) break;
 
       // ---- epilogue: O / l -> bf16 -> global; row statistics
-      const bool split = MODE != MODE_CSP && im.split;
+      const bool split = SPLIT && im.split;
       float m_stat = m_true, l_stat = (it > 0 && l > 0.f) ? l * fast_exp2(m_ref - m_true) : 0.f;
       if (MODE == MODE_CSP && row_ok) {
         // Column-sparse: the epilogue adds this row of the accumulate input (or the four rows of the coarser grid
@@ -1221,7 +1226,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                   if (t == s || D == 64) ok = mbar_wait(&bars->o_empty[t], (n_o[t] & 1) ^ 1, wc, DEV_TIMEOUT_MMA);
                 if (!ok) break;
               }
-              if (s == 1 && im.split) {  // the slots of a split tile have a K tile each
+              if (SPLIT && s == 1 && im.split) {  // the slots of a split tile have a K tile each
                 ks = kc % kStages;
                 kp = (kc / kStages) & 1;
                 ++kc;
@@ -1242,7 +1247,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               }
               umma_commit_if(leader, &bars->cs_full[s][buf]);
               ++n_cst[s][buf];
-              if (s == 1 || !cur.has[1] || im.split) umma_commit_if(leader, &bars->k_empty[ks]);  // last reader of the K stage
+              if (s == 1 || !cur.has[1] || (SPLIT && im.split)) umma_commit_if(leader, &bars->k_empty[ks]);  // last reader of the K stage
             }
           }
           // the next item's attention sweep writes S_s and O_s again: the softmax warps' last reads first
@@ -1407,10 +1412,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // -------------------------------------------------------------------------------------------------
 namespace {
 
-template <int D, int MODE>
+template <int D, int MODE, bool SPLIT>
 int launch_mode(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p, dim3 grid,
                 cudaStream_t stream, bool serialize_launch) {
-  auto kern = attn_fwd_kernel<D, MODE>;
+  auto kern = attn_fwd_kernel<D, MODE, SPLIT>;
   static bool attr_set[16] = {false};
   int dev = 0;
   LVAR_CUDA_OK(cudaGetDevice(&dev));
@@ -1438,13 +1443,18 @@ int launch_mode(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
 template <int D>
 int launch_d(int mode, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p,
              dim3 grid, cudaStream_t stream, bool serialize_launch) {
+  const bool splits = p.split_singles != 0 && p.n_pair_items < p.total_items;
   switch (mode) {
-    case MODE_DENSE: return launch_mode<D, MODE_DENSE>(tq, tk, tv, p, grid, stream, serialize_launch);
-    case MODE_BLOCK: return launch_mode<D, MODE_BLOCK>(tq, tk, tv, p, grid, stream, serialize_launch);
-    case MODE_DENSE_CS: return launch_mode<D, MODE_DENSE_CS>(tq, tk, tv, p, grid, stream, serialize_launch);
-    case MODE_CS_ONLY: return launch_mode<D, MODE_CS_ONLY>(tq, tk, tv, p, grid, stream, serialize_launch);
-    case MODE_DENSE_CS1: return launch_mode<D, MODE_DENSE_CS1>(tq, tk, tv, p, grid, stream, serialize_launch);
-    default: return launch_mode<D, MODE_CSP>(tq, tk, tv, p, grid, stream, serialize_launch);
+    case MODE_DENSE: return launch_mode<D, MODE_DENSE, true>(tq, tk, tv, p, grid, stream, serialize_launch);
+    case MODE_BLOCK: return launch_mode<D, MODE_BLOCK, true>(tq, tk, tv, p, grid, stream, serialize_launch);
+    case MODE_CS_ONLY: return launch_mode<D, MODE_CS_ONLY, true>(tq, tk, tv, p, grid, stream, serialize_launch);
+    case MODE_DENSE_CS:
+      return splits ? launch_mode<D, MODE_DENSE_CS, true>(tq, tk, tv, p, grid, stream, serialize_launch)
+                    : launch_mode<D, MODE_DENSE_CS, false>(tq, tk, tv, p, grid, stream, serialize_launch);
+    case MODE_DENSE_CS1:
+      return splits ? launch_mode<D, MODE_DENSE_CS1, true>(tq, tk, tv, p, grid, stream, serialize_launch)
+                    : launch_mode<D, MODE_DENSE_CS1, false>(tq, tk, tv, p, grid, stream, serialize_launch);
+    default: return launch_mode<D, MODE_CSP, false>(tq, tk, tv, p, grid, stream, serialize_launch);
   }
 }
 
