@@ -169,6 +169,60 @@ scalekv_scores_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* 
   }
 }
 
+// The same logits, sums and bits for few keys: a key is shared by as many lanes as it has 16-byte pieces, so that sixteen
+// times as many warps work on it, and a query slot that the window does not fill costs nothing.  Bound by latency like any
+// small launch; per key and query it needs three times the instructions of the kernel above (see launch_scalekv_scores).
+template <int D>
+__global__ void __launch_bounds__(256)
+scalekv_scores_few_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
+                          const int32_t* __restrict__ window, float* __restrict__ scores, int H, int Lq, int Lkv,
+                          int64_t q_sb, int64_t q_sh, int64_t q_sl, int64_t k_sb, int64_t k_sh, int64_t k_sl, int w,
+                          int offset) {
+  constexpr int LPK = D / 8;        // lanes per key
+  constexpr int KPB = 8 * 32 / LPK; // keys per block
+  __shared__ __align__(16) __nv_bfloat16 wq[kMaxWindow * D];
+  __shared__ int wcol[kMaxWindow];
+  const int bh = blockIdx.y, b = bh / H, h = bh % H;
+  const __nv_bfloat16* qb = q + b * q_sb + h * q_sh;
+  const __nv_bfloat16* kb = k + b * k_sb + h * k_sh;
+  for (int t = threadIdx.x; t < w * LPK; t += 256) {
+    const int i = t / LPK, c = t % LPK;
+    const int row = min(max(window[i] - offset, 0), Lq - 1);
+    reinterpret_cast<uint4*>(wq)[i * LPK + c] = *reinterpret_cast<const uint4*>(qb + (int64_t)row * q_sl + c * 8);
+  }
+  if (threadIdx.x < w) wcol[threadIdx.x] = window[threadIdx.x];
+  __syncthreads();
+  const int piece = threadIdx.x % LPK;
+  const int j = blockIdx.x * KPB + threadIdx.x / LPK;
+  float kf[8];
+  const uint4 kraw = j < Lkv ? *reinterpret_cast<const uint4*>(kb + (int64_t)j * k_sl + piece * 8) : make_uint4(0, 0, 0, 0);
+  const uint32_t ku[4] = {kraw.x, kraw.y, kraw.z, kraw.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    kf[2 * e] = __uint_as_float(ku[e] << 16);
+    kf[2 * e + 1] = __uint_as_float(ku[e] & 0xffff0000u);
+  }
+  float total = 0.f;
+  for (int i = 0; i < w; ++i) {
+    const uint4 raw = reinterpret_cast<const uint4*>(wq)[i * LPK + piece];
+    const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
+    float dot = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      dot = fmaf(__uint_as_float(u[e] << 16), kf[2 * e], dot);
+      dot = fmaf(__uint_as_float(u[e] & 0xffff0000u), kf[2 * e + 1], dot);
+    }
+#pragma unroll
+    for (int d = LPK / 2; d >= 1; d >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, d);
+    total += bf16_round(bf16_round(dot) * inv_sqrt_d<D>());
+  }
+  if (piece == 0 && j < Lkv) {
+    bool in_window = false;
+    for (int i = 0; i < w; ++i) in_window |= (wcol[i] == j);
+    scores[(int64_t)bh * Lkv + j] = in_window ? -INFINITY : bf16_round(total);
+  }
+}
+
 // pooled[j] over neighbours j - r .. j + r (r = ksize / 2); max: torch pads with -inf; average: torch pads
 // with zeros and divides by ksize, result rounded to bf16 like the input dtype.  Window columns -> +inf.
 __global__ void scalekv_pool_kernel(const float* __restrict__ scores, const int32_t* __restrict__ window, int w,
@@ -245,11 +299,22 @@ int launch_scalekv_scores(const void* q, const void* k, const int32_t* window, f
   for (int64_t s : strides)
     LVAR_REQUIRE(s % 8 == 0 && s >= 0, LVAR_ERR_ARG, "tensor strides must be non-negative multiples of 8 elements");
   LVAR_REQUIRE((int64_t)B * H <= 65535, LVAR_ERR_UNSUPPORTED, "B*H must be <= 65535");
-  dim3 grid((unsigned)((Lkv + kScoreKeys - 1) / kScoreKeys), (unsigned)(B * H));
+  // Few keys: the launch takes as long as one block, and a block of whole keys per thread pays 5.6 us plus 3 us per further
+  // group of eight queries (4.2 and 1.5 us with D = 64) where shared keys pay 2.2 us plus 0.28 us per query.  The lines
+  // are where the measured times cross, in keys times the used share of the query slots (one head of 200 keys, 16 queries:
+  // 5.9 against 8.3 us; 16 heads of 680 keys, one query, D = 64: 2.6 against 4.1 us; 32 heads of 265 keys, 16 queries: 8.8
+  // both ways).
+  const int slots = (w + kQGroup - 1) / kQGroup * kQGroup;
+  const bool few = (int64_t)B * H * Lkv * w < 9000ll * slots && (D == 128 || 4 * w <= 3 * slots);
+  const int kpb = few ? 8 * 32 / (D / 8) : kScoreKeys;
+  dim3 grid((unsigned)((Lkv + kpb - 1) / kpb), (unsigned)(B * H));
   const auto* qp = static_cast<const __nv_bfloat16*>(q);
   const auto* kp = static_cast<const __nv_bfloat16*>(k);
   const size_t smem = D == 128 ? scores_smem_bytes<128>(w) : scores_smem_bytes<64>(w);
-  if (D == 128) {
+  if (few) {
+    auto kern = D == 128 ? scalekv_scores_few_kernel<128> : scalekv_scores_few_kernel<64>;
+    kern<<<grid, 256, 0, stream>>>(qp, kp, window, scores, H, Lq, Lkv, q_sb, q_sh, q_sl, k_sb, k_sh, k_sl, w, offset);
+  } else if (D == 128) {
     LVAR_CUDA_OK(cudaFuncSetAttribute(scalekv_scores_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)scores_smem_bytes<128>(kMaxWindow)));
     scalekv_scores_kernel<128><<<grid, kScoreThreads, smem, stream>>>(qp, kp, window, scores, H, Lq, Lkv, q_sb, q_sh, q_sl,

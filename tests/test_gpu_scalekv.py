@@ -137,3 +137,17 @@ def test_gather_rows_shapes(K, B, H, L, n, D):
     idx = torch.randint(-2, L + 2, (B, H, n), generator=g, dtype=torch.int32).cuda()
     want = torch.gather(src, 2, idx.clamp(0, L - 1).long().unsqueeze(-1).expand(-1, -1, -1, D))
     assert torch.equal(K.gather_rows(src, idx), want)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("w,Lkv", [(1, 300), (4, 129), (16, 130), (9, 17), (64, 200), (6, 1000), (7, 1000)])
+def test_scores_of_few_and_many_keys_are_the_same_bits(K, D, w, Lkv):
+    """One head by itself (shared keys where the rule says few) and as one of enough heads that the rule says many."""
+    g = torch.Generator().manual_seed(w * Lkv)
+    copies = 73 + 9000 * 8 // Lkv * 8 // min(w, 8)
+    q = torch.randn(1, 1, max(w, 8), D, generator=g).bfloat16().cuda()
+    k = torch.randn(1, 1, Lkv, D, generator=g).bfloat16().cuda()
+    window = torch.randperm(max(Lkv, w), generator=g)[:w].sort().values.to(torch.int32).cuda()
+    one = K.scalekv_scores(q, k, window, 3)
+    many = K.scalekv_scores(q.expand(1, copies, -1, -1), k.expand(1, copies, -1, -1), window, 3)
+    assert torch.equal(many, one.expand_as(many))
