@@ -554,26 +554,27 @@ __global__ void bitunpack_kernel(const uint8_t* __restrict__ packed, uint8_t* __
 // Bound by the writes, which are nearly all zeros (the list rows have k_len columns): one block per list row, so that
 // no element pays for index divisions, and the tail in 16-byte stores from the first aligned column on.
 // 512 rows x 10521 columns: 6.9 us (3.1 TB/s of writes); 24.6 us with one flat index and its two 64-bit divisions per
-// element.
+// element.  Where there are fewer rows than SMs several blocks share a row (one row x 32768, all listed: 7.6 us by one
+// block).
 __global__ void __launch_bounds__(256)
 sparse_step_lists_kernel(const int32_t* __restrict__ src, const int32_t* __restrict__ remap,
                          const int32_t* __restrict__ band, int32_t* __restrict__ out, int32_t* __restrict__ counts,
                          int64_t rows, int64_t src_g_stride, int64_t src_bh_stride, int Gk, int cnt, int rep,
                          int band_count, int k_len, int out_cols, int count_value) {
-  const int tid = threadIdx.x;
+  const int tid = blockIdx.y * 256 + threadIdx.x, step = gridDim.y * 256;
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
     const int64_t bh = row / Gk;
     const int g = (int)(row - bh * Gk);
     const int32_t* s = src + bh * src_bh_stride + (int64_t)remap[g] * src_g_stride;
     const int32_t* bd = band + (int64_t)g * band_count;
     int32_t* dst = out + row * out_cols;
-    for (int c = tid; c < cnt; c += 256) dst[c] = max(0, min(s[rep == 1 ? c : c / rep], k_len - 1));
-    for (int c = tid; c < band_count; c += 256) dst[cnt + c] = bd[c];
+    for (int c = tid; c < cnt; c += step) dst[c] = max(0, min(s[rep == 1 ? c : c / rep], k_len - 1));
+    for (int c = tid; c < band_count; c += step) dst[cnt + c] = bd[c];
     const int used = cnt + band_count;
     const int first = min(out_cols, used + (int)((4 - ((reinterpret_cast<uintptr_t>(dst + used) >> 2) & 3)) & 3));
     const int quads = (out_cols - first) >> 2;
     int4* d4 = reinterpret_cast<int4*>(dst + first);
-    for (int i = tid; i < quads; i += 256) d4[i] = make_int4(0, 0, 0, 0);
+    for (int i = tid; i < quads; i += step) d4[i] = make_int4(0, 0, 0, 0);
     if (tid < first - used) dst[used + tid] = 0;
     const int rest = first + 4 * quads;
     if (tid < out_cols - rest) dst[rest + tid] = 0;
@@ -596,7 +597,10 @@ int launch_sparse_step_lists(const int32_t* src, const int32_t* remap, const int
   const int rep = src_cols >= cnt ? 1 : (cnt + src_cols - 1) / src_cols;
   const int64_t rows = BH * Gk;
   const unsigned blocks = (unsigned)(rows < (1ll << 30) ? rows : (1ll << 30));
-  sparse_step_lists_kernel<<<blocks, 256, 0, stream>>>(src, remap, band, out, counts, rows, src_g_stride, src_bh_stride,
+  // parts of at least four stores per thread
+  const int64_t parts = rows >= 148 ? 1 : (296 + rows - 1) / rows, most = (out_cols + 1023) / 1024;
+  const dim3 grid(blocks, (unsigned)(parts < most ? parts : most));
+  sparse_step_lists_kernel<<<grid, 256, 0, stream>>>(src, remap, band, out, counts, rows, src_g_stride, src_bh_stride,
                                                        Gk, cnt, rep, band_count, k_len, out_cols, count_value);
   LVAR_CUDA_OK(cudaGetLastError());
   return LVAR_OK;

@@ -249,3 +249,19 @@ def test_topk_value_distributions(K, rows, n, k):
         assert torch.equal(got[:, :k].cpu(), order) and (got[:, k:] == 0).all() and (counts == k).all()
         asc = K.topk_indices(dev, k, ascending_index=True, out_cols=cols)
         assert torch.equal(asc[:, :k].cpu(), order.sort(-1).values) and (asc[:, k:] == 0).all()
+
+
+@pytest.mark.parametrize("BH,Gk,k_len,cnt,nb", [(1, 1, 10521, 640, 0), (1, 1, 4099, 4000, 99), (3, 49, 2050, 100, 7), (4, 37, 1027, 3, 0),
+                                                 (2, 80, 2500, 64, 1)])
+def test_sparse_step_lists_row_counts(K, BH, Gk, k_len, cnt, nb):
+    """Few rows (several blocks share one), one row less than the line and as many: every element."""
+    torch.manual_seed(k_len)
+    inds = torch.randint(-5, 2 * k_len, (1, BH, 2, k_len), dtype=torch.int32)
+    remap = torch.randint(0, 2, (Gk,), dtype=torch.int32)
+    band = torch.randint(0, k_len, (Gk, nb), dtype=torch.int32) if nb else None
+    want = torch.zeros(1, BH, Gk, k_len, dtype=torch.int32)
+    want[..., :cnt] = inds[:, :, remap.long(), :cnt].clamp(0, k_len - 1)
+    if nb:
+        want[..., cnt:cnt + nb] = band
+    got, counts = K.sparse_step_lists(inds.cuda(), remap.cuda(), band.cuda() if nb else None, cnt, k_len, count_value=5)
+    assert torch.equal(got.cpu(), want) and (counts == 5).all()
