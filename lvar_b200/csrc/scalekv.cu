@@ -250,7 +250,8 @@ __global__ void scalekv_pool_kernel(const float* __restrict__ scores, const int3
 // Bound by HBM once the index arithmetic is out of the way: D/8 threads copy a row in 16-byte pieces, a thread keeps its
 // piece number and walks rows (four in flight), a (batch, head) per grid row.  2000 of 6425 rows of 256 bytes, 32 heads:
 // 7.3 us; 8.7 us with 64-bit divisions and remainders for every piece.
-constexpr int kGatherThreads = 256, kGatherRows = 4;
+constexpr int kGatherThreads = 256;
+template <int ROWS>
 __global__ void __launch_bounds__(kGatherThreads)
 gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__ idx, __nv_bfloat16* __restrict__ dst,
                    int H, int L, int n, int D, int64_t s_sb, int64_t s_sh, int64_t s_sl, int64_t idx_row_stride, int BH) {
@@ -264,20 +265,20 @@ gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restr
     const __nv_bfloat16* s = src + b * s_sb + h * s_sh;
     const int32_t* ix = idx + bh * idx_row_stride;
     uint4* d = reinterpret_cast<uint4*>(dst) + (int64_t)bh * n * ppr;
-    for (int64_t i0 = (int64_t)blockIdx.x * rpb + r; i0 < n; i0 += (int64_t)gridDim.x * rpb * kGatherRows) {
-      int row[kGatherRows];
+    for (int64_t i0 = (int64_t)blockIdx.x * rpb * ROWS + r; i0 < n; i0 += (int64_t)gridDim.x * rpb * ROWS) {
+      int row[ROWS];
 #pragma unroll
-      for (int u = 0; u < kGatherRows; ++u) {
-        const int64_t i = i0 + (int64_t)u * gridDim.x * rpb;
+      for (int u = 0; u < ROWS; ++u) {
+        const int64_t i = i0 + u * rpb;
         row[u] = i < n ? min(max(ix[i], 0), L - 1) : 0;
       }
       for (int c = c0; c < ppr; c += kGatherThreads) {  // more than one pass only for rows above 4 KB
-        uint4 v[kGatherRows];
+        uint4 v[ROWS];
 #pragma unroll
-        for (int u = 0; u < kGatherRows; ++u) v[u] = *reinterpret_cast<const uint4*>(s + row[u] * s_sl + c * 8);
+        for (int u = 0; u < ROWS; ++u) v[u] = *reinterpret_cast<const uint4*>(s + row[u] * s_sl + c * 8);
 #pragma unroll
-        for (int u = 0; u < kGatherRows; ++u) {
-          const int64_t i = i0 + (int64_t)u * gridDim.x * rpb;
+        for (int u = 0; u < ROWS; ++u) {
+          const int64_t i = i0 + u * rpb;
           if (i < n) d[i * ppr + c] = v[u];
         }
       }
@@ -351,11 +352,14 @@ int launch_gather_rows(const void* src, const int32_t* idx, void* dst, int B, in
   LVAR_REQUIRE(idx_row_stride >= n, LVAR_ERR_ARG, "index rows shorter than n");
   LVAR_REQUIRE((int64_t)B * H < (1ll << 31), LVAR_ERR_LIMIT, "too many rows");
   const int bh = B * H, rpb = D / 8 < kGatherThreads ? kGatherThreads / (D / 8) : 1;
-  const int64_t bx = ((int64_t)n + (int64_t)rpb * kGatherRows - 1) / ((int64_t)rpb * kGatherRows);
+  // four rows per thread once that still gives every SM two blocks; below, one row each
+  const int64_t bx4 = ((int64_t)n + (int64_t)rpb * 4 - 1) / ((int64_t)rpb * 4);
+  const bool four = bx4 * bh >= 2 * 148;
+  const int64_t bx = four ? bx4 : ((int64_t)n + rpb - 1) / rpb;
   const dim3 grid((unsigned)(bx < (1ll << 30) ? bx : (1ll << 30)), (unsigned)(bh < 65535 ? bh : 65535));
-  gather_rows_kernel<<<grid, kGatherThreads, 0, stream>>>(static_cast<const __nv_bfloat16*>(src), idx,
-                                                          static_cast<__nv_bfloat16*>(dst), H, L, n, D, s_sb, s_sh, s_sl,
-                                                          idx_row_stride, bh);
+  auto kern = four ? gather_rows_kernel<4> : gather_rows_kernel<1>;
+  kern<<<grid, kGatherThreads, 0, stream>>>(static_cast<const __nv_bfloat16*>(src), idx, static_cast<__nv_bfloat16*>(dst), H,
+                                            L, n, D, s_sb, s_sh, s_sl, idx_row_stride, bh);
   LVAR_CUDA_OK(cudaGetLastError());
   return LVAR_OK;
 }

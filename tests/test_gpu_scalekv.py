@@ -151,3 +151,9 @@ def test_scores_of_few_and_many_keys_are_the_same_bits(K, D, w, Lkv):
     one = K.scalekv_scores(q, k, window, 3)
     many = K.scalekv_scores(q.expand(1, copies, -1, -1), k.expand(1, copies, -1, -1), window, 3)
     assert torch.equal(many, one.expand_as(many))
+
+
+@pytest.mark.parametrize("B,H,L,n,D", [(2, 150, 20, 63, 128), (2, 150, 20, 65, 128), (1, 293, 5, 129, 64), (1, 300, 7, 1, 24), (2, 147, 3, 5, 2056)])
+def test_gather_rows_four_per_thread(K, B, H, L, n, D):
+    """Enough blocks for four rows per thread: counts below, at and off a block's share."""
+    test_gather_rows_shapes(K, B, H, L, n, D)
