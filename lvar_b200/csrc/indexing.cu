@@ -52,6 +52,31 @@ __global__ void block_scores_kernel(const float* __restrict__ cs, float* __restr
 // ------------------------------------------------------------------------------------------------
 // block mask: always U top-(k_total - |always|) of the rest
 // ------------------------------------------------------------------------------------------------
+// How many blocks come before block j among those that are not always kept: a larger key, or the same key at a lower
+// index.  Always-kept blocks have key 0, which precedes nothing but another 0 (a NaN's key): those look at the flags.  Past
+// the block's own 32 the index order is fixed, so that a comparison is all that is left: bound by issue where the rows
+// fill the chip (8192 rows of 192 blocks: 112 us with flag, key and index looked at in every step and a branch, 125 us
+// without the branch).
+__device__ __forceinline__ int rank_of(const uint32_t* keys, const uint8_t* flag, int nk, int j) {
+  const uint32_t kj = keys[j];
+  int rank = 0;
+  if (kj == 0u) {
+    for (int i = 0; i < nk; ++i) rank += !flag[i] && (keys[i] > 0u || i < j);
+    return rank;
+  }
+  const int j0 = j & ~31, j1 = min(nk, j0 + 32);
+#pragma unroll 8
+  for (int i = 0; i < j0; ++i) rank += keys[i] >= kj;
+#pragma unroll 4
+  for (int i = j0; i < j1; ++i) {
+    const uint32_t ki = keys[i];
+    rank += ki > kj || (ki == kj && i < j);
+  }
+#pragma unroll 8
+  for (int i = j1; i < nk; ++i) rank += keys[i] > kj;
+  return rank;
+}
+
 // One CTA (128 threads) per (b, h, q-block row).  Rank counting over the row held in shared memory.
 __global__ void build_block_mask_kernel(const float* __restrict__ scores, const uint8_t* __restrict__ always,
                                         uint8_t* __restrict__ mask, int32_t* __restrict__ lists,
@@ -67,8 +92,8 @@ __global__ void build_block_mask_kernel(const float* __restrict__ scores, const 
   __syncthreads();
   int local = 0;
   for (int j = threadIdx.x; j < nk; j += blockDim.x) {
-    keys[j] = ordered_key(s[j]);
     const uint8_t a = always ? (always[(int64_t)qi * nk + j] != 0) : 0;
+    keys[j] = a ? 0u : ordered_key(s[j]);
     flag[j] = a;
     local += a;
   }
@@ -79,14 +104,7 @@ __global__ void build_block_mask_kernel(const float* __restrict__ scores, const 
   for (int j = threadIdx.x; j < nk; j += blockDim.x) {
     uint8_t sel = flag[j];
     if (!sel && need > 0) {
-      const uint32_t kj = keys[j];
-      int rank = 0;
-#pragma unroll 4
-      for (int i = 0; i < nk; ++i) {
-        const uint32_t ki = keys[i];
-        rank += !flag[i] && ((ki > kj) || (ki == kj && i < j));
-      }
-      sel = rank < need;
+      sel = rank_of(keys, flag, nk, j) < need;
     }
     mrow[j] = sel;
   }
@@ -169,6 +187,7 @@ block_mask_from_colsums_kernel(const float* __restrict__ cs, int64_t cs_row_stri
   for (int j = threadIdx.x; j < nk; j += blockDim.x) {
     const uint8_t a = always ? (always[(int64_t)qi * nk + j] != 0) : 0;
     flag[j] = a;
+    if (a) keys[j] = 0u;
     local += a;
   }
   if (local) atomicAdd(&n_always, local);
@@ -178,14 +197,7 @@ block_mask_from_colsums_kernel(const float* __restrict__ cs, int64_t cs_row_stri
   for (int j = threadIdx.x; j < nk; j += blockDim.x) {
     uint8_t sel = flag[j];
     if (!sel && need > 0) {
-      const uint32_t kj = keys[j];
-      int rank = 0;
-#pragma unroll 4
-      for (int i = 0; i < nk; ++i) {
-        const uint32_t ki = keys[i];
-        rank += !flag[i] && ((ki > kj) || (ki == kj && i < j));
-      }
-      sel = rank < need;
+      sel = rank_of(keys, flag, nk, j) < need;
     }
     mrow[j] = sel;
   }

@@ -265,3 +265,31 @@ def test_sparse_step_lists_row_counts(K, BH, Gk, k_len, cnt, nb):
         want[..., cnt:cnt + nb] = band
     got, counts = K.sparse_step_lists(inds.cuda(), remap.cuda(), band.cuda() if nb else None, cnt, k_len, count_value=5)
     assert torch.equal(got.cpu(), want) and (counts == 5).all()
+
+
+@pytest.mark.parametrize("nk", [1, 31, 32, 33, 64, 95, 192, 257])
+def test_block_mask_rank_edges(K, nk):
+    """Ties across and inside the 32 blocks of a warp, rows of one value, infinities, always-kept blocks with the largest
+    and with the smallest scores, NaN scores of every sign (they select as one more value does, in a fixed order)."""
+    from oracle import indexing as oi
+    g = torch.Generator().manual_seed(nk)
+    s = torch.randint(0, 4, (1, 2, 6, nk), generator=g).float()
+    s[0, 0, 0] = -1.5
+    s[0, 0, 1] = torch.randn(nk, generator=g)
+    s[0, 0, 2, ::3] = float("inf")
+    s[0, 0, 3, ::2] = float("-inf")
+    always = torch.rand(6, nk, generator=g) < 0.2
+    always[2] = torch.isinf(s[0, 0, 2])
+    always[3] = torch.isinf(s[0, 0, 3])
+    always[4] = False
+    always[5] = True
+    for k_total in {0, 1, nk // 2, nk}:
+        want = oi.build_block_mask(s, always, k_total)
+        assert torch.equal(K.build_block_mask(s.cuda(), always.cuda(), k_total).cpu(), want)
+        cs = torch.zeros(1, 2, 6, nk * 32)
+        cs[..., ::32] = s                      # one score per block: sums of 32-wide blocks are the scores themselves
+        assert torch.equal(K.block_mask_from_colsums(cs.cuda(), always.cuda(), k_total, 32).cpu(), want)
+    bits = torch.tensor([0xffffffff, 0x7fffffff, 0xffc00000, 0x7fc00000], dtype=torch.int64).to(torch.int32).view(torch.float32)
+    s[0, 1, 4, : min(4, nk)] = bits[: min(4, nk)]
+    got = K.build_block_mask(s.cuda(), always.cuda(), max(1, nk // 2)).cpu()
+    assert (got[0, 1, 4].sum() == max(1, nk // 2)) and torch.equal(got[0, 0], oi.build_block_mask(s[:, :1], always, max(1, nk // 2))[0, 0])
