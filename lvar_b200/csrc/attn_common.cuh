@@ -121,41 +121,6 @@ __device__ __forceinline__ void exp_pack_chunk(const uint32_t (&r)[32], uint64_t
   }
 }
 
-// exp_pack_chunk (PACK) or exp_sum_chunk (not PACK; pk untouched) for chunk r, with the maximum of r and three more
-// chunks taken along the way: 32 exponentials keep the exp2 unit busy for longer than the 64 three-input maxima take to
-// issue, so the maxima are free as long as nothing waits for them.
-template <bool PACK>
-__device__ __forceinline__ void exp_max_chunk(const uint32_t (&r)[32], const uint32_t (&o1)[32], const uint32_t (&o2)[32],
-                                              const uint32_t (&o3)[32], uint64_t sc2, uint64_t nm2, uint64_t& sum_a,
-                                              uint64_t& sum_b, uint32_t (&pk)[32], float (&mx)[4]) {
-  auto max4 = [](float m, const uint32_t (&c)[32], int i) {
-    return fmax3(fmax3(m, __uint_as_float(c[i]), __uint_as_float(c[i + 1])), __uint_as_float(c[i + 2]),
-                 __uint_as_float(c[i + 3]));
-  };
-#pragma unroll
-  for (int i = 0; i < 32; i += 4) {
-    const uint64_t t0 = ffma2(pack_f32x2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), sc2, nm2);
-    const uint64_t t1 = ffma2(pack_f32x2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), sc2, nm2);
-    float a0, a1, b0, b1;
-    unpack_f32x2(t0, a0, a1);
-    unpack_f32x2(t1, b0, b1);
-    a0 = fast_exp2(a0);
-    a1 = fast_exp2(a1);
-    b0 = fast_exp2(b0);
-    b1 = fast_exp2(b1);
-    mx[0] = max4(mx[0], r, i);
-    mx[1] = max4(mx[1], o1, i);
-    mx[2] = max4(mx[2], o2, i);
-    mx[3] = max4(mx[3], o3, i);
-    sum_a = fadd2(sum_a, pack_f32x2(a0, a1));
-    sum_b = fadd2(sum_b, pack_f32x2(b0, b1));
-    if (PACK) {
-      pk[i / 2] = pack_bf16x2(a0, a1);
-      pk[i / 2 + 1] = pack_bf16x2(b0, b1);
-    }
-  }
-}
-
 // exp_pack_chunk without the packing: only the row sum of the 32 exponentials is kept.
 __device__ __forceinline__ void exp_sum_chunk(const uint32_t (&r)[32], uint64_t sc2, uint64_t nm2, uint64_t& sum_a,
                                               uint64_t& sum_b) {
