@@ -746,13 +746,16 @@ def test_overlapped_launches_keep_stream_order_for_data(K):
     assert torch.equal(chain2(0), chain2(_lib.SCHED_SERIALIZE_LAUNCH))
 
 
-@pytest.mark.parametrize("B,H,Lq,Lkv,D", [(2, 40, 640, 300, 128), (1, 75, 300, 100, 64), (1, 150, 129, 129, 64),
-                                          (2, 37, 384, 257, 128), (1, 50, 641, 520, 128), (1, 2, 300, 130, 128), (1, 3, 129, 90, 64)])
+@pytest.mark.parametrize("B,H,Lq,Lkv,D", [(3, 17, 640, 300, 128), (1, 75, 300, 100, 64), (1, 150, 129, 129, 64), (1, 150, 129, 100, 128),
+                                          (2, 38, 384, 257, 128), (1, 50, 641, 520, 128), (1, 2, 300, 130, 128), (1, 3, 129, 90, 64)])
 def test_column_sum_modes_with_split_tiles(K, B, H, Lq, Lkv, D):
     """More than one wave of work items: the last tiles run on both halves of a CTA, each with its own part of the KV
     list (odd and even tile counts per head, one KV tile only, ragged last tiles).  The modes with and without an
     output agree bit for bit, and with the one-half schedule and the stand-alone kernel to rounding.  The one-sweep mode
     splits within one wave too (last two shapes)."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    total = B * H * -(-Lq // 256)
+    assert 0 < 2 * (total % sms) <= sms and (total > sms or H < 4), "this shape does not split on this GPU"
     q, k, v = (t.cuda() for t in _qkv(B, H, Lq, Lkv, D, seed=Lq + H, peaked=True))
     st = K.new_status("cuda")
     o, cs, M, L = K.dense_colsum_attn_fwd(q, k, v, return_stats=True, status=st)
