@@ -260,7 +260,8 @@ __device__ __forceinline__ void bitonic_run(unsigned long long& x, unsigned long
 //  * The sort of the descending order keeps the steps at distances up to 32 in a warp's registers: 28 block-wide steps
 //    for 4096 pairs instead of 78, 6 instead of 36 for 256.
 //  * 512 threads where the rows fill the chip (up to four rows per SM; 256 threads measured 10 to 20 % slower on long
-//    rows, 1024 leave one row per SM), 1024 for fewer rows.
+//    rows, 1024 leave one row per SM), 1024 for fewer rows and for rows so long that an SM holds one: 149 x 24576, k =
+//    2000 descending takes 2.3 times the 148 rows' time with 512 threads.
 // rows x n, k: 224 x 4121, 256 descending 25.8 -> 15.1 us; 512 x 10521, 2176 descending 186 -> 135 us; 960 x 2500, 320
 // descending 94 -> 45 us; 32 x 10521, 1052 ascending 11.7 -> 10.8 us; 32 x 121, 12 ascending 6.1 -> 3.9 us (before: four
 // 8-bit passes always, every sorting step block-wide, 1024 threads always).
@@ -684,9 +685,12 @@ int launch_topk(const float* scores, int64_t rows, int n, int64_t row_stride, in
   int dev = 0, sms = 0;
   LVAR_CUDA_OK(cudaGetDevice(&dev));
   LVAR_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  auto kern = rows > sms ? topk_kernel<512> : topk_kernel<1024>;
+  // 512 threads where more than one row per SM is in flight: enough rows, and shared memory for two (of an SM's 228 KB a
+  // block takes 9.3 static and 1 reserved)
+  const bool half = rows > sms && 2 * (smem + 10752) <= 228 * 1024;
+  auto kern = half ? topk_kernel<512> : topk_kernel<1024>;
   LVAR_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024 + kSortRun * 8));
-  kern<<<(unsigned)rows, rows > sms ? 512 : 1024, smem, stream>>>(scores, row_stride, n, k, ascending_index, out,
+  kern<<<(unsigned)rows, half ? 512 : 1024, smem, stream>>>(scores, row_stride, n, k, ascending_index, out,
                                                                   out_stride, out_cols, counts, count_value, K2);
   LVAR_CUDA_OK(cudaGetLastError());
   return LVAR_OK;

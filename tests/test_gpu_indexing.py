@@ -293,3 +293,9 @@ def test_block_mask_rank_edges(K, nk):
     s[0, 1, 4, : min(4, nk)] = bits[: min(4, nk)]
     got = K.build_block_mask(s.cuda(), always.cuda(), max(1, nk // 2)).cpu()
     assert (got[0, 1, 4].sum() == max(1, nk // 2)) and torch.equal(got[0, 0], oi.build_block_mask(s[:, :1], always, max(1, nk // 2))[0, 0])
+
+
+@pytest.mark.parametrize("n,k", [(24000, 2000), (26001, 500), (33000, 16)])
+def test_topk_long_rows(K, n, k):
+    """More rows than SMs, each so long that an SM holds one (two in ascending order for the shorter ones)."""
+    test_topk_value_distributions(K, torch.cuda.get_device_properties(0).multi_processor_count + 2, n, k)
