@@ -103,8 +103,9 @@ typedef struct lvar_attn_args {
   uint64_t wait_limit_ns; /* per-wait limit of the kernel's bounded waits; 0 forces every pending wait to fail */
   /* scheduling switches (0 = default; for measurements and tests): LVAR_SCHED_* bits */
   int32_t sched_flags;
-  /* lvar_dense_colsum_attn_given only: the row statistics to normalise with, fp32 [B,H,Lq] contiguous, in the
-   * convention of M and L above (as lvar_dense_attn writes them) */
+  /* lvar_dense_colsum_attn_given: the row statistics to normalise with, fp32 [B,H,Lq] contiguous, in the convention of
+   * M and L above (as lvar_dense_attn writes them).  lvar_dense_colsum_attn_p: M_in holds p = 1 / sum exp(s), L_in is
+   * not read.  Not read by any other function. */
   const float* M_in;
   const float* L_in;
 } lvar_attn_args;

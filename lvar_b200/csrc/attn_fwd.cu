@@ -1600,8 +1600,9 @@ int launch_attention(const lvar_attn_args* a, int mode, cudaStream_t stream) {
   p.n_pair_items = (int)total;
   p.total_items = (int)total;
   // A single tile runs on both slots, each taking half of the tile's KV list (see the kernel's decode).  The modes that
-  // take statistics for a column-sum sweep of their own do so only when there is more than one wave of pairs: within
-  // one wave their output stays the bits of the dense kernel's one-slot schedule.
+  // take statistics for a column-sum sweep of their own do so only when there is more than one wave of pairs.  Within one
+  // wave callers may rely on their output being the bits of dense attention under LVAR_SCHED_SINGLE_ONE_SLOT (the tests
+  // hold them to it); splitting there has not been timed.
   const bool sums = mode == MODE_DENSE_CS || (mode == MODE_CS_ONLY && !stats_given);
   p.split_singles = (mode != MODE_CSP && !(a->sched_flags & LVAR_SCHED_SINGLE_ONE_SLOT) && (!sums || total > sms)) ? 1 : 0;
   if (mode != MODE_CSP && (total > sms || p.split_singles) && !(a->sched_flags & LVAR_SCHED_PAIRS_ONLY)) {

@@ -130,7 +130,7 @@ __global__ void build_block_mask_kernel(const float* __restrict__ scores, const 
 // sums once, forms the per-KV-block scores with block_scores_kernel's summation order (one warp per block: the
 // same bits) and selects as build_block_mask_kernel does.  Scores, lists and counts are optional outputs.
 // Bound by the latency of its loads: a warp has those of four 128-key blocks in flight.  1024 rows x 10521:
-// 13.5 us, 17.1 us with one block's four.
+// 10.8 us (17.1 us with one block's four and a branch per rank step).
 __global__ void __launch_bounds__(256)
 block_mask_from_colsums_kernel(const float* __restrict__ cs, int64_t cs_row_stride, const uint8_t* __restrict__ always,
                                uint8_t* __restrict__ mask, float* __restrict__ scores_out, int32_t* __restrict__ lists,
@@ -260,8 +260,8 @@ __device__ __forceinline__ void bitonic_run(unsigned long long& x, unsigned long
 //  * The sort of the descending order keeps the steps at distances up to 32 in a warp's registers: 28 block-wide steps
 //    for 4096 pairs instead of 78, 6 instead of 36 for 256.
 //  * 512 threads where the rows fill the chip (up to four rows per SM; 256 threads measured 10 to 20 % slower on long
-//    rows, 1024 leave one row per SM), 1024 for fewer rows and for rows so long that an SM holds one: 149 x 24576, k =
-//    2000 descending takes 2.3 times the 148 rows' time with 512 threads.
+//    rows, 1024 leave one row per SM), 1024 for fewer rows and for rows so long that an SM holds one (1024 x 24576, k =
+//    2000 descending: 218 us with 1024 threads, 274 with 512).
 // rows x n, k: 224 x 4121, 256 descending 25.8 -> 15.1 us; 512 x 10521, 2176 descending 186 -> 135 us; 960 x 2500, 320
 // descending 94 -> 45 us; 32 x 10521, 1052 ascending 11.7 -> 10.8 us; 32 x 121, 12 ascending 6.1 -> 3.9 us (before: four
 // 8-bit passes always, every sorting step block-wide, 1024 threads always).
@@ -566,7 +566,7 @@ __global__ void bitunpack_kernel(const uint8_t* __restrict__ packed, uint8_t* __
 //               = 0                                                 beyond;   counts[bh, g] = count_value
 // Bound by the writes, which are nearly all zeros (the list rows have k_len columns): one block per list row, so that
 // no element pays for index divisions, and the tail in 16-byte stores from the first aligned column on.
-// 512 rows x 10521 columns: 6.9 us (3.1 TB/s of writes); 24.6 us with one flat index and its two 64-bit divisions per
+// 512 rows x 10521 columns: 5.6 us (3.8 TB/s of writes); 23.3 us with one flat index and its two 64-bit divisions per
 // element.  Where there are fewer rows than SMs several blocks share a row (one row x 32768, all listed: 7.6 us by one
 // block).
 __global__ void __launch_bounds__(256)

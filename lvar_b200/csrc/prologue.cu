@@ -15,7 +15,7 @@
 // share a (b, l, h) row and hold 8 consecutive elements each (16-byte accesses), a warp takes one token and a few heads
 // so that the rotation table is read once for all of them, and every index is 32-bit.  A warp per row with 4 or 2
 // elements per lane, 64-bit index divisions and a library division per element was bound by instruction issue:
-// 66 us for 2 x 4096 tokens x 16 heads x 128 and 256 us for 8 x 4096, now 37 and 136 us (5.9 TB/s).
+// 66 us for 2 x 4096 tokens x 16 heads x 128 and 256 us for 8 x 4096, now 36 and 135 us (6.0 TB/s).
 #include <math.h>
 
 #include "common.cuh"

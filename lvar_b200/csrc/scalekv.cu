@@ -1,5 +1,5 @@
 // KV-cache compaction scores of ScaleKV (models/scalekv/scale_kv.py:232-301) and the row gather that
-// builds the compacted cache.  All three kernels are HBM-bound byte movers:
+// builds the compacted cache (pool and gather are byte movers; the scores are bound by the fp32 pipe, see below):
 //   scalekv_scores  score[b,h,j] = sum over the window queries i of bf16(bf16(q_i . k_j) / sqrt(D)), -inf on
 //                   the window's own columns (the reference's matmul, division, masked_fill and sum on bf16
 //                   tensors, rounding where torch rounds); K is read once
@@ -249,7 +249,7 @@ __global__ void scalekv_pool_kernel(const float* __restrict__ scores, const int3
 
 // Bound by HBM once the index arithmetic is out of the way: D/8 threads copy a row in 16-byte pieces, a thread keeps its
 // piece number and walks rows (four in flight), a (batch, head) per grid row.  2000 of 6425 rows of 256 bytes, 32 heads:
-// 7.3 us; 8.7 us with 64-bit divisions and remainders for every piece.
+// 5.8 us; 7.7 us with 64-bit divisions and remainders for every piece.
 constexpr int kGatherThreads = 256;
 template <int ROWS>
 __global__ void __launch_bounds__(kGatherThreads)
