@@ -1612,8 +1612,8 @@ int launch_attention(const lvar_attn_args* a, int mode, cudaStream_t stream) {
     // 1.08 ms, without 0.91 -> 0.88 ms; one sweep on 1000 x 2999 x 16 (64 pairs on 148 SMs) 63 -> 42 us.
     // Pairs are what is counted, also where the last pair of a head holds one tile: a tile on one half of a CTA takes
     // 0.8 of a pair's time (69 against 87 us for one wave at 33 KV tiles), not half of it.  Counting the left-over in
-    // tiles instead hands out too few or too many singles: dense attention with 13 tiles a
-    // head 192 -> 220 us at 48 heads and 265 -> 274 at 64, 5 tiles 122 -> 151 at 60, 9 tiles 117 -> 142 at 32.
+    // tiles instead hands out too few or too many singles: dense attention with 13 tiles a head 192 -> 220 us at 48 heads
+    // and 265 -> 274 at 64, 5 tiles 122 -> 151 at 60, 9 tiles 117 -> 142 at 32.
     const int64_t rem = total % sms;
     if (rem > 0 && 2 * rem <= sms) {
       p.n_pair_items = (int)(total - rem);
