@@ -7,15 +7,22 @@
 // same round is loaded once (always the case for dense and column-sparse attention).
 //   warps 0-3   softmax warpgroup of slot 0 (thread = one query row = one TMEM lane)
 //   warps 4-7   softmax warpgroup of slot 1
-//   warp  8     K loader (+ the two Q tiles): TMA, or 16-byte cp.async row gathers for csp (four lanes share
-//               a row; the tile's barrier takes one arrival per lane as its copies land)
-//   warp  9     V loader
-//   warp  10    allocates TMEM; lane 0 issues every tcgen05.mma (descriptor words precomputed, all lanes
-//               run the bookkeeping so that it stays out of a divergent branch)
-//   warp  11    scheduler: takes work items from the global counter and builds their KV-tile lists
-// TMEM (512 columns x 128 lanes, fp32): S0 | S1 | O0 | O1.  S_s = Q_s K^T lands in S_s; the softmax
-// warpgroup overwrites the first 64 columns of S_s with bf16 P_s, which is then the TMEM A operand of
-// O_s += P_s V.  Shared memory: Q0,Q1 + 2 K stages + 2 V stages, all 128-byte-swizzled [128][64]
+//   warp  8     loader of Q, K and V by TMA; column-sparse: of Q by TMA and of K by 16-byte cp.async row gathers (four
+//               lanes share a row; the tile's barrier takes one arrival per lane as its copies land)
+//   warp  9     one lane issues the P V products; column-sparse: V gather
+//   warp  10    allocates TMEM; one lane issues the Q K^T products
+//   warp  11    scheduler: takes work items from the global counter and builds their KV-tile lists; column-sparse: also
+//               issues the P V products
+// TMEM (512 columns x 128 lanes, fp32): P0 [0, 64) | S [64, 192) | P1 [192, 256) | O0 | O1.  The two slots take turns with
+// ONE score buffer: S = Q_s K^T is read into registers as soon as it lands, which frees the buffer for the other slot's
+// product, while the slot's own P has columns of its own.  A slot's next scores are then ready when its softmax warps
+// are, instead of a P V and a Q K^T product after they have written P (P used to lie over the slot's own scores): the
+// time of a round of both slots fell from 3800 to 2600 cycles of 2048 that the tensor pipe works (dense attention, 4096
+// x 10521 x 32: 622 -> 519 us; 1024 x 2521 x 32: 52 -> 39).  What is left is the way of the buffer: scores seen, read,
+// release seen, product, 1100 cycles a slot when the tensor pipe is otherwise idle (measured alone), 1300 beside P V
+// products.  Taking turns also keeps the warpgroups out of step, which is worth more than buffers: with head dimension
+// 64 there is room for a score buffer per slot, and dense attention took 720 us with it against 634.
+// Shared memory: Q0,Q1 + 2 K stages + 2 V stages, all 128-byte-swizzled [128][64]
 // bf16 sub-tiles (exactly what a [64 x 128] TMA box writes), K-major for Q/K and MN-major for V.
 //
 // Softmax keeps a per-row reference maximum that is only moved when the running maximum exceeds it
@@ -39,15 +46,11 @@ namespace lvar {
 
 namespace {
 
-constexpr int kThreads = 384;  // 8 softmax warps + K loader + V loader + MMA issuer + scheduler
+constexpr int kThreads = 384;  // 8 softmax warps, loader, P V issuer, Q K^T issuer, scheduler
 constexpr int kRegsSoftmax = 208, kRegsOther = 72;
 constexpr int kMaxSteps = 1024;  // per-slot KV tile list capacity (block-sparse: Lkv <= 131072)
 constexpr int kStages = 2;
 constexpr int kSchedStages = 2;
-// TMEM buffers per slot for S^T in the column-sum sweep: 1 (S_s) or 2 (S_s and the O region).  Two buffers let
-// the MMA of the next tile run under the softmax warps' reads and measured 6 % slower, like every other
-// change that keeps the tensor pipe busy while TMEM is being read.
-constexpr int kCsBufs = 1;
 // Column-sum sweep: which of the 8 groups of four exponentials per 32-column chunk are evaluated on the FMA
 // pipe (polynomial) instead of the exp2 unit, the sweep's bottleneck.  A quarter of them measured best
 // (0.47 -> 0.42 ms for the sweep at 4096 x 10521 x 32 heads; three eighths or a half: 0.43-0.45 ms); the same
@@ -161,14 +164,14 @@ struct Bars {
   uint64_t q_full, q_empty;
   uint64_t k_full[kStages], k_empty[kStages];
   uint64_t v_full[kStages], v_empty[kStages];
-  uint64_t s_full[2], p_full[2], o_full[2], o_empty[2];
+  uint64_t s_full[2], s_read, p_full[2], pv_done[2], o_empty[2];
   uint64_t sched_full[kSchedStages], sched_empty[kSchedStages];
-  uint64_t mma_done;
+  uint64_t mma_done[2];  // [Q K^T issuer, P V issuer]
+  uint64_t pv_all;  // second sweep to follow: every P V product of the item has completed
   uint64_t xchg_full[2];  // split tile: slot 1's partial result is complete (128 arrivals), by item parity
   uint64_t part_full[2][2];  // MODE_DENSE_CS1: the four warps' column sums of a tile are in shared memory [slot][buffer]
   uint64_t rowl_full[2];     // MODE_DENSE_CS1: the rows' probability sums of an item are in shared memory [slot]
-  // column-sum sweep (MODE_DENSE_CS): S^T of a slot is double-buffered, [slot][buffer]
-  uint64_t cs_full[2][2], cs_empty[2][2];
+  uint64_t cs_full[2], cs_empty[2];  // column-sum sweep: S^T of a slot has landed / has been read
   SchedEntry sched[kSchedStages];
   uint32_t tmem_base;
   int abort_flag;
@@ -192,12 +195,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   constexpr int KSTEPS_QK = D / 16;
   constexpr uint32_t IDESC_QK = make_idesc_bf16(128, 128, 0, 0);
   constexpr uint32_t IDESC_PV = make_idesc_bf16(128, D, 0, 1);
-  constexpr uint32_t TM_O = 256;
+  constexpr uint32_t TM_S = 64, TM_P1 = 192, TM_O = 256;
   constexpr bool kHasCs = MODE == MODE_DENSE_CS || MODE == MODE_CS_ONLY;  // column-sum sweep after the first one
-  // Epilogue form: O_s read out in one go and stored with 256-bit stores, or 32 columns at a time with 128-bit
-  // stores.  Chosen per mode by measurement (block-sparse +2.4 % with the first form, dense attention at 83 KV
-  // tiles per item -1.6 %: the kernel is sensitive to the size and placement of code it runs once per item).
-  constexpr bool kRegisterEpilogue = MODE == MODE_BLOCK || MODE == MODE_DENSE_CS || MODE == MODE_DENSE_CS1;
+  // Columns that are not attended become -inf in TMEM before the scores are read, in a loop of a few instructions, or in
+  // registers.  The loop suits the modes that meet such tiles often and whose items are short (column-sparse 65 -> 57 us
+  // at 1600 x 4121 x 32); in the dense modes its test ahead of the read lengthens the way from one slot's scores to the
+  // other's next product (dense 4096 x 10521 x 32: 520 -> 580 us).
+  constexpr bool kMaskInTmem = MODE == MODE_CSP || MODE == MODE_BLOCK;
   // MODE_CS_ONLY with the caller's row statistics: no first sweep at all
   const bool stats_given = MODE == MODE_CS_ONLY && p.M_in != nullptr;
 
@@ -227,18 +231,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     for (int s = 0; s < 2; ++s) {
       mbar_init(&bars->s_full[s], 1);
       mbar_init(&bars->p_full[s], 128);
-      mbar_init(&bars->o_full[s], 1);
+      mbar_init(&bars->pv_done[s], 1);
       mbar_init(&bars->o_empty[s], 128);
-      for (int b = 0; b < 2; ++b) {
-        mbar_init(&bars->cs_full[s][b], 1);
-        mbar_init(&bars->cs_empty[s][b], 128);
-      }
+      mbar_init(&bars->cs_full[s], 1);
+      mbar_init(&bars->cs_empty[s], 128);
     }
     for (int i = 0; i < kSchedStages; ++i) {
       mbar_init(&bars->sched_full[i], 1);
-      mbar_init(&bars->sched_empty[i], 11);  // 8 softmax warps + K loader + V loader + MMA issuer
+      mbar_init(&bars->sched_empty[i], 12);  // every warp
     }
-    mbar_init(&bars->mma_done, 1);
+    mbar_init(&bars->s_read, 128);
+    mbar_init(&bars->mma_done[0], 1);
+    mbar_init(&bars->mma_done[1], 1);
+    mbar_init(&bars->pv_all, 1);
     mbar_init(&bars->xchg_full[0], 128);
     mbar_init(&bars->xchg_full[1], 128);
     if (kHasCs) mbar_init(&bars->xchg_back, 128);
@@ -333,9 +338,83 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (s == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
     else asm volatile("bar.sync 2, 128;" ::: "memory");
   };
+  // Both slots want the same KV tile in round r (it is then loaded once).
+  auto round_shared = [&](const uint16_t* l0, const uint16_t* l1, const SchedEntry& e, int r) {
+    return r < e.n0 && r < e.n1 && (MODE == MODE_BLOCK ? ((l0[r] ^ l1[r]) & 0xFFF) == 0 : e.off1 == 0);
+  };
+  // Waits (bounded) until every MMA this thread has issued is complete: TMEM must not be freed, nor the CTA retire,
+  // while one is in flight, also on abort.
+  auto drain_mma = [&](uint64_t* bar) {
+    umma_commit(bar);
+    const uint64_t t0 = globaltimer_ns();
+    while (!mbar_try_wait(bar, 0)) {
+      if (globaltimer_ns() - t0 > 2000000000ull) {
+        if (p.status) atomicCAS(p.status, 0, (int)DEV_TIMEOUT_DRAIN);
+        break;
+      }
+    }
+  };
   uint8_t* sQ = smem + SM::kQ;
   uint8_t* sK = smem + SM::kK;
   uint8_t* sV = smem + SM::kV;
+
+  // The P V products of rounds [r0, r1) of an item; one thread.
+  struct PvState {
+    uint32_t vc = 0, n_p0 = 0, n_p1 = 0, n_o0 = 1, n_o1 = 1;
+  };
+  auto pv_rounds = [&](PvState& ps, const SchedEntry& e, int n, int r0, int r1) -> bool {
+    constexpr uint32_t DESC_HI = sw128_desc_hi(1024);
+    constexpr uint32_t TILE16 = SM::kTile >> 4;
+    const uint32_t v_lo = sw128_desc_lo(smem_u32(sV), 16384);
+    const uint16_t* l0 = lists + ((n % kSchedStages) * 2) * kMaxSteps;
+    const uint16_t* l1 = l0 + kMaxSteps;
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait(bar, parity, wc, DEV_TIMEOUT_MMA); };
+    auto issue = [&](uint32_t tO, uint32_t tPs, uint32_t st, uint32_t acc) {
+      const uint32_t vb = v_lo + st * TILE16;
+      umma_ts_if(1u, tO, tPs, vb, DESC_HI, IDESC_PV, acc);
+#pragma unroll
+      for (int i = 1; i < 8; ++i) umma_ts_if(1u, tO, tPs + i * 8, vb + i * 128, DESC_HI, IDESC_PV, 1u);
+    };
+    for (int r = r0; r < r1; ++r) {
+      const bool h0 = r < e.n0, h1 = r < e.n1, shared = round_shared(l0, l1, e, r);
+      if (h0) {
+        const uint32_t st = ps.vc & 1;
+        if (!wait(&bars->v_full[st], (ps.vc >> 1) & 1)) return false;
+        // first PV of the item overwrites O_s: the previous item's epilogue must have read it
+        if (r == 0 && !wait(&bars->o_empty[0], ps.n_o0 & 1)) return false;
+        if (!wait(&bars->p_full[0], ps.n_p0 & 1)) return false;
+        ++ps.n_p0;
+        // column-sparse: V came by cp.async (generic proxy), the MMA reads it through the async proxy
+        if (MODE == MODE_CSP) fence_proxy_async_smem();
+        tc_fence_after();
+        issue(tmem_base + TM_O, tmem_base, st, r > 0 ? 1u : 0u);
+        umma_commit(&bars->pv_done[0]);
+        if (!shared) {
+          umma_commit(&bars->v_empty[st]);
+          ++ps.vc;
+        }
+      }
+      if (h1) {
+        const uint32_t st = ps.vc & 1;
+        if (!shared && !wait(&bars->v_full[st], (ps.vc >> 1) & 1)) return false;
+        if (r == 0 && !wait(&bars->o_empty[1], ps.n_o1 & 1)) return false;
+        if (!wait(&bars->p_full[1], ps.n_p1 & 1)) return false;
+        ++ps.n_p1;
+        if (MODE == MODE_CSP) fence_proxy_async_smem();
+        tc_fence_after();
+        issue(tmem_base + TM_O + D, tmem_base + TM_P1, st, r > 0 ? 1u : 0u);
+        umma_commit(&bars->pv_done[1]);
+        umma_commit(&bars->v_empty[st]);
+        ++ps.vc;
+      }
+    }
+    return true;
+  };
+  auto pv_end = [&](PvState& ps, const SchedEntry& e) {  // after the item's last round
+    if (kHasCs && max(e.n0, e.n1) > 0) umma_commit(&bars->pv_all);
+    if (e.n0 > 0) ++ps.n_o0;
+    if (e.n1 > 0) ++ps.n_o1;
+  };
 
   if (warp < 8) {
     // ============================================================ softmax warpgroups
@@ -344,11 +423,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int quad = warp & 3;
     const int r_in_tile = quad * 32 + lane;
     const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
-    const uint32_t tS = tmem_base + lane_off + (uint32_t)s * 128u;
+    const uint32_t tS = tmem_base + lane_off + TM_S;  // scores of this slot's next tile
+    const uint32_t tP = tmem_base + lane_off + (uint32_t)s * TM_P1;
+    const uint32_t tT = tmem_base + lane_off + (uint32_t)s * 128u;  // S^T of the column-sum sweep
     const uint32_t tO = tmem_base + lane_off + TM_O + (uint32_t)s * D;
     int n_s = 0;  // S tiles consumed by this slot so far (parity of s_full)
-    int n_o = 0;  // items in which this slot produced an output (parity of o_full)
-    int n_cs[2] = {0, 0};  // column-sum sweep: S^T tiles read per buffer (parity of cs_full)
+    int n_pv = 0;  // P V products of this slot waited for so far (parity of pv_done)
+    int n_cs = 0;          // column-sum sweep: S^T tiles read (parity of cs_full)
     int n_xc[2] = {0, 0};  // split tiles merged so far, by item parity (parity of xchg_full)
     int n_back = 0;        // split tiles whose constants came back (parity of xchg_back)
     int n_part[2] = {0, 0};  // MODE_DENSE_CS1: tiles reduced per buffer (parity of part_full)
@@ -406,29 +487,39 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if (!ok) break;
           ++n_s;
           tc_fence_after();
+          const int valid = n_keys - j * 128;
+          if (__builtin_expect(valid < 128, 0)) {  // columns past the end of K
+            mask_columns(tS, valid, 128);
+            tmem_wait_st();
+          }
           uint32_t ra[64], rb[64];
           tmem_ld_16x256b_x16(tS, ra);
           tmem_ld_16x256b_x16(tS + (16u << 16), rb);
           tmem_wait_ld();
-          const int valid = n_keys - j * 128;
+          tc_fence_before();
+          mbar_arrive(&bars->s_read);
+          if (D == 128 && j > 0) {
+            // P of the tile before has been read.  Asked here, not where the answer is needed, with head dimension 128: 152
+            // against 168 us for 1600 x 4121 x 32 (the products of the two slots then alternate).
+            ok = __all_sync(0xffffffffu, mbar_wait(&bars->pv_done[s], n_pv & 1, wc, DEV_TIMEOUT_SOFTMAX));
+            if (!ok) break;
+            ++n_pv;
+            tc_fence_after();
+          }
           uint64_t acc2[16];
-          auto half_tile = [&](const uint32_t (&r)[64], int h, auto masked_tag) {
-            constexpr bool MASKED = decltype(masked_tag)::value;
+          auto half_tile = [&](const uint32_t (&r)[64], int h) {
             const uint64_t nA = pack_f32x2(ncst[2 * h], ncst[2 * h]), nB = pack_f32x2(ncst[2 * h + 1], ncst[2 * h + 1]);
             uint32_t pk[32];
+            bool pv_early = false;
 #pragma unroll
             for (int kk = 0; kk < 16; ++kk) {
+              if (D == 64 && h == 0 && kk == 12) pv_early = mbar_test_wait(&bars->pv_done[s], n_pv & 1);
               const uint64_t X = ffma2(pack_f32x2(__uint_as_float(r[4 * kk]), __uint_as_float(r[4 * kk + 1])), sc2, nA);
               const uint64_t Y = ffma2(pack_f32x2(__uint_as_float(r[4 * kk + 2]), __uint_as_float(r[4 * kk + 3])), sc2, nB);
               float x0, x1, y0, y1;
               unpack_f32x2(X, x0, x1);
               unpack_f32x2(Y, y0, y1);
               x0 = fast_exp2(x0); x1 = fast_exp2(x1); y0 = fast_exp2(y0); y1 = fast_exp2(y1);
-              if (MASKED) {  // columns past the end of K
-                const int c = 8 * kk + 2 * tc;
-                if (c >= valid) x0 = y0 = 0.f;
-                if (c + 1 >= valid) x1 = y1 = 0.f;
-              }
               const uint64_t PX = pack_f32x2(x0, x1), PY = pack_f32x2(y0, y1);
               rs2[2 * h] = fadd2(rs2[2 * h], PX);
               rs2[2 * h + 1] = fadd2(rs2[2 * h + 1], PY);
@@ -436,15 +527,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               pk[2 * kk] = pack_bf16x2(x0, x1);
               pk[2 * kk + 1] = pack_bf16x2(y0, y1);
             }
-            tmem_st_16x128b_x16(tS + ((uint32_t)(16 * h) << 16), pk);
+            if (D == 64 && h == 0 && j > 0) {
+              // the product that reads the P of the tile before is over (asked ahead: the answer is there by now)
+              if (!__all_sync(0xffffffffu, pv_early)) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&bars->pv_done[s], n_pv & 1, wc, DEV_TIMEOUT_SOFTMAX));
+                if (!ok) return;
+              }
+              ++n_pv;
+              tc_fence_after();
+            }
+            tmem_st_16x128b_x16(tP + ((uint32_t)(16 * h) << 16), pk);
           };
-          if (valid < 128) {
-            half_tile(ra, 0, std::true_type{});
-            half_tile(rb, 1, std::true_type{});
-          } else {
-            half_tile(ra, 0, std::false_type{});
-            half_tile(rb, 1, std::false_type{});
-          }
+          half_tile(ra, 0);
+          if (!ok) break;
+          half_tile(rb, 1);
           tmem_wait_st();
           tc_fence_before();
           mbar_arrive(&bars->p_full[s]);
@@ -512,6 +608,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         ++n_s;
         tc_fence_after();
 
+        const int valid = (MODE == MODE_CSP) ? (cnt_total - j * 128) : (p.Lkv - kvb * 128);
+        if (kMaskInTmem && __builtin_expect(valid < 128 || sub != 3u, 0)) {
+          // columns past the end of K, and (64-wide masks) the column half this row's half does not attend
+          if (!(sub & 1u)) mask_columns(tS, 0, 64);
+          mask_columns(tS, (sub & 2u) ? valid : min(valid, 64), 128);
+          tmem_wait_st();
+        }
         // raw fp32 bits of the S row, four 32-column chunks kept in registers
         uint32_t s0[32], s1[32], s2[32], s3[32];
         tmem_ld_x32(tS + 0, s0);
@@ -519,30 +622,25 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tmem_ld_x32(tS + 64, s2);
         tmem_ld_x32(tS + 96, s3);
         tmem_wait_ld();
-        if (MODE == MODE_CS_ONLY) {
-          // nothing goes back into S_s: the next tile's product may land while this one is exponentiated
-          tc_fence_before();
-          mbar_arrive(&bars->p_full[s]);
-        }
+        // the scores are in registers: the next product (the other slot's, or with MODE_CS_ONLY this slot's) may land
+        tc_fence_before();
+        mbar_arrive(&bars->s_read);
+        bool pv_waited = MODE == MODE_CS_ONLY || j == 0;  // the product that reads this slot's last P has completed
 
-        const int valid = (MODE == MODE_CSP) ? (cnt_total - j * 128) : (p.Lkv - kvb * 128);
-        if (valid < 128 || sub != 3u) {
-          // columns past the end of K, and (64-wide masks) the column half this row's half does not attend
-          const int lo = (sub & 1u) ? 0 : 64;
-          const int hi = (sub & 2u) ? valid : min(valid, 64);
+        if (!kMaskInTmem && __builtin_expect(valid < 128, 0)) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            if (i < lo || i >= hi) s0[i] = 0xff800000u;  // -inf
-            if (i + 32 < lo || i + 32 >= hi) s1[i] = 0xff800000u;
-            if (i + 64 < lo || i + 64 >= hi) s2[i] = 0xff800000u;
-            if (i + 96 < lo || i + 96 >= hi) s3[i] = 0xff800000u;
+            if (i >= valid) s0[i] = 0xff800000u;  // -inf
+            if (i + 32 >= valid) s1[i] = 0xff800000u;
+            if (i + 64 >= valid) s2[i] = 0xff800000u;
+            if (i + 96 >= valid) s3[i] = 0xff800000u;
           }
         }
         const float mx = fmax3(fmaxf(chunk_max(s0), chunk_max(s1)), chunk_max(s2), chunk_max(s3));
         const float mx_s = mx * p.scale_log2;
         m_true = fmaxf(m_true, mx_s);
         const bool need = mx_s > m_ref + kRescaleThreshold;
-        if (__any_sync(0xffffffffu, need)) {
+        if (__builtin_expect(__any_sync(0xffffffffu, need), 0)) {
           float alpha = 1.0f;
           if (need) {
             alpha = fast_exp2(m_ref - mx_s);
@@ -550,21 +648,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           }
           l *= alpha;
           if (MODE != MODE_CS_ONLY && it > 0) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&bars->pv_done[s], n_pv & 1, wc, DEV_TIMEOUT_SOFTMAX));
+            if (!ok) break;
+            ++n_pv;
+            pv_waited = true;
+            tc_fence_after();
             const uint64_t a2 = pack_f32x2(alpha, alpha);
-#pragma unroll
-            for (int c = 0; c < D / 32; ++c) {
-              uint32_t r[32];
-              tmem_ld_x32(tO + c * 32, r);
+#pragma unroll 1
+            for (int c = 0; c < D; c += 16) {
+              uint32_t r[16];
+              tmem_ld_x16(tO + c, r);
               tmem_wait_ld();
 #pragma unroll
-              for (int i = 0; i < 16; ++i) {
+              for (int i = 0; i < 8; ++i) {
                 const uint64_t t = fmul2(pack_f32x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), a2);
                 float x0, x1;
                 unpack_f32x2(t, x0, x1);
                 r[2 * i] = __float_as_uint(x0);
                 r[2 * i + 1] = __float_as_uint(x1);
               }
-              tmem_st_x32(tO + c * 32, r);
+              tmem_st_x16(tO + c, r);
             }
             tmem_wait_st();
           }
@@ -579,18 +682,24 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           exp_sum_chunk(s2, sc2, nm2, sum_a, sum_b);
           exp_sum_chunk(s3, sc2, nm2, sum_a, sum_b);
         } else {
-          {
-            uint32_t pk[32];
-            exp_pack_chunk(s0, sc2, nm2, sum_a, sum_b, pk, 0);
-            exp_pack_chunk(s1, sc2, nm2, sum_a, sum_b, pk, 16);
-            tmem_st_x32(tS, pk);
+          // P stays in registers until the whole row is done: by then the product that reads the P before it is over,
+          // as a rule (asked ahead, the answer is there when it is needed)
+          uint32_t pk[32], pk2[32];
+          exp_pack_chunk(s0, sc2, nm2, sum_a, sum_b, pk, 0);
+          exp_pack_chunk(s1, sc2, nm2, sum_a, sum_b, pk, 16);
+          exp_pack_chunk(s2, sc2, nm2, sum_a, sum_b, pk2, 0);
+          const bool pv_early = mbar_test_wait(&bars->pv_done[s], n_pv & 1);
+          exp_pack_chunk(s3, sc2, nm2, sum_a, sum_b, pk2, 16);
+          if (!pv_waited) {
+            if (!__all_sync(0xffffffffu, pv_early)) {
+              ok = __all_sync(0xffffffffu, mbar_wait(&bars->pv_done[s], n_pv & 1, wc, DEV_TIMEOUT_SOFTMAX));
+              if (!ok) break;
+            }
+            ++n_pv;
+            tc_fence_after();
           }
-          {
-            uint32_t pk[32];
-            exp_pack_chunk(s2, sc2, nm2, sum_a, sum_b, pk, 0);
-            exp_pack_chunk(s3, sc2, nm2, sum_a, sum_b, pk, 16);
-            tmem_st_x32(tS + 32, pk);
-          }
+          tmem_st_x32(tP, pk);
+          tmem_st_x32(tP + 32, pk2);
         }
         {
           float a0, a1, b0, b1;
@@ -658,9 +767,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       if (MODE != MODE_CS_ONLY) {
         if (it > 0) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_full[s], n_o & 1, wc, DEV_TIMEOUT_SOFTMAX));
+          ok = __all_sync(0xffffffffu, mbar_wait(&bars->pv_done[s], n_pv & 1, wc, DEV_TIMEOUT_SOFTMAX));
           if (!ok) break;
-          ++n_o;
+          ++n_pv;
           tc_fence_after();
         }
         if (split && s == 1) {
@@ -717,120 +826,71 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             tp = bilinear_taps(row / p.o_side, row % p.o_side, p.oi_side, p.oi_ratio);
             ibase = p.o_in + im.b * p.oi_sb + im.h * p.oi_sh;
           }
-          if (kRegisterEpilogue) {
-            // All of O_s goes to registers at once (the tile's S registers are dead here): one exposed TMEM
-            // latency instead of one per 32 columns, the accumulator is released before any arithmetic, and a row
-            // leaves in 32-byte stores.
-            uint32_t ra[D / 32][32];
+          // Sixteen columns at a time in a loop that is not unrolled: this code runs once per item, from instruction
+          // lines that the tile loop has displaced, and fetching them is what its time went into.
+#pragma unroll 1
+          for (int c = 0; c < D; c += 16) {
+            uint32_t r[16];
             if (it > 0) {
-#pragma unroll
-              for (int c = 0; c < D / 32; ++c) tmem_ld_x32(tO + c * 32, ra[c]);
+              tmem_ld_x16(tO + c, r);
               tmem_wait_ld();
             } else {
 #pragma unroll
-              for (int c = 0; c < D / 32; ++c)
-#pragma unroll
-                for (int i = 0; i < 32; ++i) ra[c][i] = 0u;
-            }
-            float wf = w0;
-            if (split && other) {
-#pragma unroll
-              for (int c = 0; c < D / 32; ++c) {
-                uint32_t r1[32];
-                tmem_ld_x32(tO1 + c * 32, r1);
-                tmem_wait_ld();
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                  ra[c][i] = __float_as_uint(fmaf(__uint_as_float(r1[i]), w1, __uint_as_float(ra[c][i]) * w0));
-              }
-              wf = 1.0f;
-            }
-            // O has been read out of TMEM: the MMA warp may overwrite it for the next item.  For a split tile
-            // this warpgroup read slot 1's accumulator too and releases it in its owner's stead.
-            tc_fence_before();
-            if (it > 0) mbar_arrive(&bars->o_empty[s]);
-            if (split && other) mbar_arrive(&bars->o_empty[1]);
-            if (row_ok) {
-#pragma unroll
-              for (int c = 0; c < D / 32; ++c) {
-#pragma unroll
-                for (int h8 = 0; h8 < 2; ++h8) {
-                  uint32_t w[8];
-#pragma unroll
-                  for (int i = 0; i < 8; ++i)
-                    w[i] = pack_bf16x2(__uint_as_float(ra[c][h8 * 16 + 2 * i]) * wf,
-                                       __uint_as_float(ra[c][h8 * 16 + 2 * i + 1]) * wf);
-                  if (p.o_align32) {
-                    st_global_v8(orow + c * 32 + h8 * 16, w);
-                  } else {
-                    *reinterpret_cast<uint4*>(orow + c * 32 + h8 * 16) = make_uint4(w[0], w[1], w[2], w[3]);
-                    *reinterpret_cast<uint4*>(orow + c * 32 + h8 * 16 + 8) = make_uint4(w[4], w[5], w[6], w[7]);
-                  }
-                }
-              }
-            }
-          } else {
-#pragma unroll
-          for (int c = 0; c < D / 32; ++c) {
-            uint32_t r[32];
-            if (it > 0) {
-              tmem_ld_x32(tO + c * 32, r);
-              tmem_wait_ld();
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = 0u;
+              for (int i = 0; i < 16; ++i) r[i] = 0u;
             }
             if (split && other) {
-              uint32_t r1[32];
-              tmem_ld_x32(tO1 + c * 32, r1);
+              uint32_t r1[16];
+              tmem_ld_x16(tO1 + c, r1);
               tmem_wait_ld();
 #pragma unroll
-              for (int i = 0; i < 32; ++i)
+              for (int i = 0; i < 16; ++i)
                 r[i] = __float_as_uint(fmaf(__uint_as_float(r1[i]), w1, __uint_as_float(r[i]) * w0));
             } else {
 #pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * w0);
-            }
-            if (c == D / 32 - 1) {
-              // O has been read out of TMEM: the MMA warp may overwrite it for the next item.  For a split tile
-              // this warpgroup read slot 1's accumulator too and releases it in its owner's stead.
-              tc_fence_before();
-              if (it > 0) mbar_arrive(&bars->o_empty[s]);
-              if (split && other) mbar_arrive(&bars->o_empty[1]);
+              for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * w0);
             }
             if (row_ok) {
+              uint32_t w[8];
 #pragma unroll
-              for (int q4 = 0; q4 < 4; ++q4) {
-                uint32_t w[4];
+              for (int i = 0; i < 8; ++i) w[i] = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+              if (MODE == MODE_CSP) {
+                // out = bf16(o_in + o_scale * bf16(delta)): same rounding points as the reference's
+                // `o + o_delta * o_scale` on bf16 tensors (kernels/sparse_attn/sparse_attn_ops.py:288).
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                  w[i] = pack_bf16x2(__uint_as_float(r[q4 * 8 + 2 * i]), __uint_as_float(r[q4 * 8 + 2 * i + 1]));
-                if (MODE == MODE_CSP) {
-                  // out = bf16(o_in + o_scale * bf16(delta)): same rounding points as the reference's
-                  // `o + o_delta * o_scale` on bf16 tensors (kernels/sparse_attn/sparse_attn_ops.py:288).
+                for (int h8 = 0; h8 < 2; ++h8) {
                   uint4 prev;
                   if (resize) {
-                    const __nv_bfloat16* ib = ibase + c * 32 + q4 * 8;
+                    const __nv_bfloat16* ib = ibase + c + h8 * 8;
                     prev = bilinear_mix8(tp, *reinterpret_cast<const uint4*>(ib + (int64_t)tp.r00 * p.oi_sl),
                                          *reinterpret_cast<const uint4*>(ib + (int64_t)tp.r01 * p.oi_sl),
                                          *reinterpret_cast<const uint4*>(ib + (int64_t)tp.r10 * p.oi_sl),
                                          *reinterpret_cast<const uint4*>(ib + (int64_t)tp.r11 * p.oi_sl));
                   } else {
-                    prev = *reinterpret_cast<const uint4*>(irow + c * 32 + q4 * 8);
+                    prev = *reinterpret_cast<const uint4*>(irow + c + h8 * 8);
                   }
                   const uint32_t pv[4] = {prev.x, prev.y, prev.z, prev.w};
 #pragma unroll
                   for (int i = 0; i < 4; ++i) {
-                    const float d0 = __uint_as_float(w[i] << 16), d1 = __uint_as_float(w[i] & 0xffff0000u);
+                    const uint32_t d = w[h8 * 4 + i];
+                    const float d0 = __uint_as_float(d << 16), d1 = __uint_as_float(d & 0xffff0000u);
                     const float a0 = __uint_as_float(pv[i] << 16), a1 = __uint_as_float(pv[i] & 0xffff0000u);
-                    w[i] = pack_bf16x2(fmaf(p.o_scale, d0, a0), fmaf(p.o_scale, d1, a1));
+                    w[h8 * 4 + i] = pack_bf16x2(fmaf(p.o_scale, d0, a0), fmaf(p.o_scale, d1, a1));
                   }
                 }
-                *reinterpret_cast<uint4*>(orow + c * 32 + q4 * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+              }
+              if (p.o_align32) {
+                st_global_v8(orow + c, w);
+              } else {
+                *reinterpret_cast<uint4*>(orow + c) = make_uint4(w[0], w[1], w[2], w[3]);
+                *reinterpret_cast<uint4*>(orow + c + 8) = make_uint4(w[4], w[5], w[6], w[7]);
               }
             }
           }
-          }
+          // O has been read out of TMEM: the P V issuer may overwrite it for the next item.  For a split tile this
+          // warpgroup read slot 1's accumulator too and releases it in its owner's stead.
+          tc_fence_before();
+          if (it > 0) mbar_arrive(&bars->o_empty[s]);
+          if (split && other) mbar_arrive(&bars->o_empty[1]);
         }
       }
       if (stats_given) {
@@ -879,13 +939,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         auto cs_sweep = [&](auto poly_tag) -> bool {
           constexpr uint32_t POLY = decltype(poly_tag)::value;
           for (int j = 0; j < n_mine; ++j) {
-            // tile j of the sweep sits in buffer j % kCsBufs: S_s, or the (by now written out) O region
-            const int buf = j % kCsBufs;
-            ok = __all_sync(0xffffffffu, mbar_wait(&bars->cs_full[s][buf], n_cs[buf] & 1, wc, DEV_TIMEOUT_SOFTMAX));
+            ok = __all_sync(0xffffffffu, mbar_wait(&bars->cs_full[s], n_cs & 1, wc, DEV_TIMEOUT_SOFTMAX));
             if (!ok) return false;
-            ++n_cs[buf];
+            ++n_cs;
             tc_fence_after();
-            const uint32_t tT = buf == 0 ? tS : tmem_base + lane_off + TM_O + (uint32_t)s * 128u;
             float acc = 0.f;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -894,9 +951,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               tmem_wait_ld();
               acc += colsum_chunk<POLY>(r, nc4 + c * 8, sc2);
             }
-            // S^T has been read: the MMA warp may overwrite the buffer with the tile after the next
+            // S^T has been read: the next product may land
             tc_fence_before();
-            mbar_arrive(&bars->cs_empty[s][buf]);
+            mbar_arrive(&bars->cs_empty[s]);
             const int key = j * 128 + r_in_tile;
             if (key < n_keys) {
               // two addends onto zero give the same bits in either order
@@ -915,11 +972,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
     }
   } else if (warp == 8) {
-    // ============================================================ K (and Q) loader
+    // ============================================================ Q, K and V loader; column-sparse: Q loader, K gather
     setmaxnreg_dec<kRegsOther>();
     bool ok = true;
-    int kc = 0;       // K tiles issued so far (stage = kc % kStages)
-    int nq_items = 0; // items with at least one step (parity of q_full / q_empty)
+    int kc = 0, vc = 0;  // K and V tiles issued so far (stage = count % kStages)
+    int nq_items = 0;    // items with at least one step (parity of q_full / q_empty)
     const bool issuer = (MODE == MODE_CSP) || lane == 0;
     if (issuer) {
       for (int n = 0; ok; ++n) {
@@ -961,6 +1018,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 tma_load_4d(sK + st * SM::kTile + sub * 16384, &tmK, &bars->k_full[st], sub * 64, rd.kvb[s] * 128, im.h,
                             im.b);
               ++kc;
+            }
+            // V behind K in one thread: loads of V by a thread of its own measured slower (dense 4096 x 10521 x 32 537 us
+            // against 527, block-sparse 160 against 148)
+            if (MODE != MODE_CS_ONLY && rr < rounds) {
+              for (int s = 0; s < 2 && ok; ++s) {
+                if (!rd.has[s] || (s == 1 && rd.shared)) continue;
+                const int st = vc % kStages;
+                ok = mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER);
+                if (!ok) break;
+                mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile);
+                for (int sub = 0; sub < NSUB; ++sub)
+                  tma_load_4d(sV + st * SM::kTile + sub * 16384, &tmV, &bars->v_full[st], sub * 64, rd.kvb[s] * 128, im.h,
+                              im.b);
+                ++vc;
+              }
             }
           }
         } else {
@@ -1007,88 +1079,78 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                    globaltimer_ns() - t1 < 2000000000ull) {
             }
           }
+          for (int c = max(0, vc - kStages); c < vc; ++c) {
+            const uint64_t t1 = globaltimer_ns();
+            while (!mbar_try_wait(&bars->v_full[c % kStages], (c / kStages) & 1) &&
+                   globaltimer_ns() - t1 < 2000000000ull) {
+            }
+          }
         }
       }
     }
     __syncwarp();
   } else if (warp == 9) {
-    // ============================================================ V loader
+    // ============================================================ P V issuer; column-sparse: V gather
     setmaxnreg_dec<kRegsOther>();
     bool ok = true;
-    int vc = 0;
-    const bool issuer = (MODE == MODE_CSP) || lane == 0;
-    if (issuer) {
+    if (MODE == MODE_CSP) {
+      int vc = 0;
       for (int n = 0; ok; ++n) {
         SchedEntry e;
-        ok = acquire_item(n, e, DEV_TIMEOUT_PRODUCER);
-        if (MODE == MODE_CSP) ok = __all_sync(0xffffffffu, ok);
+        ok = __all_sync(0xffffffffu, acquire_item(n, e, DEV_TIMEOUT_PRODUCER));
         if (!ok || e.item < 0) break;
         const Item im = decode(e.item, e.half);
-        const uint16_t* l0 = lists + ((n % kSchedStages) * 2) * kMaxSteps;
-        const uint16_t* l1 = l0 + kMaxSteps;
         const int rounds = max(e.n0, e.n1);
-        if (MODE == MODE_CS_ONLY) {
-          // no V in this mode: the warp only follows the schedule
-        } else if (MODE != MODE_CSP) {
-          for (int r = 0; r < rounds && ok; ++r) {
-            const Round rd = round_info(l0, l1, e, r);
-            for (int s = 0; s < 2; ++s) {
-              if (!rd.has[s] || (s == 1 && rd.shared)) continue;
-              const int st = vc % kStages;
-              ok = mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER);
-              if (!ok) break;
+        const int32_t* idx = p.indices + im.b * p.i_sb + im.h * p.i_sh + (int64_t)im.group * p.i_sg;
+        const __nv_bfloat16* vbase = p.v + im.b * p.v_sb + im.h * p.v_sh;
+        int kv[4];
+        if (rounds > 0) gather_rows_of_tile(kv, idx, e.aux, 0, p.Lkv, lane, nullptr);
+        for (int j = 0; j < rounds; ++j) {
+          const int st = vc % kStages;
+          ok = __all_sync(0xffffffffu, mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
+          if (!ok) break;
+          if (tile_is_run(kv, e.aux, j, p.Lkv, lane)) {
+            if (lane == 0) {
               mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile);
               for (int sub = 0; sub < NSUB; ++sub)
-                tma_load_4d(sV + st * SM::kTile + sub * 16384, &tmV, &bars->v_full[st], sub * 64, rd.kvb[s] * 128, im.h,
-                            im.b);
-              ++vc;
-            }
-          }
-        } else {
-          const int32_t* idx = p.indices + im.b * p.i_sb + im.h * p.i_sh + (int64_t)im.group * p.i_sg;
-          const __nv_bfloat16* vbase = p.v + im.b * p.v_sb + im.h * p.v_sh;
-          int kv[4];
-          if (rounds > 0) gather_rows_of_tile(kv, idx, e.aux, 0, p.Lkv, lane, nullptr);
-          for (int j = 0; j < rounds; ++j) {
-            const int st = vc % kStages;
-            ok = __all_sync(0xffffffffu, mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
-            if (!ok) break;
-            if (tile_is_run(kv, e.aux, j, p.Lkv, lane)) {
-              if (lane == 0) {
-                mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile);
-                for (int sub = 0; sub < NSUB; ++sub)
-                  tma_load_4d(sV + st * SM::kTile + sub * 16384, &tmV, &bars->v_full[st], sub * 64, kv[0], im.h, im.b);
-              } else {
-                mbar_arrive(&bars->v_full[st]);
-              }
+                tma_load_4d(sV + st * SM::kTile + sub * 16384, &tmV, &bars->v_full[st], sub * 64, kv[0], im.h, im.b);
             } else {
-              gather_tile<D>(smem_u32(sV + st * SM::kTile), vbase, p.v_sl, kv, lane);
-              cp_async_mbar_arrive(&bars->v_full[st]);
+              mbar_arrive(&bars->v_full[st]);
             }
-            if (j + 1 < rounds) gather_rows_of_tile(kv, idx, e.aux, j + 1, p.Lkv, lane, nullptr);
-            ++vc;
+          } else {
+            gather_tile<D>(smem_u32(sV + st * SM::kTile), vbase, p.v_sl, kv, lane);
+            cp_async_mbar_arrive(&bars->v_full[st]);
           }
+          if (j + 1 < rounds) gather_rows_of_tile(kv, idx, e.aux, j + 1, p.Lkv, lane, nullptr);
+          ++vc;
         }
         if (!ok) break;
         if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
       }
-      if (MODE == MODE_CSP) cp_async_wait<0>();
-      if (MODE != MODE_CSP && lane == 0 && bars->abort_flag) {
-        for (int c = max(0, vc - kStages); c < vc; ++c) {
-          const uint64_t t1 = globaltimer_ns();
-          while (!mbar_try_wait(&bars->v_full[c % kStages], (c / kStages) & 1) &&
-                 globaltimer_ns() - t1 < 2000000000ull) {
-          }
+      cp_async_wait<0>();
+    } else if (elect_one()) {
+      // One lane runs the whole role: the issue of sixteen MMAs took it 640 cycles against 880 for a warp that runs
+      // the bookkeeping on all lanes and predicates the issue (1024 is what they execute in).
+      PvState ps;
+      for (int n = 0; ok; ++n) {
+        SchedEntry e;
+        ok = acquire_item(n, e, DEV_TIMEOUT_MMA);
+        if (!ok || e.item < 0) break;
+        if (MODE != MODE_CS_ONLY) {
+          ok = pv_rounds(ps, e, n, 0, max(e.n0, e.n1));
+          if (!ok) break;
+          pv_end(ps, e);
         }
+        mbar_arrive(&bars->sched_empty[n % kSchedStages]);
       }
+      drain_mma(&bars->mma_done[1]);
     }
     __syncwarp();
   } else if (warp == 10) {
-    // ============================================================ MMA issuer (one thread)
+    // ============================================================ Q K^T issuer (and the column-sum sweep's products)
     setmaxnreg_dec<kRegsOther>();
-    // Every lane runs the (warp-uniform) bookkeeping; lane 0 alone issues the MMAs, commits and arrivals.
-    const uint32_t leader = lane == 0 ? 1u : 0u;
-    {
+    if (elect_one()) {
+      constexpr uint32_t leader = 1u;
       bool ok = true;
       // Descriptor words: the high word is the same for every operand tile, the low word is the tile's
       // base plus (byte offset >> 4) of the stage and of the 16-element K step.
@@ -1096,12 +1158,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       constexpr uint32_t TILE16 = SM::kTile >> 4;
       const uint32_t q_lo = sw128_desc_lo(smem_u32(sQ), 16);
       const uint32_t k_lo = sw128_desc_lo(smem_u32(sK), 16);
-      const uint32_t v_lo = sw128_desc_lo(smem_u32(sV), 16384);
-      int kc = 0, vc = 0;        // K / V tiles consumed so far
+      int kc = 0;                // K tiles consumed so far
       int nq_items = 0;          // items with steps (parity of q_full)
-      int n_p[2] = {0, 0};       // P tiles consumed per slot (parity of p_full)
-      int n_o[2] = {0, 0};       // items in which the slot produced an output (parity of o_empty)
-      int n_cst[2][2] = {{0, 0}, {0, 0}};  // column-sum sweep: S^T tiles issued per [slot][buffer]
+      uint32_t n_sr = 1;         // score tiles issued, of either slot (parity of s_read of the one before)
+      uint32_t n_cst[2] = {1, 1};  // column-sum sweep: S^T tiles issued per buffer (parity of cs_empty)
       for (int n = 0; ok; ++n) {
         SchedEntry e;
         ok = acquire_item(n, e, DEV_TIMEOUT_MMA);
@@ -1115,161 +1175,100 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if (!ok) break;
           ++nq_items;
         }
-        Round prev;
-        prev.has[0] = prev.has[1] = prev.shared = false;
-        prev.kvb[0] = prev.kvb[1] = 0;
-        int pvs[2] = {0, 0}, pvp[2] = {0, 0};  // V stage / parity of the previous round, per slot
-        int npv[2] = {0, 0};
         const int rounds_first = stats_given ? 0 : rounds;
-        for (int r = 0; r <= rounds_first && ok; ++r) {
-          Round cur;
-          cur.has[0] = cur.has[1] = cur.shared = false;
-          cur.kvb[0] = cur.kvb[1] = 0;
-          if (r < rounds_first) cur = round_info(l0, l1, e, r);
-          // stages of this round's tiles (same order as the loaders issue them)
-          int ks[2] = {0, 0}, kp[2] = {0, 0}, vs[2] = {0, 0}, vp[2] = {0, 0};
-          for (int s = 0; s < 2; ++s) {
-            if (!cur.has[s]) continue;
-            if (s == 1 && cur.shared) {
-              ks[1] = ks[0]; kp[1] = kp[0]; vs[1] = vs[0]; vp[1] = vp[0];
-              continue;
-            }
-            ks[s] = kc % kStages; kp[s] = (kc / kStages) & 1; ++kc;
-            vs[s] = vc % kStages; vp[s] = (vc / kStages) & 1; ++vc;
-          }
-          for (int s = 0; s < 2 && ok; ++s) {
-            if (prev.has[s] && MODE == MODE_CS_ONLY) {
-              // statistics sweep: no PV; S_s is free again once the softmax warps have read the last product
-              ok = mbar_wait(&bars->p_full[s], n_p[s] & 1, wc, DEV_TIMEOUT_MMA);
-              if (!ok) break;
-              ++n_p[s];
-            } else if (prev.has[s]) {
-              if (!(s == 1 && prev.shared)) {
-                ok = mbar_wait(&bars->v_full[pvs[s]], pvp[s], wc, DEV_TIMEOUT_MMA);
-                if (!ok) break;
-              }
-              if (npv[s] == 0) {
-                // first PV of the item overwrites O_s: the previous item's epilogue must have read it
-                ok = mbar_wait(&bars->o_empty[s], (n_o[s] & 1) ^ 1, wc, DEV_TIMEOUT_MMA);
-                if (!ok) break;
-              }
-              ok = mbar_wait(&bars->p_full[s], n_p[s] & 1, wc, DEV_TIMEOUT_MMA);
-              if (!ok) break;
-              ++n_p[s];
-              // column-sparse: V came by cp.async (generic proxy), the MMA reads it through the async proxy
-              if (MODE == MODE_CSP) fence_proxy_async_smem();
-              tc_fence_after();
-              const uint32_t tP = tmem_base + (uint32_t)s * 128u;
-              const uint32_t tOs = tmem_base + TM_O + (uint32_t)s * D;
-              const uint32_t vb = v_lo + (uint32_t)pvs[s] * TILE16;
-              umma_ts_if(leader, tOs, tP, vb, DESC_HI, IDESC_PV, npv[s] > 0 ? 1u : 0u);
+        // S_s = Q_s K^T of one tile, once the buffer it lands in has been read
+        auto product = [&](auto s_tag, int st, bool wait_k) -> bool {
+          constexpr int s = decltype(s_tag)::value;
+          if (wait_k && !mbar_wait(&bars->k_full[st], (kc >> 1) & 1, wc, DEV_TIMEOUT_MMA)) return false;
+          // the scores of the product before (the other slot's, as a rule) have left the score buffer
+          if (!mbar_wait(&bars->s_read, n_sr & 1, wc, DEV_TIMEOUT_MMA)) return false;
+          ++n_sr;
+          // column-sparse: K came by cp.async (generic proxy), the MMA reads it through the async proxy
+          if (MODE == MODE_CSP && wait_k) fence_proxy_async_smem();
+          tc_fence_after();
+          const uint32_t tSs = tmem_base + TM_S;
+          const uint32_t qa = q_lo + (uint32_t)s * TILE16, kb = k_lo + (uint32_t)st * TILE16;
 #pragma unroll
-              for (int ks8 = 1; ks8 < 8; ++ks8)
-                umma_ts_if(leader, tOs, tP + ks8 * 8, vb + ks8 * 128, DESC_HI, IDESC_PV, 1u);
-              ++npv[s];
-              // release the V stage after its last user
-              if (!(s == 0 && prev.shared)) umma_commit_if(leader, &bars->v_empty[pvs[s]]);
-            }
-            if (cur.has[s]) {
-              if (!(s == 1 && cur.shared)) {
-                ok = mbar_wait(&bars->k_full[ks[s]], kp[s], wc, DEV_TIMEOUT_MMA);
-                if (!ok) break;
-                if (MODE == MODE_CSP) fence_proxy_async_smem();
-                tc_fence_after();
-              }
-              const uint32_t tSs = tmem_base + (uint32_t)s * 128u;
-              const uint32_t qa = q_lo + (uint32_t)s * TILE16, kb = k_lo + (uint32_t)ks[s] * TILE16;
-#pragma unroll
-              for (int kq = 0; kq < KSTEPS_QK; ++kq) {
-                const uint32_t koff = (kq >> 2) * 1024 + (kq & 3) * 2;  // (byte offset of the K step) >> 4
-                umma_ss_if(leader, tSs, qa + koff, DESC_HI, kb + koff, DESC_HI, IDESC_QK, kq > 0 ? 1u : 0u);
-              }
-              umma_commit_if(leader, &bars->s_full[s]);
-              if (!(s == 0 && cur.shared)) umma_commit_if(leader, &bars->k_empty[ks[s]]);
-            }
+          for (int kq = 0; kq < KSTEPS_QK; ++kq) {
+            const uint32_t koff = (kq >> 2) * 1024 + (kq & 3) * 2;  // (byte offset of the K step) >> 4
+            umma_ss_if(leader, tSs, qa + koff, DESC_HI, kb + koff, DESC_HI, IDESC_QK, kq > 0 ? 1u : 0u);
           }
-          if (!ok) break;
-          prev = cur;
-          pvs[0] = vs[0]; pvs[1] = vs[1]; pvp[0] = vp[0]; pvp[1] = vp[1];
-        }
-        if (!ok) break;
-        for (int s = 0; s < 2; ++s) {
-          if (npv[s] > 0) {
-            umma_commit_if(leader, &bars->o_full[s]);
-            ++n_o[s];
-          }
-        }
-        if (kHasCs) {
-          // ---- column-sum sweep: S_s^T = K Q_s^T per KV tile (the operands swap roles, the tiles stay where
-          // they are); a slot's next product waits until its softmax warps have read the previous one.
-          for (int r = 0; r < rounds && ok; ++r) {
-            const Round cur = round_info(l0, l1, e, r);
-            int ks = 0, kp = 0;
-            if (cur.has[0] || cur.has[1]) {
-              ks = kc % kStages;
-              kp = (kc / kStages) & 1;
+          umma_commit(&bars->s_full[s]);
+          return true;
+        };
+        for (int r = 0; r < rounds_first && ok; ++r) {
+          const bool h0 = r < e.n0, h1 = r < e.n1, shared = round_shared(l0, l1, e, r);
+          if (h0) {
+            const int st = kc & 1;
+            ok = product(std::integral_constant<int, 0>{}, st, true);
+            if (!ok) break;
+            if (!shared) {
+              umma_commit(&bars->k_empty[st]);
               ++kc;
             }
-            const int buf = r % kCsBufs;
-            bool waited = false;
-            for (int s = 0; s < 2 && ok; ++s) {
-              if (!cur.has[s]) continue;
-              // the buffer is free once the softmax warps have read the tile before the previous one out of it
-              if (n_cst[s][buf] > 0) {
-                ok = mbar_wait(&bars->cs_empty[s][buf], (n_cst[s][buf] - 1) & 1, wc, DEV_TIMEOUT_MMA);
-                if (!ok) break;
-              }
-              if (kCsBufs == 2 && r == 1) {
-                // first use of the second buffer, which lies over the O accumulators (over both slots' when the
-                // head dimension is 64): this item's epilogues must have read them
-                for (int t = 0; t < 2 && ok; ++t)
-                  if (t == s || D == 64) ok = mbar_wait(&bars->o_empty[t], (n_o[t] & 1) ^ 1, wc, DEV_TIMEOUT_MMA);
-                if (!ok) break;
-              }
-              if (SPLIT && s == 1 && im.split) {  // the slots of a split tile have a K tile each
-                ks = kc % kStages;
-                kp = (kc / kStages) & 1;
-                ++kc;
-                waited = false;
-              }
-              if (!waited) {
-                ok = mbar_wait(&bars->k_full[ks], kp, wc, DEV_TIMEOUT_MMA);
-                if (!ok) break;
-                waited = true;
-              }
-              tc_fence_after();
-              const uint32_t tT = tmem_base + (buf == 0 ? (uint32_t)s * 128u : TM_O + (uint32_t)s * 128u);
-              const uint32_t qb = q_lo + (uint32_t)s * TILE16, ka = k_lo + (uint32_t)ks * TILE16;
+          }
+          if (h1) {
+            const int st = kc & 1;
+            ok = product(std::integral_constant<int, 1>{}, st, !shared);
+            if (!ok) break;
+            umma_commit(&bars->k_empty[st]);
+            ++kc;
+          }
+        }
+        if (!ok) break;
+        if (kHasCs) {
+          if (rounds_first > 0) {
+            // S^T of both slots lies over the score buffer and over P0 and P1: the last scores have been read and the last
+            // P V products have completed
+            ok = mbar_wait(&bars->s_read, n_sr & 1, wc, DEV_TIMEOUT_MMA) &&
+                 (MODE == MODE_CS_ONLY || mbar_wait(&bars->pv_all, (nq_items - 1) & 1, wc, DEV_TIMEOUT_MMA));
+            if (!ok) break;
+          }
+          // ---- column-sum sweep: S_s^T = K Q_s^T per KV tile (the operands swap roles, the tiles stay where they are)
+          auto sweep_product = [&](auto s_tag, int st, bool wait_k) -> bool {
+            constexpr int s = decltype(s_tag)::value, b = s;
+            if (wait_k && !mbar_wait(&bars->k_full[st], (kc >> 1) & 1, wc, DEV_TIMEOUT_MMA)) return false;
+            if (!mbar_wait(&bars->cs_empty[b], n_cst[b] & 1, wc, DEV_TIMEOUT_MMA)) return false;
+            ++n_cst[b];
+            tc_fence_after();
+            const uint32_t tT = tmem_base + (uint32_t)s * 128u;
+            const uint32_t qb = q_lo + (uint32_t)s * TILE16, ka = k_lo + (uint32_t)st * TILE16;
 #pragma unroll
-              for (int kq = 0; kq < KSTEPS_QK; ++kq) {
-                const uint32_t koff = (kq >> 2) * 1024 + (kq & 3) * 2;
-                umma_ss_if(leader, tT, ka + koff, DESC_HI, qb + koff, DESC_HI, IDESC_QK, kq > 0 ? 1u : 0u);
+            for (int kq = 0; kq < KSTEPS_QK; ++kq) {
+              const uint32_t koff = (kq >> 2) * 1024 + (kq & 3) * 2;
+              umma_ss_if(leader, tT, ka + koff, DESC_HI, qb + koff, DESC_HI, IDESC_QK, kq > 0 ? 1u : 0u);
+            }
+            umma_commit_if(leader, &bars->cs_full[s]);
+            return true;
+          };
+          for (int r = 0; r < rounds && ok; ++r) {
+            const bool h0 = r < e.n0, h1 = r < e.n1, shared = round_shared(l0, l1, e, r);
+            if (h0) {
+              const int st = kc & 1;
+              ok = sweep_product(std::integral_constant<int, 0>{}, st, true);
+              if (!ok) break;
+              if (!shared) {
+                umma_commit_if(leader, &bars->k_empty[st]);
+                ++kc;
               }
-              umma_commit_if(leader, &bars->cs_full[s][buf]);
-              ++n_cst[s][buf];
-              if (s == 1 || !cur.has[1] || (SPLIT && im.split)) umma_commit_if(leader, &bars->k_empty[ks]);  // last reader of the K stage
+            }
+            if (h1) {
+              const int st = kc & 1;
+              ok = sweep_product(std::integral_constant<int, 1>{}, st, !shared);
+              if (!ok) break;
+              umma_commit_if(leader, &bars->k_empty[st]);
+              ++kc;
             }
           }
-          // the next item's attention sweep writes S_s and O_s again: the softmax warps' last reads first
-          for (int s = 0; s < 2 && ok; ++s)
-            for (int b = 0; b < 2 && ok; ++b)
-              if (n_cst[s][b] > 0) ok = mbar_wait(&bars->cs_empty[s][b], (n_cst[s][b] - 1) & 1, wc, DEV_TIMEOUT_MMA);
+          // the next item's products land in the same columns: the softmax warps' last reads first
+          if (ok) ok = mbar_wait(&bars->cs_empty[0], n_cst[0] & 1, wc, DEV_TIMEOUT_MMA) &&
+                       mbar_wait(&bars->cs_empty[1], n_cst[1] & 1, wc, DEV_TIMEOUT_MMA);
           if (!ok) break;
         }
-        if (rounds > 0) umma_commit_if(leader, &bars->q_empty);
-        if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
+        if (rounds > 0) umma_commit(&bars->q_empty);
+        mbar_arrive(&bars->sched_empty[n % kSchedStages]);
       }
-      // TMEM must not be freed (nor the CTA retire) while an MMA is still in flight, also on abort.
-      if (lane == 0) {
-        umma_commit(&bars->mma_done);
-        const uint64_t t0 = globaltimer_ns();
-        while (!mbar_try_wait(&bars->mma_done, 0)) {
-          if (globaltimer_ns() - t0 > 2000000000ull) {
-            if (p.status) atomicCAS(p.status, 0, (int)DEV_TIMEOUT_DRAIN);
-            break;
-          }
-        }
-      }
+      drain_mma(&bars->mma_done[0]);
     }
     __syncwarp();
   } else {
@@ -1281,12 +1280,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     // under the tail of the grid before this one in the stream; the work counter, the inputs and the output
     // are only touched after that grid has completed.  Every other role starts from an item this warp publishes.
     griddep_wait();
-    bool ok = true;
-    for (int n = 0; ok; ++n) {
+    // takes the next work item and publishes it as the CTA's n-th; false on abort
+    auto publish = [&](int n) -> bool {
       const int slot = n % kSchedStages;
-      ok = __all_sync(0xffffffffu,
-                      mbar_wait(&bars->sched_empty[slot], ((n / kSchedStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
-      if (!ok) break;
+      if (!__all_sync(0xffffffffu,
+                      mbar_wait(&bars->sched_empty[slot], ((n / kSchedStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER)))
+        return false;
       int item = -1, half = -1;
       if (lane == 0) {
         const int idx = atomicAdd(p.sched_counter, 1);
@@ -1385,7 +1384,37 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         bars->sched[slot].aux = aux;
         mbar_arrive(&bars->sched_full[slot]);
       }
-      if (item < 0) break;
+      __syncwarp();
+      return true;
+    };
+    if (MODE == MODE_CSP) {
+      // column-sparse: this warp issues the P V products as well (warps 8 and 9 gather rows); the next item is taken
+      // after the second round of the present one
+      PvState ps;
+      bool ok = publish(0);
+      for (int n = 0; ok; ++n) {
+        const SchedEntry e = bars->sched[n % kSchedStages];
+        if (e.item < 0) break;
+        const int rounds = max(e.n0, e.n1);
+        if (lane == 0) ok = pv_rounds(ps, e, n, 0, min(2, rounds));
+        ok = __all_sync(0xffffffffu, ok) && publish(n + 1);
+        if (ok && lane == 0) {
+          ok = pv_rounds(ps, e, n, 2, rounds);
+          if (ok) pv_end(ps, e);
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
+      }
+      if (lane == 0) drain_mma(&bars->mma_done[1]);
+      __syncwarp();
+    } else {
+      bool ok = publish(0);
+      for (int n = 0; ok; ++n) {
+        if (bars->sched[n % kSchedStages].item < 0) break;
+        ok = publish(n + 1);
+        if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
+      }
+      __syncwarp();
     }
     if (lane == 0) {
       __threadfence();

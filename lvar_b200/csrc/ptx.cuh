@@ -74,6 +74,21 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// One look at a phase, without waiting.
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Shared per-CTA wait context: every wait in a kernel is bounded.  `abort_flag` lives in shared
 // memory; once any role times out it is raised so the other roles leave their waits promptly
 // instead of each sitting out its own limit.
@@ -84,18 +99,21 @@ struct WaitCtx {
 };
 
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const WaitCtx& w, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (__builtin_expect(mbar_try_wait(bar, parity), 1)) return true;
   if (w.limit_ns == 0) {
     if (w.status) atomicCAS(w.status, 0, (int)DEV_FORCED_TIMEOUT);
     *w.abort_flag = 1;
     return false;
   }
-  const uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;
   uint32_t spins = 0;
   while (!mbar_try_wait(bar, parity)) {
-    if ((++spins & 63u) == 0) {
+    if (__builtin_expect((++spins & 255u) == 0, 0)) {
       if (*w.abort_flag) return false;
-      if (globaltimer_ns() - t0 > w.limit_ns) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) {
+        t0 = now;
+      } else if (now - t0 > w.limit_ns) {
         if (w.status) atomicCAS(w.status, 0, code);
         *w.abort_flag = 1;
         return false;
@@ -304,6 +322,38 @@ __device__ __forceinline__ void tmem_st_x32(uint32_t taddr, const uint32_t (&r)[
         "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
         "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
+}
+__device__ __forceinline__ void tmem_ld_x16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      :
+      : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+// Columns [a, b) of the warp's 32 TMEM lanes become -inf (a, b warp-uniform).
+__device__ __forceinline__ void mask_columns(uint32_t taddr, int a, int b) {
+  const uint32_t ninf = 0xff800000u;
+#pragma unroll 1
+  while (a < b) {
+    if ((a & 7) == 0 && a + 8 <= b) {
+      asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr + a),
+                   "r"(ninf)
+                   : "memory");
+      a += 8;
+    } else {
+      asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr + a), "r"(ninf) : "memory");
+      ++a;
+    }
+  }
 }
 // Warp-collective TMEM load in the 16x256b shape, 16 repetitions: 16 TMEM lanes (starting at the lane in taddr,
 // which must be the base of the warp's 32-lane window or that base + 16) x 128 columns.  Thread t receives, for
