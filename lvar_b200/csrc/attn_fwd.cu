@@ -49,7 +49,7 @@ namespace {
 constexpr int kThreads = 384;  // 8 softmax warps, loader, P V issuer, Q K^T issuer, scheduler
 constexpr int kRegsSoftmax = 208, kRegsOther = 72;
 constexpr int kMaxSteps = 1024;  // per-slot KV tile list capacity (block-sparse: Lkv <= 131072)
-constexpr int kStages = 2;
+constexpr int kMaxStages = 4;  // of K and of V each
 constexpr int kSchedStages = 2;
 // Column-sum sweep: which of the 8 groups of four exponentials per 32-column chunk are evaluated on the FMA
 // pipe (polynomial) instead of the exp2 unit, the sweep's bottleneck.  A quarter of them measured best
@@ -124,6 +124,9 @@ struct AttnParams {
 template <int D>
 struct Smem {
   static constexpr int kTile = 128 * D * 2;  // bytes of one Q/K/V tile
+  // Tiles in flight, of K and of V each.  What shared memory holds beside Q: two with head dimension 128; four with 64
+  // (block-sparse 4 x 16 x 4096 x 8192: 176 us with two, 157 with four).
+  static constexpr int kStages = D == 64 ? 4 : 2;
   static constexpr int kQ = 0;
   static constexpr int kK = kQ + 2 * kTile;
   static constexpr int kV = kK + kStages * kTile;
@@ -162,8 +165,8 @@ struct Round {
 
 struct Bars {
   uint64_t q_full, q_empty;
-  uint64_t k_full[kStages], k_empty[kStages];
-  uint64_t v_full[kStages], v_empty[kStages];
+  uint64_t k_full[kMaxStages], k_empty[kMaxStages];
+  uint64_t v_full[kMaxStages], v_empty[kMaxStages];
   uint64_t s_full[2], s_read, p_full[2], pv_done[2], o_empty[2];
   uint64_t sched_full[kSchedStages], sched_empty[kSchedStages];
   uint64_t mma_done[2];  // [Q K^T issuer, P V issuer]
@@ -191,6 +194,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const AttnParams p) {
   using SM = Smem<D>;
+  constexpr int kStages = SM::kStages;
   constexpr int NSUB = D / 64;
   constexpr int KSTEPS_QK = D / 16;
   constexpr uint32_t IDESC_QK = make_idesc_bf16(128, 128, 0, 0);
@@ -378,8 +382,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     for (int r = r0; r < r1; ++r) {
       const bool h0 = r < e.n0, h1 = r < e.n1, shared = round_shared(l0, l1, e, r);
       if (h0) {
-        const uint32_t st = ps.vc & 1;
-        if (!wait(&bars->v_full[st], (ps.vc >> 1) & 1)) return false;
+        const uint32_t st = ps.vc % kStages;
+        if (!wait(&bars->v_full[st], (ps.vc / kStages) & 1)) return false;
         // first PV of the item overwrites O_s: the previous item's epilogue must have read it
         if (r == 0 && !wait(&bars->o_empty[0], ps.n_o0 & 1)) return false;
         if (!wait(&bars->p_full[0], ps.n_p0 & 1)) return false;
@@ -395,8 +399,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       }
       if (h1) {
-        const uint32_t st = ps.vc & 1;
-        if (!shared && !wait(&bars->v_full[st], (ps.vc >> 1) & 1)) return false;
+        const uint32_t st = ps.vc % kStages;
+        if (!shared && !wait(&bars->v_full[st], (ps.vc / kStages) & 1)) return false;
         if (r == 0 && !wait(&bars->o_empty[1], ps.n_o1 & 1)) return false;
         if (!wait(&bars->p_full[1], ps.n_p1 & 1)) return false;
         ++ps.n_p1;
@@ -826,63 +830,67 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             tp = bilinear_taps(row / p.o_side, row % p.o_side, p.oi_side, p.oi_ratio);
             ibase = p.o_in + im.b * p.oi_sb + im.h * p.oi_sh;
           }
-          // Sixteen columns at a time in a loop that is not unrolled: this code runs once per item, from instruction
-          // lines that the tile loop has displaced, and fetching them is what its time went into.
+          // A loop that is not unrolled: this code runs once per item, from instruction lines that the tile loop has
+          // displaced, and fetching them is much of its time.
+          constexpr int EC = MODE == MODE_CSP || MODE == MODE_BLOCK ? 32 : 16;  // columns at a time
 #pragma unroll 1
-          for (int c = 0; c < D; c += 16) {
-            uint32_t r[16];
+          for (int c = 0; c < D; c += EC) {
+            uint32_t r[EC];
             if (it > 0) {
-              tmem_ld_x16(tO + c, r);
+              tmem_ld(tO + c, r);
               tmem_wait_ld();
             } else {
 #pragma unroll
-              for (int i = 0; i < 16; ++i) r[i] = 0u;
+              for (int i = 0; i < EC; ++i) r[i] = 0u;
             }
             if (split && other) {
-              uint32_t r1[16];
-              tmem_ld_x16(tO1 + c, r1);
+              uint32_t r1[EC];
+              tmem_ld(tO1 + c, r1);
               tmem_wait_ld();
 #pragma unroll
-              for (int i = 0; i < 16; ++i)
+              for (int i = 0; i < EC; ++i)
                 r[i] = __float_as_uint(fmaf(__uint_as_float(r1[i]), w1, __uint_as_float(r[i]) * w0));
             } else {
 #pragma unroll
-              for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * w0);
+              for (int i = 0; i < EC; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * w0);
             }
             if (row_ok) {
-              uint32_t w[8];
 #pragma unroll
-              for (int i = 0; i < 8; ++i) w[i] = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-              if (MODE == MODE_CSP) {
-                // out = bf16(o_in + o_scale * bf16(delta)): same rounding points as the reference's
-                // `o + o_delta * o_scale` on bf16 tensors (kernels/sparse_attn/sparse_attn_ops.py:288).
+              for (int h = 0; h < EC / 16; ++h) {
+                uint32_t w[8];
 #pragma unroll
-                for (int h8 = 0; h8 < 2; ++h8) {
-                  uint4 prev;
-                  if (resize) {
-                    const __nv_bfloat16* ib = ibase + c + h8 * 8;
-                    prev = bilinear_mix8(tp, *reinterpret_cast<const uint4*>(ib + (int64_t)tp.r00 * p.oi_sl),
-                                         *reinterpret_cast<const uint4*>(ib + (int64_t)tp.r01 * p.oi_sl),
-                                         *reinterpret_cast<const uint4*>(ib + (int64_t)tp.r10 * p.oi_sl),
-                                         *reinterpret_cast<const uint4*>(ib + (int64_t)tp.r11 * p.oi_sl));
-                  } else {
-                    prev = *reinterpret_cast<const uint4*>(irow + c + h8 * 8);
-                  }
-                  const uint32_t pv[4] = {prev.x, prev.y, prev.z, prev.w};
+                for (int i = 0; i < 8; ++i) w[i] = pack_bf16x2(__uint_as_float(r[16 * h + 2 * i]), __uint_as_float(r[16 * h + 2 * i + 1]));
+                if (MODE == MODE_CSP) {
+                  // out = bf16(o_in + o_scale * bf16(delta)): same rounding points as the reference's
+                  // `o + o_delta * o_scale` on bf16 tensors (kernels/sparse_attn/sparse_attn_ops.py:288).
 #pragma unroll
-                  for (int i = 0; i < 4; ++i) {
-                    const uint32_t d = w[h8 * 4 + i];
-                    const float d0 = __uint_as_float(d << 16), d1 = __uint_as_float(d & 0xffff0000u);
-                    const float a0 = __uint_as_float(pv[i] << 16), a1 = __uint_as_float(pv[i] & 0xffff0000u);
-                    w[h8 * 4 + i] = pack_bf16x2(fmaf(p.o_scale, d0, a0), fmaf(p.o_scale, d1, a1));
+                  for (int h8 = 0; h8 < 2; ++h8) {
+                    uint4 prev;
+                    if (resize) {
+                      const __nv_bfloat16* ib = ibase + c + h * 16 + h8 * 8;
+                      prev = bilinear_mix8(tp, *reinterpret_cast<const uint4*>(ib + (int64_t)tp.r00 * p.oi_sl),
+                                           *reinterpret_cast<const uint4*>(ib + (int64_t)tp.r01 * p.oi_sl),
+                                           *reinterpret_cast<const uint4*>(ib + (int64_t)tp.r10 * p.oi_sl),
+                                           *reinterpret_cast<const uint4*>(ib + (int64_t)tp.r11 * p.oi_sl));
+                    } else {
+                      prev = *reinterpret_cast<const uint4*>(irow + c + h * 16 + h8 * 8);
+                    }
+                    const uint32_t pv[4] = {prev.x, prev.y, prev.z, prev.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                      const uint32_t d = w[h8 * 4 + i];
+                      const float d0 = __uint_as_float(d << 16), d1 = __uint_as_float(d & 0xffff0000u);
+                      const float a0 = __uint_as_float(pv[i] << 16), a1 = __uint_as_float(pv[i] & 0xffff0000u);
+                      w[h8 * 4 + i] = pack_bf16x2(fmaf(p.o_scale, d0, a0), fmaf(p.o_scale, d1, a1));
+                    }
                   }
                 }
-              }
-              if (p.o_align32) {
-                st_global_v8(orow + c, w);
-              } else {
-                *reinterpret_cast<uint4*>(orow + c) = make_uint4(w[0], w[1], w[2], w[3]);
-                *reinterpret_cast<uint4*>(orow + c + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+                if (p.o_align32) {
+                  st_global_v8(orow + c + h * 16, w);
+                } else {
+                  *reinterpret_cast<uint4*>(orow + c + h * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+                  *reinterpret_cast<uint4*>(orow + c + h * 16 + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+                }
               }
             }
           }
@@ -1003,35 +1011,71 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           ++nq_items;
         }
         if (MODE != MODE_CSP) {
-          // MODE_DENSE_CS streams the K tiles a second time for the column-sum sweep
-          const int sweeps = (kHasCs && !stats_given) ? 2 : 1;
-          for (int rr = 0; rr < sweeps * rounds && ok; ++rr) {
-            const int r = rr < rounds ? rr : rr - rounds;
-            const Round rd = round_info(l0, l1, e, r);
-            for (int s = 0; s < 2; ++s) {
-              if (!rd.has[s] || (s == 1 && rd.shared)) continue;
+          if constexpr (MODE == MODE_BLOCK && D == 128) {
+            // The order in which two stages come free when the slots want different tiles: a slot's product of a round is
+            // over before the P V of its round before, so the next round's K goes ahead of this round's V (151 -> 148 us at
+            // 4096 x 10521 x 32 with 17 of 83 blocks, 17.8 -> 17.2 at 1024 x 2521 x 32).  Where the tiles are shared, K and
+            // V of a round one behind the other is the better order (attention with column sums, 1600 x 4121 x 32: 213
+            // against 218 us).
+            // one tile of round r for slot s, unless the slot has none there or shares slot 0's
+            auto load_k = [&](int r, int s) -> bool {
+              const Round rd = round_info(l0, l1, e, r);
+              if (!rd.has[s] || (s == 1 && rd.shared)) return true;
               const int st = kc % kStages;
-              ok = mbar_wait(&bars->k_empty[st], ((kc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER);
-              if (!ok) break;
+              if (!mbar_wait(&bars->k_empty[st], ((kc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER)) return false;
               mbar_arrive_expect_tx(&bars->k_full[st], SM::kTile);
               for (int sub = 0; sub < NSUB; ++sub)
-                tma_load_4d(sK + st * SM::kTile + sub * 16384, &tmK, &bars->k_full[st], sub * 64, rd.kvb[s] * 128, im.h,
-                            im.b);
+                tma_load_4d(sK + st * SM::kTile + sub * 16384, &tmK, &bars->k_full[st], sub * 64, rd.kvb[s] * 128, im.h, im.b);
               ++kc;
+              return true;
+            };
+            auto load_v = [&](int r, int s) -> bool {
+              const Round rd = round_info(l0, l1, e, r);
+              if (!rd.has[s] || (s == 1 && rd.shared)) return true;
+              const int st = vc % kStages;
+              if (!mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER)) return false;
+              mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile);
+              for (int sub = 0; sub < NSUB; ++sub)
+                tma_load_4d(sV + st * SM::kTile + sub * 16384, &tmV, &bars->v_full[st], sub * 64, rd.kvb[s] * 128, im.h, im.b);
+              ++vc;
+              return true;
+            };
+            ok = rounds == 0 || (load_k(0, 0) && load_k(0, 1));
+            for (int r = 0; r < rounds && ok; ++r) {
+              const bool more = r + 1 < rounds;
+              ok = (!more || load_k(r + 1, 0)) && load_v(r, 0) && (!more || load_k(r + 1, 1)) && load_v(r, 1);
             }
-            // V behind K in one thread: loads of V by a thread of its own measured slower (dense 4096 x 10521 x 32 537 us
-            // against 527, block-sparse 160 against 148)
-            if (MODE != MODE_CS_ONLY && rr < rounds) {
-              for (int s = 0; s < 2 && ok; ++s) {
+          } else {
+            // MODE_DENSE_CS streams the K tiles a second time for the column-sum sweep
+            const int sweeps = (kHasCs && !stats_given) ? 2 : 1;
+            for (int rr = 0; rr < sweeps * rounds && ok; ++rr) {
+              const int r = rr < rounds ? rr : rr - rounds;
+              const Round rd = round_info(l0, l1, e, r);
+              for (int s = 0; s < 2; ++s) {
                 if (!rd.has[s] || (s == 1 && rd.shared)) continue;
-                const int st = vc % kStages;
-                ok = mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER);
+                const int st = kc % kStages;
+                ok = mbar_wait(&bars->k_empty[st], ((kc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER);
                 if (!ok) break;
-                mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile);
+                mbar_arrive_expect_tx(&bars->k_full[st], SM::kTile);
                 for (int sub = 0; sub < NSUB; ++sub)
-                  tma_load_4d(sV + st * SM::kTile + sub * 16384, &tmV, &bars->v_full[st], sub * 64, rd.kvb[s] * 128, im.h,
+                  tma_load_4d(sK + st * SM::kTile + sub * 16384, &tmK, &bars->k_full[st], sub * 64, rd.kvb[s] * 128, im.h,
                               im.b);
-                ++vc;
+                ++kc;
+              }
+              // V of the round behind its K in the same thread: a thread of its own for V measured slower (dense 4096 x 10521 x
+              // 32 537 us against 527, block-sparse 160 against 148)
+              if (MODE != MODE_CS_ONLY && rr < rounds) {
+                for (int s = 0; s < 2 && ok; ++s) {
+                  if (!rd.has[s] || (s == 1 && rd.shared)) continue;
+                  const int st = vc % kStages;
+                  ok = mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER);
+                  if (!ok) break;
+                  mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile);
+                  for (int sub = 0; sub < NSUB; ++sub)
+                    tma_load_4d(sV + st * SM::kTile + sub * 16384, &tmV, &bars->v_full[st], sub * 64, rd.kvb[s] * 128, im.h,
+                                im.b);
+                  ++vc;
+                }
               }
             }
           }
@@ -1179,7 +1223,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         // S_s = Q_s K^T of one tile, once the buffer it lands in has been read
         auto product = [&](auto s_tag, int st, bool wait_k) -> bool {
           constexpr int s = decltype(s_tag)::value;
-          if (wait_k && !mbar_wait(&bars->k_full[st], (kc >> 1) & 1, wc, DEV_TIMEOUT_MMA)) return false;
+          if (wait_k && !mbar_wait(&bars->k_full[st], (kc / kStages) & 1, wc, DEV_TIMEOUT_MMA)) return false;
           // the scores of the product before (the other slot's, as a rule) have left the score buffer
           if (!mbar_wait(&bars->s_read, n_sr & 1, wc, DEV_TIMEOUT_MMA)) return false;
           ++n_sr;
@@ -1199,7 +1243,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int r = 0; r < rounds_first && ok; ++r) {
           const bool h0 = r < e.n0, h1 = r < e.n1, shared = round_shared(l0, l1, e, r);
           if (h0) {
-            const int st = kc & 1;
+            const int st = kc % kStages;
             ok = product(std::integral_constant<int, 0>{}, st, true);
             if (!ok) break;
             if (!shared) {
@@ -1208,7 +1252,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             }
           }
           if (h1) {
-            const int st = kc & 1;
+            const int st = kc % kStages;
             ok = product(std::integral_constant<int, 1>{}, st, !shared);
             if (!ok) break;
             umma_commit(&bars->k_empty[st]);
@@ -1227,7 +1271,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           // ---- column-sum sweep: S_s^T = K Q_s^T per KV tile (the operands swap roles, the tiles stay where they are)
           auto sweep_product = [&](auto s_tag, int st, bool wait_k) -> bool {
             constexpr int s = decltype(s_tag)::value, b = s;
-            if (wait_k && !mbar_wait(&bars->k_full[st], (kc >> 1) & 1, wc, DEV_TIMEOUT_MMA)) return false;
+            if (wait_k && !mbar_wait(&bars->k_full[st], (kc / kStages) & 1, wc, DEV_TIMEOUT_MMA)) return false;
             if (!mbar_wait(&bars->cs_empty[b], n_cst[b] & 1, wc, DEV_TIMEOUT_MMA)) return false;
             ++n_cst[b];
             tc_fence_after();
@@ -1244,7 +1288,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           for (int r = 0; r < rounds && ok; ++r) {
             const bool h0 = r < e.n0, h1 = r < e.n1, shared = round_shared(l0, l1, e, r);
             if (h0) {
-              const int st = kc & 1;
+              const int st = kc % kStages;
               ok = sweep_product(std::integral_constant<int, 0>{}, st, true);
               if (!ok) break;
               if (!shared) {
@@ -1253,7 +1297,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               }
             }
             if (h1) {
-              const int st = kc & 1;
+              const int st = kc % kStages;
               ok = sweep_product(std::integral_constant<int, 1>{}, st, !shared);
               if (!ok) break;
               umma_commit_if(leader, &bars->k_empty[st]);
