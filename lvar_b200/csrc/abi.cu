@@ -62,6 +62,20 @@ int encode_bhld_map(CUtensorMap* out, const void* base, int B, int H, int L, int
   return LVAR_OK;
 }
 
+int encode_rows_map(CUtensorMap* out, const void* base, int64_t rows, int64_t width, int64_t pitch) {
+  EncodeTiledFn fn = get_encode_fn();
+  LVAR_REQUIRE(fn != nullptr, LVAR_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available (no CUDA driver?)");
+  cuuint64_t dims[2] = {(cuuint64_t)width, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)pitch * 2};
+  cuuint32_t box[2] = {64u, 1u};
+  cuuint32_t estr[2] = {1u, 1u};
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  LVAR_REQUIRE(r == CUDA_SUCCESS, LVAR_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+  return LVAR_OK;
+}
+
 int launch_attention(const lvar_attn_args* a, int mode, cudaStream_t stream);
 int launch_colsum(const void* q, const void* k, const float* M, const float* L, float* cs, int B, int H, int Lq,
                   int Lkv, int D, int64_t q_sb, int64_t q_sh, int64_t q_sl, int64_t k_sb, int64_t k_sh, int64_t k_sl,

@@ -6,11 +6,11 @@
 
 namespace lvar {
 
-// Column-sparse attention gathers the 128 rows of KV tile `j` of an index list into a swizzled [128][D]
-// tile with 16-byte cp.async copies, one warp per tile.  The tile's 128 indices are read first, coalesced
-// (lane l holds those of rows l, l+32, l+64, l+96; gather_rows_of_tile, which the loaders call one tile ahead
-// so that the index latency is off the critical path).  gather_tile then copies 8 rows per instruction:
-// four lanes share a row (its index comes by shuffle, one row pointer per pass) and copy adjacent chunks
+// Column-sparse attention gathers the 128 rows of KV tile `j` of an index list into a swizzled [128][D] tile, two warps
+// per tile.  Where the tensor allows it (launch_attention) by TMA, four rows a request; otherwise with 16-byte cp.async
+// copies.  For the copies lane l holds the indices of rows l, l+32, l+64, l+96 (gather_rows_of_tile, which the loaders
+// call one tile ahead so that the index latency is off the critical path).  gather_half_tile then copies 8 rows per
+// instruction: four lanes share a row (its index comes by shuffle, one row pointer per pass) and copy adjacent chunks
 // of it, which keeps both the number of cache lines per instruction (8) and the address arithmetic per
 // copy low.  List positions past `cnt` read row 0 (their P columns are zero).
 __device__ __forceinline__ void gather_rows_of_tile(int (&kv)[4], const int32_t* idx, int cnt, int j, int Lkv,
@@ -35,18 +35,54 @@ __device__ __forceinline__ bool tile_is_run(const int (&kv)[4], int cnt, int j, 
   for (int i = 0; i < 4; ++i) run = run && kv[i] == first + i * 32 + lane;
   return __all_sync(0xffffffffu, run);
 }
+// The same for the TMA gather, where lane l holds the keys of rows 4 l .. 4 l + 3: the list entries of a tile, read ahead of
+// the copies of the tile before, and their check, which waits for them.
+__device__ __forceinline__ void gather4_read(int (&kv)[4], const int32_t* idx, int cnt, int j, int lane) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int pos = j * 128 + 4 * lane + i;
+    // volatile: the load stays ahead of the copies that are issued between it and the check
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.lt.s32 p, %2, %3;\n"
+        "mov.b32 %0, 0;\n"
+        "@p ld.global.nc.b32 %0, [%1];\n"
+        "}\n"
+        : "=r"(kv[i])
+        : "l"(idx + pos), "r"(pos), "r"(cnt));
+  }
+}
+__device__ __forceinline__ void gather4_check(int (&kv)[4], int Lkv, int* status) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if ((unsigned)kv[i] >= (unsigned)Lkv) {
+      if (status) atomicCAS(status, 0, (int)DEV_BAD_INDEX);
+      kv[i] = 0;
+    }
+  }
+}
+__device__ __forceinline__ bool tile4_is_run(const int (&kv)[4], int cnt, int j, int Lkv, int lane) {
+  const int first = __shfl_sync(0xffffffffu, kv[0], 0);
+  bool run = (j + 1) * 128 <= cnt && first + 128 <= Lkv;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) run = run && kv[i] == first + 4 * lane + i;
+  return __all_sync(0xffffffffu, run);
+}
 template <int D>
-__device__ __forceinline__ void gather_tile(uint32_t dst, const __nv_bfloat16* base, int64_t row_stride,
-                                            const int (&kv)[4], int lane) {
+__device__ __forceinline__ void gather_half_tile(uint32_t dst, const __nv_bfloat16* base, int64_t row_stride,
+                                                 const int (&kv)[4], int lane, int half) {
   constexpr int CH = D / 8;      // 16-byte chunks per row
   constexpr int RPI = 8;         // rows per instruction (measured: 8 beats 2, 4, 16 and 32)
   constexpr int LPR = 32 / RPI;  // lanes that share a row
   constexpr int CPL = CH / LPR;  // chunks per lane and row
   const int g = lane / LPR, cq = lane % LPR;
+  const int kh[2] = {half ? kv[2] : kv[0], half ? kv[3] : kv[1]};
+  dst += (uint32_t)half * 8192u;
 #pragma unroll
-  for (int pass = 0; pass < 128 / RPI; ++pass) {
+  for (int pass = 0; pass < 64 / RPI; ++pass) {
     const int r = pass * RPI + g;
-    const int row = __shfl_sync(0xffffffffu, kv[(pass * RPI) >> 5], r & 31);
+    const int row = __shfl_sync(0xffffffffu, kh[(pass * RPI) >> 5], r & 31);
     const __nv_bfloat16* src = base + (int64_t)row * row_stride;
     const uint32_t drow = dst + (uint32_t)r * 128u;
     const uint32_t x = (uint32_t)(r & 7);

@@ -7,12 +7,12 @@
 // same round is loaded once (always the case for dense and column-sparse attention).
 //   warps 0-3   softmax warpgroup of slot 0 (thread = one query row = one TMEM lane)
 //   warps 4-7   softmax warpgroup of slot 1
-//   warp  8     loader of Q, K and V by TMA; column-sparse: of Q by TMA and of K by 16-byte cp.async row gathers (four
-//               lanes share a row; the tile's barrier takes one arrival per lane as its copies land)
-//   warp  9     one lane issues the P V products; column-sparse: V gather
+//   warp  8     loader of Q, K and V by TMA
+//   warp  9     one lane issues the P V products
 //   warp  10    allocates TMEM; one lane issues the Q K^T products
-//   warp  11    scheduler: takes work items from the global counter and builds their KV-tile lists; column-sparse: also
-//               issues the P V products
+//   warp  11    scheduler: takes work items from the global counter and builds their KV-tile lists
+// Column-sparse attention has four more warps: 8 (Q too) and 9 gather K rows, 12 and 13 V rows, 14 issues the P V products,
+// 15 has no role.
 // TMEM (512 columns x 128 lanes, fp32): P0 [0, 64) | S [64, 192) | P1 [192, 256) | O0 | O1.  The two slots take turns with
 // ONE score buffer: S = Q_s K^T is read into registers as soon as it lands, which frees the buffer for the other slot's
 // product, while the slot's own P has columns of its own.  A slot's next scores are then ready when its softmax warps
@@ -46,8 +46,12 @@ namespace lvar {
 
 namespace {
 
-constexpr int kThreads = 384;  // 8 softmax warps, loader, P V issuer, Q K^T issuer, scheduler
-constexpr int kRegsSoftmax = 208, kRegsOther = 72;
+// Threads of a block and registers a thread of the softmax and the other warps; their sum is what the block is launched
+// with, 384 x 168 or 512 x 128.  Column-sparse attention gives registers of its softmax warps away for four more warps
+// (see the row gather).
+__host__ __device__ constexpr int threads_of(int mode) { return mode == 2 ? 512 : 384; }
+__host__ __device__ constexpr int regs_softmax_of(int mode) { return mode == 2 ? 192 : 208; }
+__host__ __device__ constexpr int regs_other_of(int mode) { return mode == 2 ? 64 : 72; }
 constexpr int kMaxSteps = 1024;  // per-slot KV tile list capacity (block-sparse: Lkv <= 131072)
 constexpr int kMaxStages = 4;  // of K and of V each
 constexpr int kSchedStages = 2;
@@ -103,6 +107,9 @@ struct AttnParams {
   const __nv_bfloat16* k;  // raw pointers for the gather
   const __nv_bfloat16* v;
   int64_t k_sb, k_sh, k_sl, v_sb, v_sh, v_sl;
+  // TMA row gather: K and V as 2-D tensors of rows; row b * rb + h * rh + key, columns from h * ch on (see launch_attention)
+  int gather4;  // 0: cp.async copies from the raw pointers
+  int kg_rb, kg_rh, kg_ch, vg_rb, vg_rh, vg_ch;
   const __nv_bfloat16* o_in;  // accumulate input (may alias o)
   int64_t oi_sb, oi_sh, oi_sl;
   float o_scale;
@@ -119,6 +126,14 @@ struct AttnParams {
   // plumbing
   int* status;
   unsigned long long wait_limit_ns;
+};
+
+// Tensor maps of the row gather (column-sparse attention only).
+template <int MODE>
+struct GatherMaps {};
+template <>
+struct GatherMaps<MODE_CSP> {
+  CUtensorMap k, v;
 };
 
 template <int D>
@@ -190,10 +205,11 @@ static_assert(sizeof(Bars) <= 512, "barrier block too large");
 // code.  What the schedule alone decides (decode, the loaders) is the same code either way: fewer run-time choices there
 // measured 2 % slower.  The other modes measured the same with and without.
 template <int D, int MODE, bool SPLIT>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(threads_of(MODE), 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                const __grid_constant__ CUtensorMap tmV, const AttnParams p) {
+                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ GatherMaps<MODE> gm, const AttnParams p) {
   using SM = Smem<D>;
+  constexpr int kRegsSoftmax = regs_softmax_of(MODE), kRegsOther = regs_other_of(MODE);
   constexpr int kStages = SM::kStages;
   constexpr int NSUB = D / 64;
   constexpr int KSTEPS_QK = D / 16;
@@ -201,7 +217,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   constexpr uint32_t IDESC_PV = make_idesc_bf16(128, D, 0, 1);
   constexpr uint32_t TM_S = 64, TM_P1 = 192, TM_O = 256;
   constexpr bool kHasCs = MODE == MODE_DENSE_CS || MODE == MODE_CS_ONLY;  // column-sum sweep after the first one
-  // Columns that are not attended become -inf in TMEM before the scores are read, in a loop of a few instructions, or in
+  // Columns past the end of K become -inf in TMEM before the scores are read, in a loop of a few instructions, or in
   // registers.  The loop suits the modes that meet such tiles often and whose items are short (column-sparse 65 -> 57 us
   // at 1600 x 4121 x 32); in the dense modes its test ahead of the read lengthens the way from one slot's scores to the
   // other's next product (dense 4096 x 10521 x 32: 520 -> 580 us).
@@ -223,40 +239,54 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int lane = tid & 31;
 
   // ---------------------------------------------------------------- setup
-  if (tid == 0) {
-    mbar_init(&bars->q_full, 1);
-    mbar_init(&bars->q_empty, 1);
-    for (int i = 0; i < kStages; ++i) {
-      mbar_init(&bars->k_full[i], MODE == MODE_CSP ? 32 : 1);
-      mbar_init(&bars->k_empty[i], 1);
-      mbar_init(&bars->v_full[i], MODE == MODE_CSP ? 32 : 1);
-      mbar_init(&bars->v_empty[i], 1);
-    }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&bars->s_full[s], 1);
-      mbar_init(&bars->p_full[s], 128);
-      mbar_init(&bars->pv_done[s], 1);
-      mbar_init(&bars->o_empty[s], 128);
+  auto init_stage = [&](int i) {
+    // column-sparse: as many arrivals as warps, or lanes, fetch
+    const uint32_t fetchers = MODE != MODE_CSP ? 1 : p.gather4 ? 2 : 64;
+    mbar_init(&bars->k_full[i], fetchers);
+    mbar_init(&bars->k_empty[i], 1);
+    mbar_init(&bars->v_full[i], fetchers);
+    mbar_init(&bars->v_empty[i], 1);
+  };
+  auto init_slot = [&](int s) {
+    mbar_init(&bars->s_full[s], 1);
+    mbar_init(&bars->p_full[s], 128);
+    mbar_init(&bars->pv_done[s], 1);
+    mbar_init(&bars->o_empty[s], 128);
+    mbar_init(&bars->xchg_full[s], 128);
+    if (kHasCs) {
       mbar_init(&bars->cs_full[s], 1);
       mbar_init(&bars->cs_empty[s], 128);
     }
-    for (int i = 0; i < kSchedStages; ++i) {
-      mbar_init(&bars->sched_full[i], 1);
-      mbar_init(&bars->sched_empty[i], 12);  // every warp
-    }
-    mbar_init(&bars->s_read, 128);
-    mbar_init(&bars->mma_done[0], 1);
-    mbar_init(&bars->mma_done[1], 1);
-    mbar_init(&bars->pv_all, 1);
-    mbar_init(&bars->xchg_full[0], 128);
-    mbar_init(&bars->xchg_full[1], 128);
-    if (kHasCs) mbar_init(&bars->xchg_back, 128);
-    for (int s = 0; s < 2; ++s) {
+    if (MODE == MODE_DENSE_CS1) {
       mbar_init(&bars->part_full[s][0], 128);
       mbar_init(&bars->part_full[s][1], 128);
       mbar_init(&bars->rowl_full[s], 128);
     }
+    mbar_init(&bars->mma_done[s], 1);
+  };
+  auto init_rest = [&]() {
+    for (int i = 0; i < kSchedStages; ++i) {
+      mbar_init(&bars->sched_full[i], 1);
+      mbar_init(&bars->sched_empty[i], MODE == MODE_CSP ? 15 : 12);  // every warp that has a role
+    }
+    mbar_init(&bars->q_full, 1);
+    mbar_init(&bars->q_empty, 1);
+    mbar_init(&bars->s_read, 128);
+    mbar_init(&bars->pv_all, 1);
+    if (kHasCs) mbar_init(&bars->xchg_back, 128);
     bars->abort_flag = 0;
+  };
+  if constexpr (MODE == MODE_BLOCK || MODE == MODE_CSP) {
+    // three warps share the work.  Only in the sparse modes, by measurement of whole launches (block-sparse 4096 x 10521 x
+    // 32 with 17 of 83 blocks 146 -> 139 us; dense 64 x 121 x 32 8.15 -> 8.35).
+    if (tid < kStages) init_stage(tid);
+    else if (warp == 1 && lane < 2) init_slot(lane);
+    else if (warp == 2 && lane == 0) init_rest();
+    if (warp < 3) mbar_fence_init();
+  } else if (tid == 0) {
+    for (int i = 0; i < kStages; ++i) init_stage(i);
+    for (int s = 0; s < 2; ++s) init_slot(s);
+    init_rest();
     mbar_fence_init();
   }
   if (warp == 10) {
@@ -613,10 +643,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tc_fence_after();
 
         const int valid = (MODE == MODE_CSP) ? (cnt_total - j * 128) : (p.Lkv - kvb * 128);
-        if (kMaskInTmem && __builtin_expect(valid < 128 || sub != 3u, 0)) {
-          // columns past the end of K, and (64-wide masks) the column half this row's half does not attend
-          if (!(sub & 1u)) mask_columns(tS, 0, 64);
-          mask_columns(tS, (sub & 2u) ? valid : min(valid, 64), 128);
+        if (kMaskInTmem && __builtin_expect(valid < 128, 0)) {  // columns past the end of K
+          mask_columns(tS, valid, 128);
           tmem_wait_st();
         }
         // raw fp32 bits of the S row, four 32-column chunks kept in registers
@@ -631,6 +659,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         mbar_arrive(&bars->s_read);
         bool pv_waited = MODE == MODE_CS_ONLY || j == 0;  // the product that reads this slot's last P has completed
 
+        if (MODE == MODE_BLOCK && sub != 3u) {
+          // 64-wide masks: the column half that this row's half does not attend
+          if (!(sub & 1u)) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) s0[i] = s1[i] = 0xff800000u;  // -inf
+          }
+          if (!(sub & 2u)) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) s2[i] = s3[i] = 0xff800000u;
+          }
+        }
         if (!kMaskInTmem && __builtin_expect(valid < 128, 0)) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
@@ -979,7 +1018,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
     }
-  } else if (warp == 8) {
+  } else if (warp == 8 || (MODE == MODE_CSP && warp == 9)) {
     // ============================================================ Q, K and V loader; column-sparse: Q loader, K gather
     setmaxnreg_dec<kRegsOther>();
     bool ok = true;
@@ -997,7 +1036,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const uint16_t* l1 = l0 + kMaxSteps;
         const int rounds = max(e.n0, e.n1);
         if (rounds > 0) {
-          if (lane == 0) {
+          if (lane == 0 && warp == 8) {
             ok = mbar_wait(&bars->q_empty, (nq_items & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER);
             if (ok) {
               mbar_arrive_expect_tx(&bars->q_full, 2 * SM::kTile);
@@ -1010,7 +1049,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if (!ok) break;
           ++nq_items;
         }
-        if (MODE != MODE_CSP) {
+        if constexpr (MODE != MODE_CSP) {
           if constexpr (MODE == MODE_BLOCK && D == 128) {
             // The order in which two stages come free when the slots want different tiles: a slot's product of a round is
             // over before the P V of its round before, so the next round's K goes ahead of this round's V (151 -> 148 us at
@@ -1081,29 +1120,70 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           }
         } else {
           const int32_t* idx = p.indices + im.b * p.i_sb + im.h * p.i_sh + (int64_t)im.group * p.i_sg;
-          const __nv_bfloat16* kbase = p.k + im.b * p.k_sb + im.h * p.k_sh;
-          int kv[4];
-          if (rounds > 0) gather_rows_of_tile(kv, idx, e.aux, 0, p.Lkv, lane, p.status);
-          for (int j = 0; j < rounds; ++j) {
-            const int st = kc % kStages;
-            ok = __all_sync(0xffffffffu, mbar_wait(&bars->k_empty[st], ((kc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
-            if (!ok) break;
-            if (tile_is_run(kv, e.aux, j, p.Lkv, lane)) {
-              // 128 consecutive keys (the local band of a list): one tile copy instead of 2048 row pieces
+          if (p.gather4) {
+            // One lane requests four rows of 64 columns; a request takes its warp about 80 cycles, and what bounds the gather is
+            // their issue (2600 cycles for half a tile beside 2048 of tensor work on both slots).  So a tile's requests are
+            // split between two warps: by 64-column halves, or with head dimension 64 by 64-row halves.  The copies pass
+            // the load/store unit by, where the 2048 sixteen-byte copies of a tile held up every barrier of the block:
+            // 1408 of 10521 keys, 4096 queries, 32 heads 169 -> 128 us; copies by two warps per operand 160.  A fifth warp
+            // with a share of both operands' requests was slower (134).
+            const int row0 = im.b * p.kg_rb + im.h * p.kg_rh, col0 = im.h * p.kg_ch;
+            const int sub = D == 128 ? (warp & 1) : 0;
+            const bool mine = D == 128 || (lane >> 4) == (warp & 1);
+            int kv[4], nx[4];
+            if (rounds > 0) gather4_read(nx, idx, e.aux, 0, lane);
+            for (int j = 0; j < rounds; ++j) {
+              gather4_check(nx, p.Lkv, p.status);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) kv[i] = nx[i];
+              if (j + 1 < rounds) gather4_read(nx, idx, e.aux, j + 1, lane);
+              const int st = kc % kStages;
+              ok = __all_sync(0xffffffffu, mbar_wait(&bars->k_empty[st], ((kc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
+              if (!ok) break;
+              uint8_t* tile = sK + st * SM::kTile;
+              // every warp that fetches arrives for every tile, so that none falls two phases behind on tiles it is not needed for
               if (lane == 0) {
-                mbar_arrive_expect_tx(&bars->k_full[st], SM::kTile);
-                for (int sub = 0; sub < NSUB; ++sub)
-                  tma_load_4d(sK + st * SM::kTile + sub * 16384, &tmK, &bars->k_full[st], sub * 64, kv[0], im.h, im.b);
-              } else {
-                mbar_arrive(&bars->k_full[st]);
+                if (warp == 8) mbar_arrive_expect_tx(&bars->k_full[st], SM::kTile);
+                else mbar_arrive(&bars->k_full[st]);
               }
-            } else {
-              gather_tile<D>(smem_u32(sK + st * SM::kTile), kbase, p.k_sl, kv, lane);
-              // each lane's arrival follows its own copies; nobody waits here (the MMA warp fences the proxies)
-              cp_async_mbar_arrive(&bars->k_full[st]);
+              if (tile4_is_run(kv, e.aux, j, p.Lkv, lane)) {
+                // 128 consecutive keys (the local band of a list): one tile copy
+                if (lane == 0 && warp == 8) {
+                  for (int s2 = 0; s2 < NSUB; ++s2)
+                    tma_load_4d(tile + s2 * 16384, &tmK, &bars->k_full[st], s2 * 64, kv[0], im.h, im.b);
+                }
+              } else if (mine) {
+                tma_gather4(tile + sub * 16384 + lane * 512, &gm.k, &bars->k_full[st], col0 + sub * 64, row0 + kv[0], row0 + kv[1],
+                            row0 + kv[2], row0 + kv[3]);
+              }
+              __syncwarp();
+              ++kc;
             }
-            if (j + 1 < rounds) gather_rows_of_tile(kv, idx, e.aux, j + 1, p.Lkv, lane, p.status);
-            ++kc;
+          } else {
+            const __nv_bfloat16* kbase = p.k + im.b * p.k_sb + im.h * p.k_sh;
+            int kv[4];
+            if (rounds > 0) gather_rows_of_tile(kv, idx, e.aux, 0, p.Lkv, lane, p.status);
+            for (int j = 0; j < rounds; ++j) {
+              const int st = kc % kStages;
+              ok = __all_sync(0xffffffffu, mbar_wait(&bars->k_empty[st], ((kc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
+              if (!ok) break;
+              if (tile_is_run(kv, e.aux, j, p.Lkv, lane)) {
+                // 128 consecutive keys (the local band of a list): one tile copy instead of 2048 row pieces
+                if (lane == 0 && warp == 8) {
+                  mbar_arrive_expect_tx(&bars->k_full[st], SM::kTile);
+                  for (int sub = 0; sub < NSUB; ++sub)
+                    tma_load_4d(sK + st * SM::kTile + sub * 16384, &tmK, &bars->k_full[st], sub * 64, kv[0], im.h, im.b);
+                } else {
+                  mbar_arrive(&bars->k_full[st]);
+                }
+              } else {
+                gather_half_tile<D>(smem_u32(sK + st * SM::kTile), kbase, p.k_sl, kv, lane, warp & 1);
+                // each lane's arrival follows its own copies; nobody waits here (the MMA warp fences the proxies)
+                cp_async_mbar_arrive(&bars->k_full[st]);
+              }
+              if (j + 1 < rounds) gather_rows_of_tile(kv, idx, e.aux, j + 1, p.Lkv, lane, p.status);
+              ++kc;
+            }
           }
         }
         if (!ok) break;
@@ -1113,10 +1193,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       // Drain on abort: copies in flight must land before the CTA's shared memory is released.
       if (lane == 0 && bars->abort_flag) {
         const uint64_t t0 = globaltimer_ns();
-        if (nq_items > 0)
+        if (nq_items > 0 && warp == 8)
           while (!mbar_try_wait(&bars->q_full, (nq_items - 1) & 1) && globaltimer_ns() - t0 < 2000000000ull) {
           }
-        if (MODE != MODE_CSP) {
+        if (MODE != MODE_CSP || p.gather4) {
           for (int c = max(0, kc - kStages); c < kc; ++c) {
             const uint64_t t1 = globaltimer_ns();
             while (!mbar_try_wait(&bars->k_full[c % kStages], (c / kStages) & 1) &&
@@ -1133,11 +1213,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
     __syncwarp();
-  } else if (warp == 9) {
-    // ============================================================ P V issuer; column-sparse: V gather
+  } else if (MODE == MODE_CSP ? warp >= 12 : warp == 9) {
+    // ============================================================ P V issuer; column-sparse: V gather (12, 13), P V issuer (14)
     setmaxnreg_dec<kRegsOther>();
     bool ok = true;
-    if (MODE == MODE_CSP) {
+    if (MODE == MODE_CSP && warp < 14) {
+      if constexpr (MODE == MODE_CSP) {
       int vc = 0;
       for (int n = 0; ok; ++n) {
         SchedEntry e;
@@ -1146,33 +1227,76 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const Item im = decode(e.item, e.half);
         const int rounds = max(e.n0, e.n1);
         const int32_t* idx = p.indices + im.b * p.i_sb + im.h * p.i_sh + (int64_t)im.group * p.i_sg;
-        const __nv_bfloat16* vbase = p.v + im.b * p.v_sb + im.h * p.v_sh;
-        int kv[4];
-        if (rounds > 0) gather_rows_of_tile(kv, idx, e.aux, 0, p.Lkv, lane, nullptr);
-        for (int j = 0; j < rounds; ++j) {
-          const int st = vc % kStages;
-          ok = __all_sync(0xffffffffu, mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
-          if (!ok) break;
-          if (tile_is_run(kv, e.aux, j, p.Lkv, lane)) {
+        if (p.gather4) {
+          const int row0 = im.b * p.vg_rb + im.h * p.vg_rh, col0 = im.h * p.vg_ch;
+          const int sub = D == 128 ? (warp & 1) : 0;
+          const bool mine = D == 128 || (lane >> 4) == (warp & 1);
+          int kv[4], nx[4];
+          if (rounds > 0) gather4_read(nx, idx, e.aux, 0, lane);
+          for (int j = 0; j < rounds; ++j) {
+            gather4_check(nx, p.Lkv, nullptr);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) kv[i] = nx[i];
+            if (j + 1 < rounds) gather4_read(nx, idx, e.aux, j + 1, lane);
+            const int st = vc % kStages;
+            ok = __all_sync(0xffffffffu, mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
+            if (!ok) break;
+            uint8_t* tile = sV + st * SM::kTile;
             if (lane == 0) {
-              mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile);
-              for (int sub = 0; sub < NSUB; ++sub)
-                tma_load_4d(sV + st * SM::kTile + sub * 16384, &tmV, &bars->v_full[st], sub * 64, kv[0], im.h, im.b);
-            } else {
-              mbar_arrive(&bars->v_full[st]);
+              if (warp == 12) mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile);
+              else mbar_arrive(&bars->v_full[st]);
             }
-          } else {
-            gather_tile<D>(smem_u32(sV + st * SM::kTile), vbase, p.v_sl, kv, lane);
-            cp_async_mbar_arrive(&bars->v_full[st]);
+            if (tile4_is_run(kv, e.aux, j, p.Lkv, lane)) {
+              // 128 consecutive keys (the local band of a list): one tile copy
+              if (lane == 0 && warp == 12) {
+                for (int s2 = 0; s2 < NSUB; ++s2)
+                  tma_load_4d(tile + s2 * 16384, &tmV, &bars->v_full[st], s2 * 64, kv[0], im.h, im.b);
+              }
+            } else if (mine) {
+              tma_gather4(tile + sub * 16384 + lane * 512, &gm.v, &bars->v_full[st], col0 + sub * 64, row0 + kv[0], row0 + kv[1],
+                          row0 + kv[2], row0 + kv[3]);
+            }
+            __syncwarp();
+            ++vc;
           }
-          if (j + 1 < rounds) gather_rows_of_tile(kv, idx, e.aux, j + 1, p.Lkv, lane, nullptr);
-          ++vc;
+        } else {
+          const __nv_bfloat16* vbase = p.v + im.b * p.v_sb + im.h * p.v_sh;
+          int kv[4];
+          if (rounds > 0) gather_rows_of_tile(kv, idx, e.aux, 0, p.Lkv, lane, nullptr);
+          for (int j = 0; j < rounds; ++j) {
+            const int st = vc % kStages;
+            ok = __all_sync(0xffffffffu, mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
+            if (!ok) break;
+            if (tile_is_run(kv, e.aux, j, p.Lkv, lane)) {
+              if (lane == 0 && warp == 12) {
+                mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile);
+                for (int sub = 0; sub < NSUB; ++sub)
+                  tma_load_4d(sV + st * SM::kTile + sub * 16384, &tmV, &bars->v_full[st], sub * 64, kv[0], im.h, im.b);
+              } else {
+                mbar_arrive(&bars->v_full[st]);
+              }
+            } else {
+              gather_half_tile<D>(smem_u32(sV + st * SM::kTile), vbase, p.v_sl, kv, lane, warp & 1);
+              cp_async_mbar_arrive(&bars->v_full[st]);
+            }
+            if (j + 1 < rounds) gather_rows_of_tile(kv, idx, e.aux, j + 1, p.Lkv, lane, nullptr);
+            ++vc;
+          }
         }
         if (!ok) break;
         if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
       }
       cp_async_wait<0>();
-    } else if (elect_one()) {
+      if (lane == 0 && p.gather4 && bars->abort_flag) {
+        for (int c = max(0, vc - kStages); c < vc; ++c) {
+          const uint64_t t1 = globaltimer_ns();
+          while (!mbar_try_wait(&bars->v_full[c % kStages], (c / kStages) & 1) &&
+                 globaltimer_ns() - t1 < 2000000000ull) {
+          }
+        }
+      }
+      }
+    } else if (warp != 15 && elect_one()) {
       // One lane runs the whole role: the issue of sixteen MMAs took it 640 cycles against 880 for a warp that runs
       // the bookkeeping on all lanes and predicates the issue (1024 is what they execute in).
       PvState ps;
@@ -1431,35 +1555,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       __syncwarp();
       return true;
     };
-    if (MODE == MODE_CSP) {
-      // column-sparse: this warp issues the P V products as well (warps 8 and 9 gather rows); the next item is taken
-      // after the second round of the present one
-      PvState ps;
-      bool ok = publish(0);
-      for (int n = 0; ok; ++n) {
-        const SchedEntry e = bars->sched[n % kSchedStages];
-        if (e.item < 0) break;
-        const int rounds = max(e.n0, e.n1);
-        if (lane == 0) ok = pv_rounds(ps, e, n, 0, min(2, rounds));
-        ok = __all_sync(0xffffffffu, ok) && publish(n + 1);
-        if (ok && lane == 0) {
-          ok = pv_rounds(ps, e, n, 2, rounds);
-          if (ok) pv_end(ps, e);
-        }
-        ok = __all_sync(0xffffffffu, ok);
-        if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
-      }
-      if (lane == 0) drain_mma(&bars->mma_done[1]);
-      __syncwarp();
-    } else {
-      bool ok = publish(0);
-      for (int n = 0; ok; ++n) {
-        if (bars->sched[n % kSchedStages].item < 0) break;
-        ok = publish(n + 1);
-        if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
-      }
-      __syncwarp();
+    bool ok = publish(0);
+    for (int n = 0; ok; ++n) {
+      if (bars->sched[n % kSchedStages].item < 0) break;
+      ok = publish(n + 1);
+      if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
     }
+    __syncwarp();
     if (lane == 0) {
       __threadfence();
       if (atomicAdd(p.sched_counter + 1, 1) == (int)gridDim.x - 1) {
@@ -1487,7 +1589,7 @@ namespace {
 
 template <int D, int MODE, bool SPLIT>
 int launch_mode(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p, dim3 grid,
-                cudaStream_t stream, bool serialize_launch) {
+                cudaStream_t stream, bool serialize_launch, const GatherMaps<MODE>& gm = {}) {
   auto kern = attn_fwd_kernel<D, MODE, SPLIT>;
   static bool attr_set[16] = {false};
   int dev = 0;
@@ -1500,7 +1602,7 @@ int launch_mode(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(threads_of(MODE));
   cfg.dynamicSmemBytes = Smem<D>::kDynamic;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -1508,14 +1610,14 @@ int launch_mode(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = serialize_launch ? 0 : 1;
-  LVAR_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, p));
+  LVAR_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, gm, p));
   LVAR_CUDA_OK(cudaGetLastError());
   return LVAR_OK;
 }
 
 template <int D>
 int launch_d(int mode, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p,
-             dim3 grid, cudaStream_t stream, bool serialize_launch) {
+             dim3 grid, cudaStream_t stream, bool serialize_launch, const GatherMaps<MODE_CSP>& gm) {
   const bool splits = p.split_singles != 0 && p.n_pair_items < p.total_items;
   switch (mode) {
     case MODE_DENSE: return launch_mode<D, MODE_DENSE, true>(tq, tk, tv, p, grid, stream, serialize_launch);
@@ -1527,8 +1629,38 @@ int launch_d(int mode, const CUtensorMap& tq, const CUtensorMap& tk, const CUten
     case MODE_DENSE_CS1:
       return splits ? launch_mode<D, MODE_DENSE_CS1, true>(tq, tk, tv, p, grid, stream, serialize_launch)
                     : launch_mode<D, MODE_DENSE_CS1, false>(tq, tk, tv, p, grid, stream, serialize_launch);
-    default: return launch_mode<D, MODE_CSP, false>(tq, tk, tv, p, grid, stream, serialize_launch);
+    default: return launch_mode<D, MODE_CSP, false>(tq, tk, tv, p, grid, stream, serialize_launch, gm);
   }
+}
+
+}  // namespace
+
+namespace {
+
+// A [B, H, L, D] view as a 2-D tensor of rows: key l of (b, h) is row b * rb + h * rh + l, from column h * ch on.
+struct RowsView {
+  bool ok;
+  int rb, rh, ch;
+  int64_t rows, width;
+};
+RowsView rows_view(int B, int H, int L, int D, int64_t sb, int64_t sh, int64_t sl) {
+  RowsView r = {};
+  if (sl < D || (B > 1 && sb % sl != 0)) return r;
+  const int64_t rb = B > 1 ? sb / sl : 0;
+  int64_t rh = 0, ch = 0;
+  if (H > 1) {
+    if (sh % sl == 0) rh = sh / sl;
+    else if ((H - 1) * sh + D <= sl) ch = sh;
+    else return r;
+  }
+  r.rows = (B - 1) * rb + (H - 1) * rh + L;
+  r.width = (H - 1) * ch + D;
+  if (r.rows > 0x7fffffff || r.width > 0x7fffffff || sl * 2 >= (1ll << 40)) return r;
+  r.rb = (int)rb;
+  r.rh = (int)rh;
+  r.ch = (int)ch;
+  r.ok = true;
+  return r;
 }
 
 }  // namespace
@@ -1707,9 +1839,26 @@ int launch_attention(const lvar_attn_args* a, int mode, cudaStream_t stream) {
     if (rc != LVAR_OK) return rc;
   }
 
+  GatherMaps<MODE_CSP> gm = {};
+  if (mode == MODE_CSP) {
+    // K and V rows are gathered by TMA where each tensor is one 2-D tensor of rows of pitch sl: batches are whole rows apart,
+    // and heads are whole rows apart ([B, H, L, D]) or lie side by side inside a row ([B, L, H, D]).  Anything else goes
+    // through cp.async.
+    const RowsView kr = rows_view(a->B, a->H, a->Lkv, a->D, a->k_sb, a->k_sh, a->k_sl);
+    const RowsView vr = rows_view(a->B, a->H, a->Lkv, a->D, a->v_sb, a->v_sh, a->v_sl);
+    if (kr.ok && vr.ok) {
+      p.gather4 = 1;
+      p.kg_rb = kr.rb; p.kg_rh = kr.rh; p.kg_ch = kr.ch;
+      p.vg_rb = vr.rb; p.vg_rh = vr.rh; p.vg_ch = vr.ch;
+      rc = encode_rows_map(&gm.k, a->k, kr.rows, kr.width, a->k_sl);
+      if (rc != LVAR_OK) return rc;
+      rc = encode_rows_map(&gm.v, a->v, vr.rows, vr.width, a->v_sl);
+      if (rc != LVAR_OK) return rc;
+    }
+  }
   const bool serialize_launch = (a->sched_flags & LVAR_SCHED_SERIALIZE_LAUNCH) != 0;
-  if (a->D == 128) return launch_d<128>(mode, tq, tk, tv, p, grid, stream, serialize_launch);
-  return launch_d<64>(mode, tq, tk, tv, p, grid, stream, serialize_launch);
+  if (a->D == 128) return launch_d<128>(mode, tq, tk, tv, p, grid, stream, serialize_launch, gm);
+  return launch_d<64>(mode, tq, tk, tv, p, grid, stream, serialize_launch, gm);
 }
 
 }  // namespace lvar

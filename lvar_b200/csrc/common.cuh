@@ -32,6 +32,10 @@ int fail(int code, const char* fmt, ...);
 int encode_bhld_map(CUtensorMap* out, const void* base, int B, int H, int L, int D, int64_t sb, int64_t sh,
                     int64_t sl, int box_rows);
 
+// Encodes a 2-D bf16 tensor map over `rows` rows of `width` elements, `pitch` elements apart, with a box of one row of 64
+// elements and 128-byte swizzle, as the four-row TMA gather wants it.  Returns an LVAR_* code.
+int encode_rows_map(CUtensorMap* out, const void* base, int64_t rows, int64_t width, int64_t pitch);
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Bilinear resize between two square token grids (align_corners = False): the four source tokens and the
