@@ -352,6 +352,10 @@ __device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t (&r)[
 }
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld_x16(taddr, r); }
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld_x32(taddr, r); }
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[64]) {
+  tmem_ld_x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+  tmem_ld_x32(taddr + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
+}
 // Columns [a, b) of the warp's 32 TMEM lanes become -inf (a, b warp-uniform).
 __device__ __forceinline__ void mask_columns(uint32_t taddr, int a, int b) {
   const uint32_t ninf = 0xff800000u;
