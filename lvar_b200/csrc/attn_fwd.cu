@@ -1180,7 +1180,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 }
               } else {
                 gather_half_tile<D>(smem_u32(sK + st * SM::kTile), kbase, p.k_sl, kv, lane, warp & 1);
-                // each lane's arrival follows its own copies; nobody waits here (the MMA warp fences the proxies)
+                // each lane's arrival follows its own copies; nobody waits here (the issuing lane fences the proxies)
                 cp_async_mbar_arrive(&bars->k_full[st]);
               }
               if (j + 1 < rounds) gather_rows_of_tile(kv, idx, e.aux, j + 1, p.Lkv, lane, p.status);
