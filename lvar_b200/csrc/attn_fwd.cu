@@ -193,6 +193,7 @@ struct Bars {
   SchedEntry sched[kSchedStages];
   uint32_t tmem_base;
   int abort_flag;
+  int fetched[4];  // column-sparse: tiles that the gather warps (8, 9: K; 12, 13: V) have fetched, written as they leave
   uint64_t xchg_back;  // split tile, column-sum sweep to follow: slot 1's merged row constants are in place (128 arrivals)
 };
 static_assert(sizeof(Bars) <= 512, "barrier block too large");
@@ -387,6 +388,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         break;
       }
     }
+  };
+  // Column-sparse: half of a tile of 128 consecutive keys, 64 columns or with head dimension 64 (whose maps have a box of 64
+  // rows, see launch_attention) 64 rows.
+  auto load_run = [&](uint8_t* tile, const CUtensorMap* map, uint64_t* full, int key, const Item& im, int half) {
+    if (D == 128) tma_load_4d(tile + half * 16384, map, full, half * 64, key, im.h, im.b);
+    else tma_load_4d(tile + half * 8192, map, full, 0, key + half * 64, im.h, im.b);
   };
   uint8_t* sQ = smem + SM::kQ;
   uint8_t* sK = smem + SM::kK;
@@ -1143,17 +1150,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               ok = __all_sync(0xffffffffu, mbar_wait(&bars->k_empty[st], ((kc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
               if (!ok) break;
               uint8_t* tile = sK + st * SM::kTile;
-              // every warp that fetches arrives for every tile, so that none falls two phases behind on tiles it is not needed for
-              if (lane == 0) {
-                if (warp == 8) mbar_arrive_expect_tx(&bars->k_full[st], SM::kTile);
-                else mbar_arrive(&bars->k_full[st]);
-              }
+              // every warp that fetches arrives for every tile, so that none falls two phases behind on tiles it is not needed
+              // for, and announces half of the tile
+              if (lane == 0) mbar_arrive_expect_tx(&bars->k_full[st], SM::kTile / 2);
               if (tile4_is_run(kv, e.aux, j, p.Lkv, lane)) {
-                // 128 consecutive keys (the local band of a list): one tile copy
-                if (lane == 0 && warp == 8) {
-                  for (int s2 = 0; s2 < NSUB; ++s2)
-                    tma_load_4d(tile + s2 * 16384, &tmK, &bars->k_full[st], s2 * 64, kv[0], im.h, im.b);
-                }
+                // 128 consecutive keys (the local band of a list): one copy a warp
+                if (lane == 0) load_run(tile, &tmK, &bars->k_full[st], kv[0], im, warp & 1);
               } else if (mine) {
                 tma_gather4(tile + sub * 16384 + lane * 512, &gm.k, &bars->k_full[st], col0 + sub * 64, row0 + kv[0], row0 + kv[1],
                             row0 + kv[2], row0 + kv[3]);
@@ -1173,8 +1175,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 // 128 consecutive keys (the local band of a list): one tile copy instead of 2048 row pieces
                 if (lane == 0 && warp == 8) {
                   mbar_arrive_expect_tx(&bars->k_full[st], SM::kTile);
-                  for (int sub = 0; sub < NSUB; ++sub)
-                    tma_load_4d(sK + st * SM::kTile + sub * 16384, &tmK, &bars->k_full[st], sub * 64, kv[0], im.h, im.b);
+                  for (int half = 0; half < 2; ++half)
+                    load_run(sK + st * SM::kTile, &tmK, &bars->k_full[st], kv[0], im, half);
                 } else {
                   mbar_arrive(&bars->k_full[st]);
                 }
@@ -1191,14 +1193,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (!ok) break;
         if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
       }
-      if (MODE == MODE_CSP) cp_async_wait<0>();  // drains on abort too
-      // Drain on abort: copies in flight must land before the CTA's shared memory is released.
+      if (MODE == MODE_CSP && lane == 0) bars->fetched[warp - 8] = kc;
+      // Drain on abort: copies in flight must land before the CTA's shared memory is released (gathered tiles: see the
+      // teardown).
       if (lane == 0 && bars->abort_flag) {
         const uint64_t t0 = globaltimer_ns();
         if (nq_items > 0 && warp == 8)
           while (!mbar_try_wait(&bars->q_full, (nq_items - 1) & 1) && globaltimer_ns() - t0 < 2000000000ull) {
           }
-        if (MODE != MODE_CSP || p.gather4) {
+        if (MODE != MODE_CSP) {
           for (int c = max(0, kc - kStages); c < kc; ++c) {
             const uint64_t t1 = globaltimer_ns();
             while (!mbar_try_wait(&bars->k_full[c % kStages], (c / kStages) & 1) &&
@@ -1244,16 +1247,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             ok = __all_sync(0xffffffffu, mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
             if (!ok) break;
             uint8_t* tile = sV + st * SM::kTile;
-            if (lane == 0) {
-              if (warp == 12) mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile);
-              else mbar_arrive(&bars->v_full[st]);
-            }
+            if (lane == 0) mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile / 2);
             if (tile4_is_run(kv, e.aux, j, p.Lkv, lane)) {
-              // 128 consecutive keys (the local band of a list): one tile copy
-              if (lane == 0 && warp == 12) {
-                for (int s2 = 0; s2 < NSUB; ++s2)
-                  tma_load_4d(tile + s2 * 16384, &tmV, &bars->v_full[st], s2 * 64, kv[0], im.h, im.b);
-              }
+              if (lane == 0) load_run(tile, &tmV, &bars->v_full[st], kv[0], im, warp & 1);
             } else if (mine) {
               tma_gather4(tile + sub * 16384 + lane * 512, &gm.v, &bars->v_full[st], col0 + sub * 64, row0 + kv[0], row0 + kv[1],
                           row0 + kv[2], row0 + kv[3]);
@@ -1272,8 +1268,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             if (tile_is_run(kv, e.aux, j, p.Lkv, lane)) {
               if (lane == 0 && warp == 12) {
                 mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile);
-                for (int sub = 0; sub < NSUB; ++sub)
-                  tma_load_4d(sV + st * SM::kTile + sub * 16384, &tmV, &bars->v_full[st], sub * 64, kv[0], im.h, im.b);
+                for (int half = 0; half < 2; ++half)
+                  load_run(sV + st * SM::kTile, &tmV, &bars->v_full[st], kv[0], im, half);
               } else {
                 mbar_arrive(&bars->v_full[st]);
               }
@@ -1288,15 +1284,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (!ok) break;
         if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
       }
-      cp_async_wait<0>();
-      if (lane == 0 && p.gather4 && bars->abort_flag) {
-        for (int c = max(0, vc - kStages); c < vc; ++c) {
-          const uint64_t t1 = globaltimer_ns();
-          while (!mbar_try_wait(&bars->v_full[c % kStages], (c / kStages) & 1) &&
-                 globaltimer_ns() - t1 < 2000000000ull) {
-          }
-        }
-      }
+      if (lane == 0) bars->fetched[warp - 10] = vc;
       }
     } else if (warp != 15 && elect_one()) {
       // One lane runs the whole role: the issue of sixteen MMAs took it 640 cycles against 880 for a warp that runs
@@ -1582,6 +1570,32 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+  if constexpr (MODE == MODE_CSP) {
+    // Abort: the gather warps stay until the copies in flight have landed.  A tile's barrier completes when both warps have
+    // arrived and the bytes they announced are there; no role listens any more, so the warp that left first arrives for the
+    // tiles that only the other one has fetched, which the stages limit to one phase of each barrier.
+    const bool k_warp = warp == 8 || warp == 9, v_warp = warp == 12 || warp == 13;
+    if (bars->abort_flag && (k_warp || v_warp)) {
+      const int me = k_warp ? warp - 8 : warp - 10;
+      uint64_t* full = k_warp ? bars->k_full : bars->v_full;
+      const int own = bars->fetched[me], other = bars->fetched[me ^ 1];
+      for (int c = own; c < other; ++c) {
+        if (!p.gather4 || lane == 0) mbar_arrive(&full[c % kStages]);
+      }
+      if (lane == 0) {
+        // a tile whose stage the other warp has filled again was consumed before that
+        for (int c = max(0, max(own, other) - kStages); c < own; ++c) {
+          const uint64_t t0 = globaltimer_ns();
+          while (!mbar_try_wait(&full[c % kStages], (c / kStages) & 1)) {
+            if (globaltimer_ns() - t0 > 2000000000ull) {
+              if (p.status) atomicCAS(p.status, 0, (int)DEV_TIMEOUT_DRAIN);
+              break;
+            }
+          }
+        }
+      }
+    }
+  }
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -1832,12 +1846,14 @@ int launch_attention(const lvar_attn_args* a, int mode, cudaStream_t stream) {
   CUtensorMap tq, tk, tv;
   int rc = encode_bhld_map(&tq, a->q, a->B, a->H, a->Lq, a->D, a->q_sb, a->q_sh, a->q_sl, 128);
   if (rc != LVAR_OK) return rc;
-  rc = encode_bhld_map(&tk, a->k, a->B, a->H, a->Lkv, a->D, a->k_sb, a->k_sh, a->k_sl, 128);
+  // column-sparse: two warps share the copy of a run of keys, by columns or with head dimension 64 by rows
+  const int kv_box = mode == MODE_CSP && a->D == 64 ? 64 : 128;
+  rc = encode_bhld_map(&tk, a->k, a->B, a->H, a->Lkv, a->D, a->k_sb, a->k_sh, a->k_sl, kv_box);
   if (rc != LVAR_OK) return rc;
   if (qk_only) {
     tv = tk;  // never used by the kernel in this mode
   } else {
-    rc = encode_bhld_map(&tv, a->v, a->B, a->H, a->Lkv, a->D, a->v_sb, a->v_sh, a->v_sl, 128);
+    rc = encode_bhld_map(&tv, a->v, a->B, a->H, a->Lkv, a->D, a->v_sb, a->v_sh, a->v_sl, kv_box);
     if (rc != LVAR_OK) return rc;
   }
 

@@ -1,0 +1,68 @@
+"""A wait limit of zero in every form of the attention kernel: the launch gives up at its first unfinished wait, returns with
+a status word, and leaves the device, the work counter and the next call as they were.
+
+Nothing faults here: a wait that runs out ends in an ordinary return."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+B, H, LQ, LKV, ROWS = 2, 3, 600, 1500, 256
+
+
+def _qkv(D):
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    return [torch.randn(B, H, n, D, generator=gen, device="cuda").bfloat16() for n in (LQ, LKV, LKV)]
+
+
+def _copy_only(x):
+    """The values of x with batches that are not whole rows apart: no 2-D tensor of rows, so rows are copied."""
+    b, h, L, D = x.shape
+    y = torch.empty(b * (h * L * D + 8), device=x.device, dtype=x.dtype).as_strided(x.shape, (h * L * D + 8, L * D, D, 1))
+    return y.copy_(x)
+
+
+def _lists(G):
+    """Whole runs of consecutive keys, scattered tiles between them and a short last tile."""
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    idx = torch.arange(LKV, device="cuda", dtype=torch.int32).expand(B, H, G, LKV).clone()
+    for at in (128, 512, 768):
+        idx[..., at:at + 128] = torch.randint(0, LKV, (B, H, G, 128), generator=gen, device="cuda", dtype=torch.int32)
+    return idx, torch.full((B, H, G), 1100, dtype=torch.int32, device="cuda")
+
+
+def _csp(layout):
+    def call(K, D, status):
+        q, k, v = _qkv(D)
+        if layout == "copies":
+            k, v = _copy_only(k), _copy_only(v)
+        idx, counts = _lists(-(-LQ // ROWS))
+        return (K.csp_attn_fwd(q, k, v, idx, counts, torch.zeros_like(q), 1, ROWS, status=status),)
+    return call
+
+
+def _block(K, D, status):
+    q, k, v = _qkv(D)
+    mask = (torch.arange(-(-LKV // 128), device="cuda")[None] + torch.arange(-(-LQ // 128), device="cuda")[:, None]) % 3 != 0
+    return (K.block_sparse_attn_fwd(q, k, v, mask, status=status),)
+
+
+CALLS = {"csp rows": _csp("rows"), "csp copies": _csp("copies"), "block": _block}
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("form", list(CALLS))
+def test_wait_limit_zero_returns_a_status_and_the_next_call_is_right(form, D, monkeypatch):
+    from lvar_b200 import _lib
+    from lvar_b200 import kernels as K
+    call = CALLS[form]
+    good = K.new_status("cuda")
+    want = call(K, D, good)
+    for _ in range(3):
+        given_up = K.new_status("cuda")
+        with monkeypatch.context() as m:
+            m.setattr(_lib, "DEFAULT_WAIT_NS", 0)
+            call(K, D, given_up)
+        assert K.read_status(given_up)[0] == 6
+        assert all(torch.equal(a, b) for a, b in zip(call(K, D, good), want))
+    assert K.read_status(good)[0] == 0
