@@ -149,8 +149,8 @@ struct Smem {
   // aux: barriers then scalars then the step list
   static constexpr int kBarBytes = 512;
   static constexpr int kList = kAux + kBarBytes;
-  static constexpr int kNegC = kList + kSchedStages * 2 * kMaxSteps * 2;    // [slot][128] fp32: -(M_i + log2 L_i)
-  static constexpr int kXchg = kNegC + 2 * 128 * 4;  // [item parity][m_ref, l, m_true][128] fp32: slot 1 -> slot 0 of a split tile
+  static constexpr int kNegC = kList + kSchedStages * 2 * kMaxSteps * 2;    // [item parity][slot][128] fp32: -(M_i + log2 L_i)
+  static constexpr int kXchg = kNegC + 2 * 2 * 128 * 4;  // [item parity][m_ref, l, m_true][128] fp32: slot 1 -> slot 0 of a split tile
   // MODE_DENSE_CS1: per-warp column sums of a tile [slot][buffer][warp][128] fp32, and the rows' sums [slot][128]
   static constexpr int kPart = kXchg + 2 * 3 * 128 * 4;
   static constexpr int kRowL = kPart + 2 * 2 * 4 * 128 * 4;
@@ -190,6 +190,7 @@ struct Bars {
   uint64_t part_full[2][2];  // MODE_DENSE_CS1: the four warps' column sums of a tile are in shared memory [slot][buffer]
   uint64_t rowl_full[2];     // MODE_DENSE_CS1: the rows' probability sums of an item are in shared memory [slot]
   uint64_t cs_full[2], cs_empty[2];  // column-sum sweep: S^T of a slot has landed / has been read
+  uint64_t meet[2];  // column-sum sweep: the 128 threads of a softmax warpgroup meet
   SchedEntry sched[kSchedStages];
   uint32_t tmem_base;
   int abort_flag;
@@ -257,6 +258,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (kHasCs) {
       mbar_init(&bars->cs_full[s], 1);
       mbar_init(&bars->cs_empty[s], 128);
+      mbar_init(&bars->meet[s], 128);
     }
     if (MODE == MODE_DENSE_CS1) {
       mbar_init(&bars->part_full[s][0], 128);
@@ -368,11 +370,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     return true;
   };
 
-  // the 128 threads of softmax warpgroup s meet at named barrier 1 + s
-  auto wg_sync = [](int s) {
-    if (s == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
-    else asm volatile("bar.sync 2, 128;" ::: "memory");
-  };
   // Both slots want the same KV tile in round r (it is then loaded once).
   auto round_shared = [&](const uint16_t* l0, const uint16_t* l1, const SchedEntry& e, int r) {
     return r < e.n0 && r < e.n1 && (MODE == MODE_BLOCK ? ((l0[r] ^ l1[r]) & 0xFFF) == 0 : e.off1 == 0);
@@ -471,11 +468,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     int n_s = 0;  // S tiles consumed by this slot so far (parity of s_full)
     int n_pv = 0;  // P V products of this slot waited for so far (parity of pv_done)
     int n_cs = 0;          // column-sum sweep: S^T tiles read (parity of cs_full)
+    int n_meet = 0;        // column-sum sweep: meetings of this warpgroup (parity of meet)
     int n_xc[2] = {0, 0};  // split tiles merged so far, by item parity (parity of xchg_full)
     int n_back = 0;        // split tiles whose constants came back (parity of xchg_back)
     int n_part[2] = {0, 0};  // MODE_DENSE_CS1: tiles reduced per buffer (parity of part_full)
     int n_rowl = 0;          // MODE_DENSE_CS1: items with tiles (parity of rowl_full)
     bool ok = true;
+    // The 128 threads of the warpgroup meet.  Not at a named barrier, whose wait has no limit: a warp that has given up an
+    // earlier wait does not come.
+    auto wg_meet = [&]() -> bool {
+      mbar_arrive(&bars->meet[s]);
+      const bool met = __all_sync(0xffffffffu, mbar_wait(&bars->meet[s], n_meet & 1, wc, DEV_TIMEOUT_SOFTMAX));
+      ++n_meet;
+      return met;
+    };
 
     for (int n = 0; ok; ++n) {
       SchedEntry e;
@@ -487,6 +493,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const bool row_ok = row < im.row_end[s];
       const int cnt_total = (MODE == MODE_CSP) ? e.aux : 0;
       const int n_mine = s == 0 ? e.n0 : e.n1;
+      // row constants of this item's column-sum sweep; every warp has left the item before the last one when this one begins
+      float* nc_item = negc + (n & 1) * 256;
 
       // the keys from this slot's first KV tile on (slot 1 of a split tile starts in the middle of the list)
       const int key0 = (SPLIT && MODE != MODE_BLOCK && s == 1) ? e.off1 * 128 : 0, n_keys = p.Lkv - key0;
@@ -810,7 +818,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           m_stat = fmaxf(m_true, x[256 + r_in_tile]);
           l_stat = l > 0.f ? l * fast_exp2(mm - m_stat) : 0.f;
           if (e.n1 > 0) {
-            negc[128 + r_in_tile] = (row_ok && l > 0.f) ? -(mm + log2f(l)) : -INFINITY;
+            nc_item[128 + r_in_tile] = (row_ok && l > 0.f) ? -(mm + log2f(l)) : -INFINITY;
             mbar_arrive(&bars->xchg_back);
           }
         }
@@ -859,7 +867,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               m_ref = mm;
               l = lt;
               if (kHasCs && other) {
-                negc[128 + r_in_tile] = (row_ok && lt > 0.f) ? -(mm + log2f(lt)) : -INFINITY;
+                nc_item[128 + r_in_tile] = (row_ok && lt > 0.f) ? -(mm + log2f(lt)) : -INFINITY;
                 mbar_arrive(&bars->xchg_back);
               }
             }
@@ -981,10 +989,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if (!ok) break;
           ++n_back;
         } else {
-          negc[s * 128 + r_in_tile] = (row_ok && l > 0.f) ? -(m_ref + log2f(l)) : -INFINITY;
-          wg_sync(s);  // the warpgroup's 128 constants are in place
+          nc_item[s * 128 + r_in_tile] = (row_ok && l > 0.f) ? -(m_ref + log2f(l)) : -INFINITY;
+          ok = wg_meet();  // the warpgroup's 128 constants are in place
+          if (!ok) break;
         }
-        const float4* nc4 = reinterpret_cast<const float4*>(negc + s * 128);
+        const float4* nc4 = reinterpret_cast<const float4*>(nc_item + s * 128);
         // a tile with fewer than 128 queries carries -inf constants, which the polynomial cannot take
         const bool full_tile = im.row_end[s] - im.row0[s] >= 128;
         const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2);
@@ -1022,7 +1031,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         ok = full_tile ? cs_sweep(std::integral_constant<uint32_t, kCsPolyMask>{})
                        : cs_sweep(std::integral_constant<uint32_t, 0u>{});
         if (!ok) break;
-        wg_sync(s);  // nobody still reads the constants
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);

@@ -47,7 +47,22 @@ def _block(K, D, status):
     return (K.block_sparse_attn_fwd(q, k, v, mask, status=status),)
 
 
+def _sums(form):
+    def call(K, D, status):
+        q, k, v = _qkv(D)
+        if form == "two sweeps":
+            return K.dense_colsum_attn_fwd(q, k, v, return_stats=True, status=status)
+        if form == "no output":
+            return K.colsum_tiles_fwd(q, k, return_stats=True, status=status)
+        M, L = (torch.full((B, H, LQ), x, device="cuda") for x in (2.0, 300.0))
+        if form == "given, no output":
+            return (K.colsum_tiles_fwd(q, k, stats=(M, L), status=status),)
+        return K.dense_colsum_attn_given_fwd(q, k, v, M, L, return_stats=True, status=status)
+    return call
+
+
 CALLS = {"csp rows": _csp("rows"), "csp copies": _csp("copies"), "block": _block}
+CALLS |= {f"sums, {form}": _sums(form) for form in ("two sweeps", "no output", "given, no output", "given")}
 
 
 @pytest.mark.parametrize("D", [64, 128])
