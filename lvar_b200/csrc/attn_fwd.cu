@@ -547,9 +547,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tmem_wait_ld();
           tc_fence_before();
           mbar_arrive(&bars->s_read);
-          if (D == 128 && j > 0) {
-            // P of the tile before has been read.  Asked here, not where the answer is needed, with head dimension 128: 152
-            // against 168 us for 1600 x 4121 x 32 (the products of the two slots then alternate).
+          if (j > 0) {
+            // P of the tile before has been read.  Asked here, not where the answer is needed, so that the products of the two
+            // slots alternate: 1600 x 4121 x 32 152 us against 168, with head dimension 64 128 against 146 (a score buffer per
+            // slot, for which there is room then, 148).
             ok = __all_sync(0xffffffffu, mbar_wait(&bars->pv_done[s], n_pv & 1, wc, DEV_TIMEOUT_SOFTMAX));
             if (!ok) break;
             ++n_pv;
@@ -559,10 +560,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           auto half_tile = [&](const uint32_t (&r)[64], int h) {
             const uint64_t nA = pack_f32x2(ncst[2 * h], ncst[2 * h]), nB = pack_f32x2(ncst[2 * h + 1], ncst[2 * h + 1]);
             uint32_t pk[32];
-            bool pv_early = false;
 #pragma unroll
             for (int kk = 0; kk < 16; ++kk) {
-              if (D == 64 && h == 0 && kk == 12) pv_early = mbar_test_wait(&bars->pv_done[s], n_pv & 1);
               const uint64_t X = ffma2(pack_f32x2(__uint_as_float(r[4 * kk]), __uint_as_float(r[4 * kk + 1])), sc2, nA);
               const uint64_t Y = ffma2(pack_f32x2(__uint_as_float(r[4 * kk + 2]), __uint_as_float(r[4 * kk + 3])), sc2, nB);
               float x0, x1, y0, y1;
@@ -576,19 +575,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               pk[2 * kk] = pack_bf16x2(x0, x1);
               pk[2 * kk + 1] = pack_bf16x2(y0, y1);
             }
-            if (D == 64 && h == 0 && j > 0) {
-              // the product that reads the P of the tile before is over (asked ahead: the answer is there by now)
-              if (!__all_sync(0xffffffffu, pv_early)) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&bars->pv_done[s], n_pv & 1, wc, DEV_TIMEOUT_SOFTMAX));
-                if (!ok) return;
-              }
-              ++n_pv;
-              tc_fence_after();
-            }
             tmem_st_16x128b_x16(tP + ((uint32_t)(16 * h) << 16), pk);
           };
           half_tile(ra, 0);
-          if (!ok) break;
+          if (!ok) break;  // never taken; without it the halves are laid out differently (1000 x 2999 x 16: 33.0 -> 33.7 us)
           half_tile(rb, 1);
           tmem_wait_st();
           tc_fence_before();
