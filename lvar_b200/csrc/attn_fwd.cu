@@ -523,7 +523,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               if (Lr > 0.f) c = -(p.M_in[si] + log2f(Lr));
             }
           }
-          ncst[i] = c;
+          // +inf (M = -inf with L > 0) would take the -inf of masked columns to NaN; exp2 overflows either way, NaN stays NaN
+          ncst[i] = c > FLT_MAX ? FLT_MAX : c;
         }
         uint64_t rs2[4] = {0ull, 0ull, 0ull, 0ull};  // packed partial sums of p over this thread's columns, per row
         const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2);
