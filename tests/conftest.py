@@ -1,3 +1,5 @@
+import ctypes
+import subprocess
 import sys
 from pathlib import Path
 
@@ -51,3 +53,29 @@ def golden_scalekv():
 @pytest.fixture(scope="session")
 def golden_prologue():
     return load_golden("prologue_ref.npz")
+
+
+_ROWS_VIEW = """
+#include "rows_view.cuh"
+extern "C" int rows_view(int B, int H, int L, int D, long long sb, long long sh, long long sl, long long* out) {
+  const lvar::RowsView r = lvar::rows_view(B, H, L, D, sb, sh, sl);
+  out[0] = r.rb; out[1] = r.rh; out[2] = r.ch; out[3] = r.rows; out[4] = r.width;
+  return r.ok ? 1 : 0;
+}
+"""
+
+
+@pytest.fixture(scope="session")
+def rows_view(tmp_path_factory):
+    """The library's gather rule, compiled for the host: (shape, strides) -> (rb, rh, ch, rows, width), or None for the copies."""
+    d = tmp_path_factory.mktemp("rows_view")
+    (d / "rows_view.cpp").write_text(_ROWS_VIEW)
+    subprocess.run(["g++", "-O1", "-shared", "-fPIC", "-I", str(ROOT / "lvar_b200" / "csrc"), "-o", str(d / "rows_view.so"),
+                    str(d / "rows_view.cpp")], check=True)
+    fn = ctypes.CDLL(str(d / "rows_view.so")).rows_view
+    fn.argtypes = [ctypes.c_int] * 4 + [ctypes.c_longlong] * 3 + [ctypes.POINTER(ctypes.c_longlong)]
+
+    def call(shape, strides):
+        out = (ctypes.c_longlong * 5)()
+        return tuple(out) if fn(*shape, *strides[:3], out) else None
+    return call
