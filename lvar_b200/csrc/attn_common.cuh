@@ -1,4 +1,4 @@
-// Device helpers shared by the attention kernels: the cp.async row gather into a swizzled tile and the
+// Device helpers shared by the attention kernels: the row gathers into a swizzled tile (TMA requests or cp.async copies) and the
 // register-level softmax pieces (3-input max, packed exp2 + bf16 packing).
 #pragma once
 

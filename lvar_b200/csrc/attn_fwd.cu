@@ -22,7 +22,7 @@
 // release seen, product, 1100 cycles a slot when the tensor pipe is otherwise idle (measured alone), 1300 beside P V
 // products.  Taking turns also keeps the warpgroups out of step, which is worth more than buffers: with head dimension
 // 64 there is room for a score buffer per slot, and dense attention took 720 us with it against 634.
-// Shared memory: Q0,Q1 + 2 K stages + 2 V stages, all 128-byte-swizzled [128][64]
+// Shared memory: Q0,Q1 + 2 K stages + 2 V stages (4 + 4 with head dimension 64), all 128-byte-swizzled [128][64]
 // bf16 sub-tiles (exactly what a [64 x 128] TMA box writes), K-major for Q/K and MN-major for V.
 //
 // Softmax keeps a per-row reference maximum that is only moved when the running maximum exceeds it
@@ -397,11 +397,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint8_t* sK = smem + SM::kK;
   uint8_t* sV = smem + SM::kV;
 
-  // The P V products of rounds [r0, r1) of an item; one thread.
+  // The P V products of an item; one thread.
   struct PvState {
     uint32_t vc = 0, n_p0 = 0, n_p1 = 0, n_o0 = 1, n_o1 = 1;
   };
-  auto pv_rounds = [&](PvState& ps, const SchedEntry& e, int n, int r0, int r1) -> bool {
+  auto pv_rounds = [&](PvState& ps, const SchedEntry& e, int n) -> bool {
     constexpr uint32_t DESC_HI = sw128_desc_hi(1024);
     constexpr uint32_t TILE16 = SM::kTile >> 4;
     const uint32_t v_lo = sw128_desc_lo(smem_u32(sV), 16384);
@@ -410,11 +410,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait(bar, parity, wc, DEV_TIMEOUT_MMA); };
     auto issue = [&](uint32_t tO, uint32_t tPs, uint32_t st, uint32_t acc) {
       const uint32_t vb = v_lo + st * TILE16;
-      umma_ts_if(1u, tO, tPs, vb, DESC_HI, IDESC_PV, acc);
+      umma_ts(tO, tPs, vb, DESC_HI, IDESC_PV, acc);
 #pragma unroll
-      for (int i = 1; i < 8; ++i) umma_ts_if(1u, tO, tPs + i * 8, vb + i * 128, DESC_HI, IDESC_PV, 1u);
+      for (int i = 1; i < 8; ++i) umma_ts(tO, tPs + i * 8, vb + i * 128, DESC_HI, IDESC_PV, 1u);
     };
-    for (int r = r0; r < r1; ++r) {
+    for (int r = 0; r < max(e.n0, e.n1); ++r) {
       const bool h0 = r < e.n0, h1 = r < e.n1, shared = round_shared(l0, l1, e, r);
       if (h0) {
         const uint32_t st = ps.vc % kStages;
@@ -423,7 +423,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (r == 0 && !wait(&bars->o_empty[0], ps.n_o0 & 1)) return false;
         if (!wait(&bars->p_full[0], ps.n_p0 & 1)) return false;
         ++ps.n_p0;
-        // column-sparse: V came by cp.async (generic proxy), the MMA reads it through the async proxy
+        // column-sparse: V rows that were copied (cp.async, generic proxy) are read by the MMA through the async proxy.  Gathered
+        // rows need no fence, but a branch around it gains nothing (131 -> 130 us) and costs the copies (D = 64 106 -> 109)
         if (MODE == MODE_CSP) fence_proxy_async_smem();
         tc_fence_after();
         issue(tmem_base + TM_O, tmem_base, st, r > 0 ? 1u : 0u);
@@ -1228,67 +1229,67 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     bool ok = true;
     if (MODE == MODE_CSP && warp < 14) {
       if constexpr (MODE == MODE_CSP) {
-      int vc = 0;
-      for (int n = 0; ok; ++n) {
-        SchedEntry e;
-        ok = __all_sync(0xffffffffu, acquire_item(n, e, DEV_TIMEOUT_PRODUCER));
-        if (!ok || e.item < 0) break;
-        const Item im = decode(e.item, e.half);
-        const int rounds = max(e.n0, e.n1);
-        const int32_t* idx = p.indices + im.b * p.i_sb + im.h * p.i_sh + (int64_t)im.group * p.i_sg;
-        if (p.gather4) {
-          const int row0 = im.b * p.vg_rb + im.h * p.vg_rh, col0 = im.h * p.vg_ch;
-          const int sub = D == 128 ? (warp & 1) : 0;
-          const bool mine = D == 128 || (lane >> 4) == (warp & 1);
-          int kv[4], nx[4];
-          if (rounds > 0) gather4_read(nx, idx, e.aux, 0, lane);
-          for (int j = 0; j < rounds; ++j) {
-            gather4_check(nx, p.Lkv, nullptr);
+        int vc = 0;
+        for (int n = 0; ok; ++n) {
+          SchedEntry e;
+          ok = __all_sync(0xffffffffu, acquire_item(n, e, DEV_TIMEOUT_PRODUCER));
+          if (!ok || e.item < 0) break;
+          const Item im = decode(e.item, e.half);
+          const int rounds = max(e.n0, e.n1);
+          const int32_t* idx = p.indices + im.b * p.i_sb + im.h * p.i_sh + (int64_t)im.group * p.i_sg;
+          if (p.gather4) {
+            const int row0 = im.b * p.vg_rb + im.h * p.vg_rh, col0 = im.h * p.vg_ch;
+            const int sub = D == 128 ? (warp & 1) : 0;
+            const bool mine = D == 128 || (lane >> 4) == (warp & 1);
+            int kv[4], nx[4];
+            if (rounds > 0) gather4_read(nx, idx, e.aux, 0, lane);
+            for (int j = 0; j < rounds; ++j) {
+              gather4_check(nx, p.Lkv, nullptr);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) kv[i] = nx[i];
-            if (j + 1 < rounds) gather4_read(nx, idx, e.aux, j + 1, lane);
-            const int st = vc % kStages;
-            ok = __all_sync(0xffffffffu, mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
-            if (!ok) break;
-            uint8_t* tile = sV + st * SM::kTile;
-            if (lane == 0) mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile / 2);
-            if (tile4_is_run(kv, e.aux, j, p.Lkv, lane)) {
-              if (lane == 0) load_run(tile, &tmV, &bars->v_full[st], kv[0], im, warp & 1);
-            } else if (mine) {
-              tma_gather4(tile + sub * 16384 + lane * 512, &gm.v, &bars->v_full[st], col0 + sub * 64, row0 + kv[0], row0 + kv[1],
-                          row0 + kv[2], row0 + kv[3]);
-            }
-            __syncwarp();
-            ++vc;
-          }
-        } else {
-          const __nv_bfloat16* vbase = p.v + im.b * p.v_sb + im.h * p.v_sh;
-          int kv[4];
-          if (rounds > 0) gather_rows_of_tile(kv, idx, e.aux, 0, p.Lkv, lane, nullptr);
-          for (int j = 0; j < rounds; ++j) {
-            const int st = vc % kStages;
-            ok = __all_sync(0xffffffffu, mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
-            if (!ok) break;
-            if (tile_is_run(kv, e.aux, j, p.Lkv, lane)) {
-              if (lane == 0 && warp == 12) {
-                mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile);
-                for (int half = 0; half < 2; ++half)
-                  load_run(sV + st * SM::kTile, &tmV, &bars->v_full[st], kv[0], im, half);
-              } else {
-                mbar_arrive(&bars->v_full[st]);
+              for (int i = 0; i < 4; ++i) kv[i] = nx[i];
+              if (j + 1 < rounds) gather4_read(nx, idx, e.aux, j + 1, lane);
+              const int st = vc % kStages;
+              ok = __all_sync(0xffffffffu, mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
+              if (!ok) break;
+              uint8_t* tile = sV + st * SM::kTile;
+              if (lane == 0) mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile / 2);
+              if (tile4_is_run(kv, e.aux, j, p.Lkv, lane)) {
+                if (lane == 0) load_run(tile, &tmV, &bars->v_full[st], kv[0], im, warp & 1);
+              } else if (mine) {
+                tma_gather4(tile + sub * 16384 + lane * 512, &gm.v, &bars->v_full[st], col0 + sub * 64, row0 + kv[0], row0 + kv[1],
+                            row0 + kv[2], row0 + kv[3]);
               }
-            } else {
-              gather_half_tile<D>(smem_u32(sV + st * SM::kTile), vbase, p.v_sl, kv, lane, warp & 1);
-              cp_async_mbar_arrive(&bars->v_full[st]);
+              __syncwarp();
+              ++vc;
             }
-            if (j + 1 < rounds) gather_rows_of_tile(kv, idx, e.aux, j + 1, p.Lkv, lane, nullptr);
-            ++vc;
+          } else {
+            const __nv_bfloat16* vbase = p.v + im.b * p.v_sb + im.h * p.v_sh;
+            int kv[4];
+            if (rounds > 0) gather_rows_of_tile(kv, idx, e.aux, 0, p.Lkv, lane, nullptr);
+            for (int j = 0; j < rounds; ++j) {
+              const int st = vc % kStages;
+              ok = __all_sync(0xffffffffu, mbar_wait(&bars->v_empty[st], ((vc / kStages) & 1) ^ 1, wc, DEV_TIMEOUT_PRODUCER));
+              if (!ok) break;
+              if (tile_is_run(kv, e.aux, j, p.Lkv, lane)) {
+                if (lane == 0 && warp == 12) {
+                  mbar_arrive_expect_tx(&bars->v_full[st], SM::kTile);
+                  for (int half = 0; half < 2; ++half)
+                    load_run(sV + st * SM::kTile, &tmV, &bars->v_full[st], kv[0], im, half);
+                } else {
+                  mbar_arrive(&bars->v_full[st]);
+                }
+              } else {
+                gather_half_tile<D>(smem_u32(sV + st * SM::kTile), vbase, p.v_sl, kv, lane, warp & 1);
+                cp_async_mbar_arrive(&bars->v_full[st]);
+              }
+              if (j + 1 < rounds) gather_rows_of_tile(kv, idx, e.aux, j + 1, p.Lkv, lane, nullptr);
+              ++vc;
+            }
           }
+          if (!ok) break;
+          if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
         }
-        if (!ok) break;
-        if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
-      }
-      if (lane == 0) bars->fetched[warp - 10] = vc;
+        if (lane == 0) bars->fetched[warp - 10] = vc;
       }
     } else if (warp != 15 && elect_one()) {
       // One lane runs the whole role: the issue of sixteen MMAs took it 640 cycles against 880 for a warp that runs
@@ -1299,7 +1300,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         ok = acquire_item(n, e, DEV_TIMEOUT_MMA);
         if (!ok || e.item < 0) break;
         if (MODE != MODE_CS_ONLY) {
-          ok = pv_rounds(ps, e, n, 0, max(e.n0, e.n1));
+          ok = pv_rounds(ps, e, n);
           if (!ok) break;
           pv_end(ps, e);
         }
@@ -1312,7 +1313,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     // ============================================================ Q K^T issuer (and the column-sum sweep's products)
     setmaxnreg_dec<kRegsOther>();
     if (elect_one()) {
-      constexpr uint32_t leader = 1u;
       bool ok = true;
       // Descriptor words: the high word is the same for every operand tile, the low word is the tile's
       // base plus (byte offset >> 4) of the stage and of the 16-element K step.
@@ -1323,7 +1323,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       int kc = 0;                // K tiles consumed so far
       int nq_items = 0;          // items with steps (parity of q_full)
       uint32_t n_sr = 1;         // score tiles issued, of either slot (parity of s_read of the one before)
-      uint32_t n_cst[2] = {1, 1};  // column-sum sweep: S^T tiles issued per buffer (parity of cs_empty)
+      uint32_t n_cst[2] = {1, 1};  // column-sum sweep: S^T tiles issued per slot (parity of cs_empty)
       for (int n = 0; ok; ++n) {
         SchedEntry e;
         ok = acquire_item(n, e, DEV_TIMEOUT_MMA);
@@ -1345,7 +1345,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           // the scores of the product before (the other slot's, as a rule) have left the score buffer
           if (!mbar_wait(&bars->s_read, n_sr & 1, wc, DEV_TIMEOUT_MMA)) return false;
           ++n_sr;
-          // column-sparse: K came by cp.async (generic proxy), the MMA reads it through the async proxy
+          // column-sparse: the same for K rows
           if (MODE == MODE_CSP && wait_k) fence_proxy_async_smem();
           tc_fence_after();
           const uint32_t tSs = tmem_base + TM_S;
@@ -1353,7 +1353,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
           for (int kq = 0; kq < KSTEPS_QK; ++kq) {
             const uint32_t koff = (kq >> 2) * 1024 + (kq & 3) * 2;  // (byte offset of the K step) >> 4
-            umma_ss_if(leader, tSs, qa + koff, DESC_HI, kb + koff, DESC_HI, IDESC_QK, kq > 0 ? 1u : 0u);
+            umma_ss(tSs, qa + koff, DESC_HI, kb + koff, DESC_HI, IDESC_QK, kq > 0 ? 1u : 0u);
           }
           umma_commit(&bars->s_full[s]);
           return true;
@@ -1388,19 +1388,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           }
           // ---- column-sum sweep: S_s^T = K Q_s^T per KV tile (the operands swap roles, the tiles stay where they are)
           auto sweep_product = [&](auto s_tag, int st, bool wait_k) -> bool {
-            constexpr int s = decltype(s_tag)::value, b = s;
+            constexpr int s = decltype(s_tag)::value;
             if (wait_k && !mbar_wait(&bars->k_full[st], (kc / kStages) & 1, wc, DEV_TIMEOUT_MMA)) return false;
-            if (!mbar_wait(&bars->cs_empty[b], n_cst[b] & 1, wc, DEV_TIMEOUT_MMA)) return false;
-            ++n_cst[b];
+            if (!mbar_wait(&bars->cs_empty[s], n_cst[s] & 1, wc, DEV_TIMEOUT_MMA)) return false;
+            ++n_cst[s];
             tc_fence_after();
             const uint32_t tT = tmem_base + (uint32_t)s * 128u;
             const uint32_t qb = q_lo + (uint32_t)s * TILE16, ka = k_lo + (uint32_t)st * TILE16;
 #pragma unroll
             for (int kq = 0; kq < KSTEPS_QK; ++kq) {
               const uint32_t koff = (kq >> 2) * 1024 + (kq & 3) * 2;
-              umma_ss_if(leader, tT, ka + koff, DESC_HI, qb + koff, DESC_HI, IDESC_QK, kq > 0 ? 1u : 0u);
+              umma_ss(tT, ka + koff, DESC_HI, qb + koff, DESC_HI, IDESC_QK, kq > 0 ? 1u : 0u);
             }
-            umma_commit_if(leader, &bars->cs_full[s]);
+            umma_commit(&bars->cs_full[s]);
             return true;
           };
           for (int r = 0; r < rounds && ok; ++r) {
@@ -1410,7 +1410,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               ok = sweep_product(std::integral_constant<int, 0>{}, st, true);
               if (!ok) break;
               if (!shared) {
-                umma_commit_if(leader, &bars->k_empty[st]);
+                umma_commit(&bars->k_empty[st]);
                 ++kc;
               }
             }
@@ -1418,7 +1418,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               const int st = kc % kStages;
               ok = sweep_product(std::integral_constant<int, 1>{}, st, !shared);
               if (!ok) break;
-              umma_commit_if(leader, &bars->k_empty[st]);
+              umma_commit(&bars->k_empty[st]);
               ++kc;
             }
           }
