@@ -57,9 +57,9 @@ constexpr int kMaxSteps = 1024;  // per-slot KV tile list capacity (block-sparse
 constexpr int kMaxStages = 4;  // of K and of V each
 constexpr int kSchedStages = 2;
 // Column-sum sweep: which of the 8 groups of four exponentials per 32-column chunk are evaluated on the FMA
-// pipe (polynomial) instead of the exp2 unit, the sweep's bottleneck.  A quarter of them measured best
-// (0.47 -> 0.42 ms for the sweep at 4096 x 10521 x 32 heads; three eighths or a half: 0.43-0.45 ms); the same
-// mix in the statistics sweep of MODE_CS_ONLY gained nothing and is not used.
+// pipe (polynomial) instead of the exp2 unit.  A quarter of them measured best (0.47 -> 0.42 ms for the sweep at 4096 x 10521 x 32
+// heads when it was introduced, 0.375 at full clock and 0.44 under the power cap now; three eighths or a half: 0.43-0.45); the
+// same mix in the statistics sweep of MODE_CS_ONLY gained nothing and is not used.
 constexpr uint32_t kCsPolyMask = 0x88;
 // Log2 units by which a row maximum may exceed the row's reference maximum before the reference moves
 // (and O is rescaled).  bf16 has the exponent range of fp32, so P = exp2(s - reference) <= 2^32 is safe.

@@ -1,5 +1,5 @@
 // KV-cache compaction scores of ScaleKV (models/scalekv/scale_kv.py:232-301) and the row gather that
-// builds the compacted cache (pool and gather are byte movers; the scores are bound by the fp32 pipe, see below):
+// builds the compacted cache (pool and gather are byte movers; the scores are bound by latency, see below):
 //   scalekv_scores  score[b,h,j] = sum over the window queries i of bf16(bf16(q_i . k_j) / sqrt(D)), -inf on
 //                   the window's own columns (the reference's matmul, division, masked_fill and sum on bf16
 //                   tensors, rounding where torch rounds); K is read once
@@ -36,8 +36,9 @@ constexpr size_t scores_smem_bytes(int w) {
   return (size_t)kScoreKeys * (D * 2 + 16) + (size_t)((w + kQGroup - 1) / kQGroup) * D * kQGroup * 4;
 }
 
-// Bound by the fp32 pipe: the summation order of a logit is part of the result (its bf16 rounding decides which keys
-// stay), so the products stay on packed fp32 multiply-adds: D/8 partial sums of 8 consecutive elements, each added up
+// Bound by latency: of 35 us at 32 heads x 6425 keys x 16 queries (D = 128; kernel alone) the fp32 pipe needs 12 and K from HBM 8,
+// and the ten warps that fit an SM do not cover the rest.  The summation order of a logit is part of the result (its bf16
+// rounding decides which keys stay), so the products stay on packed fp32 multiply-adds: D/8 partial sums of 8 consecutive elements, each added up
 // in ascending order, then a pairwise tree over the partial sums p and p + D/16, p + D/32, ...  A thread owns two
 // whole keys and a group of 8 queries, so that one 16-byte shared-memory read of queries feeds four packed
 // multiply-adds; the tree is walked in the order that closes its pairs at once (a binary counter), which keeps at most
