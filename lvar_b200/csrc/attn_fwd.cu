@@ -1199,26 +1199,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (lane == 0) mbar_arrive(&bars->sched_empty[n % kSchedStages]);
       }
       if (MODE == MODE_CSP && lane == 0) bars->fetched[warp - 8] = kc;
-      // Drain on abort: copies in flight must land before the CTA's shared memory is released (gathered tiles: see the
-      // teardown).
-      if (lane == 0 && bars->abort_flag) {
-        const uint64_t t0 = globaltimer_ns();
-        if (nq_items > 0 && warp == 8)
-          while (!mbar_try_wait(&bars->q_full, (nq_items - 1) & 1) && globaltimer_ns() - t0 < 2000000000ull) {
+      // The last copies land before the loader leaves, whether or not anything has gone wrong: a role that gives up later must not
+      // let the CTA's shared memory go with copies in flight (gathered tiles: see the teardown).
+      if (lane == 0) {
+        auto landed = [&](uint64_t* bar, uint32_t parity) {
+          const uint64_t t0 = globaltimer_ns();
+          while (!mbar_try_wait(bar, parity) && globaltimer_ns() - t0 < 2000000000ull) {
           }
+        };
+        if (nq_items > 0 && warp == 8) landed(&bars->q_full, (nq_items - 1) & 1);
         if (MODE != MODE_CSP) {
-          for (int c = max(0, kc - kStages); c < kc; ++c) {
-            const uint64_t t1 = globaltimer_ns();
-            while (!mbar_try_wait(&bars->k_full[c % kStages], (c / kStages) & 1) &&
-                   globaltimer_ns() - t1 < 2000000000ull) {
-            }
-          }
-          for (int c = max(0, vc - kStages); c < vc; ++c) {
-            const uint64_t t1 = globaltimer_ns();
-            while (!mbar_try_wait(&bars->v_full[c % kStages], (c / kStages) & 1) &&
-                   globaltimer_ns() - t1 < 2000000000ull) {
-            }
-          }
+          for (int c = max(0, kc - kStages); c < kc; ++c) landed(&bars->k_full[c % kStages], (c / kStages) & 1);
+          for (int c = max(0, vc - kStages); c < vc; ++c) landed(&bars->v_full[c % kStages], (c / kStages) & 1);
         }
       }
     }
