@@ -248,7 +248,9 @@ colsum_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       }
       mbar_arrive(&bars->q_full[st]);
     }
-    if (lane == 0 && bars->abort_flag) {
+    // The last copies land before the loader leaves, also where nothing has gone wrong yet: a role that gives up later must not let
+    // the CTA's shared memory go with copies in flight.
+    if (lane == 0) {
       const uint64_t t0 = globaltimer_ns();
       while (!mbar_try_wait(&bars->k_full, 0) && globaltimer_ns() - t0 < 2000000000ull) {
       }

@@ -69,7 +69,14 @@ def _dense(K, D, size, status):
     return K.dense_attn_fwd(*_qkv(D, *size), status=status)
 
 
+def _stand_alone(K, D, size, status):
+    q, k, _ = _qkv(D, *size)
+    M, L = (torch.full((B, H, size[0]), x, device="cuda") for x in (2.0, 300.0))
+    return (K.colsum_fwd(q, k, M, L, 192, status=status),)
+
+
 CALLS = {"dense": _dense, "csp rows": _csp("rows"), "csp copies": _csp("copies"), "block": _block}
+CALLS["sums, stand-alone"] = _stand_alone
 CALLS |= {f"sums, {form}": _sums(form) for form in ("two sweeps", "no output", "given, no output", "given")}
 
 
